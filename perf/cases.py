@@ -1,0 +1,283 @@
+"""What this framework is run for, as a list of measurable cases.
+
+Five kinds of work, each through the entry points that a user's program calls:
+
+* ``train``: one optimizer step of the flow-matching MMDiT (``training.train_step`` over ``HunyuanPipeline``, the gradient
+  buffers and the ZeRO-1 AdamW): noise, forward, backward, update.  What pretraining does all day.
+* ``sample``: one evaluation of the transformer without gradients, the unit of a sampling run (a 50-step video is 50 or,
+  with guidance, 100 of these).
+* ``attention``: ``ops.attention`` forward and backward on one rank's share of the heads, as context parallelism
+  leaves it: few heads, the whole sequence.
+* ``mlp``: ``layernorm_modulate -> linear + GELU -> linear -> gated residual`` with all gradients, the text stream of a
+  dual-stream block: a few hundred rows against 75 MB of weights.
+* ``norms``: the drop-in ``fused_adaln`` / ``fused_rmsnorm`` entry points, forward and backward, for programs that were
+  written against those extensions.
+
+Widths are those of the 13B model (3072, 24 heads of 128, MLP 12288); depth is a slice of it (the sanity check's 3 dual
++ 6 single blocks for small clips, 1 + 2 for large ones: the same 1 : 2 as the full 20 + 40), because blocks repeat.
+"""
+
+import math
+import types
+
+import torch
+
+from teletron_b200 import ops
+from teletron_b200.legacy import fused_adaln, fused_rmsnorm
+from teletron_b200.models.hunyuanvideo import FlowConfig, HunyuanPipeline, HunyuanVideoTransformer3DModel, hunyuan_13b
+from teletron_b200.parallel.grad_buffer import DistributedDataParallel
+from teletron_b200.training import train_step
+from teletron_b200.training.optimizer import DistributedOptimizer, OptimizerParamScheduler
+
+HIDDEN, HEADS, HEAD_DIM, MLP, TEXT_DIM, POOLED_DIM = 3072, 24, 128, 12288, 4096, 768
+BF16 = torch.bfloat16
+
+
+def listed():
+    return [
+        # the smallest training sample: a single 256 x 256 image (16 x 16 tokens) and a full prompt; nothing is recomputed
+        dict(name="train_image_256", kind="train", dual=3, single=6, width=256, height=256, frames=1, batch=1, text=256,
+             model="t2v", recompute="none", state="split16"),
+        # the sanity-check script's clip: 640 x 368 x 9 frames, every block recomputed, fp32 master weights and moments
+        dict(name="train_368p_9f", kind="train", dual=3, single=6, width=640, height=368, frames=9, batch=1, text=120,
+             model="t2v", recompute="full", state="fp32"),
+        # image-to-video finetuning at 480P: two clips per micro-batch, 1590 tokens a frame, a token count that no tile
+        # divides, activations kept
+        dict(name="train_480p_17f_i2v", kind="train", dual=1, single=2, width=848, height=480, frames=17, batch=2, text=256,
+             model="i2v", recompute="none", state="fp32"),
+        # the headline benchmark's clip: 720P x 33 frames, blocks recomputed with the attention output kept
+        dict(name="train_720p_33f", kind="train", dual=1, single=2, width=1280, height=720, frames=33, batch=1, text=256,
+             model="t2v", recompute="keep", state="split16"),
+        # sampling a 512 x 512 image
+        dict(name="sample_image_512", kind="sample", dual=3, single=6, width=512, height=512, frames=1, batch=1, text=256,
+             model="t2v", text_mask=False),
+        # image-to-video sampling at 480P with the padded part of the prompt masked
+        dict(name="sample_480p_33f_i2v", kind="sample", dual=1, single=2, width=848, height=480, frames=33, batch=1, text=256,
+             model="i2v", text_mask=True),
+        # the sampling pipeline's default clip: 720P x 129 frames
+        dict(name="sample_720p_129f", kind="sample", dual=1, single=2, width=1280, height=720, frames=129, batch=1, text=256,
+             model="t2v", text_mask=False),
+        # one of eight context-parallel ranks at 720P x 129 frames: 3 heads, 118 800 video + 256 text tokens
+        dict(name="attention_cp8_129f", kind="attention", batch=1, heads=3, seq=119056, kv_len=0, mask_lo=0, mask_hi=0),
+        # short clips with padding keys at the tail and padded text in front, two samples
+        dict(name="attention_short_masked", kind="attention", batch=2, heads=24, seq=1237, kv_len=1201, mask_lo=180, mask_hi=256),
+        # the text stream's MLP of one dual-stream block: 256 prompt tokens
+        dict(name="mlp_text_256", kind="mlp", batch=1, rows=256),
+        # the reference's two extensions on the text stream (where calls are short) and on 720P x 33 frames
+        dict(name="norms_text_256", kind="norms", rows=256, cols=3072),
+        dict(name="norms_720p_33f", kind="norms", rows=32656, cols=3072),
+    ]
+
+
+# ------------------------------------------------------------------------------------------------ more of the same ranges
+
+def _log_int(rng, lo, hi):
+    return int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))
+
+
+def _clip(rng, lo, hi):
+    """A clip of ``lo .. hi`` video tokens: latent frames, and a grid of 16 x 16 pixel tokens of a usual aspect ratio."""
+    n = _log_int(rng, lo, hi)
+    f = rng.choice([k for k in (1, 2, 3, 5, 7, 9, 13, 17, 22, 33) if n // k >= 100 or k == 1])
+    th = max(6, int(round(math.sqrt(n / f / rng.uniform(0.6, 2.0)))))
+    tw = max(6, int(n / f / th))
+    while f * th * tw > hi:
+        tw -= 1
+    return dict(width=16 * tw, height=16 * th, frames=4 * (f - 1) + 1)
+
+
+def draw(rng):
+    kind = rng.choice(["train", "train", "sample", "sample", "attention", "attention", "mlp", "norms"])
+    if kind == "train":
+        # the least clips at the sanity check's depth, longer ones at the shallow one
+        small = rng.random() < 0.4
+        c = dict(kind=kind, dual=3 if small else 1, single=6 if small else 2, **(_clip(rng, 200, 2800) if small else _clip(rng, 2000, 32400)))
+        n = _video_tokens(c)
+        c["batch"] = rng.choice([1, 1, 2]) if n <= 8000 else 1
+        c["text"] = rng.choice([256, 120, rng.randint(40, 256)])
+        c["model"] = rng.choice(["t2v", "i2v"])
+        c["recompute"] = rng.choice(["none", "full", "keep"]) if n * c["batch"] <= 16000 else rng.choice(["full", "keep"])
+        c["state"] = rng.choice(["split16", "fp32"])
+        return c
+    if kind == "sample":
+        small = rng.random() < 0.4
+        c = dict(kind=kind, dual=3 if small else 1, single=6 if small else 2, **(_clip(rng, 200, 4000) if small else _clip(rng, 3000, 100000)))
+        c["batch"] = rng.choice([1, 1, 2]) if _video_tokens(c) <= 16000 else 1
+        c["text"] = rng.choice([256, 120, rng.randint(40, 256)])
+        c["model"] = rng.choice(["t2v", "i2v"])
+        c["text_mask"] = rng.random() < 0.5
+        return c
+    if kind == "attention":
+        heads = rng.choice([1, 2, 3, 4, 6, 8, 12, 24])
+        batch = rng.choice([1, 1, 2])
+        seq = _log_int(rng, 200, min(110000, int(100000 * math.sqrt(3.0 / (heads * batch)))))
+        c = dict(kind=kind, batch=batch, heads=heads, seq=seq, kv_len=0, mask_lo=0, mask_hi=0)
+        if rng.random() < 0.5:
+            c["kv_len"] = seq - rng.randint(1, 63)
+        if rng.random() < 0.3:
+            c["mask_lo"], c["mask_hi"] = rng.randint(20, 90), rng.randint(91, 130)
+        return c
+    if kind == "mlp":
+        return dict(kind=kind, batch=rng.choice([1, 1, 2]), rows=rng.randint(40, 512) if rng.random() < 0.7 else _log_int(rng, 40, 2000))
+    return dict(kind=kind, rows=_log_int(rng, 100, 60000), cols=rng.choice([3072, 3072, 1024, 2048, 4096, 6144]))
+
+
+# ------------------------------------------------------------------------------------------------ inputs
+
+def _video_tokens(c):
+    return ((c["frames"] - 1) // 4 + 1) * (c["height"] // 16) * (c["width"] // 16)
+
+
+def _config(c, seed):
+    rec = c.get("recompute", "none")
+    return hunyuan_13b(in_channels=33 if c["model"] == "i2v" else 16, num_layers=c["dual"], num_single_layers=c["single"],
+                       recompute_granularity=None if rec == "none" else "full", recompute_save_attention=rec == "keep",
+                       apply_text_mask=bool(c.get("text_mask", False)), seed=seed)
+
+
+def _batch(c, g, dev):
+    """Latents are close to standard normal after the VAE's scaling; so are the language model's hidden states."""
+    rn = lambda *s: torch.randn(*s, device=dev, generator=g).to(BF16)  # noqa: E731
+    f, B = (c["frames"] - 1) // 4 + 1, c["batch"]
+    valid = torch.randint(c["text"] // 4, c["text"] + 1, (B,), device=dev, generator=g)
+    batch = {"latents": rn(B, 16, f, c["height"] // 8, c["width"] // 8), "prompt_embeds": rn(B, c["text"], TEXT_DIM),
+             "clip_text_embed": rn(B, POOLED_DIM), "prompt_attention_mask": torch.arange(c["text"], device=dev)[None] < valid[:, None]}
+    if c["model"] == "i2v":
+        batch["first_frame_latents"] = rn(B, 16, 1, c["height"] // 8, c["width"] // 8)
+    return batch
+
+
+def prepare(case, seed):
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(seed)
+    kind = case["kind"]
+    if kind == "train":
+        pipe = HunyuanPipeline(_config(case, seed), FlowConfig(model_type=case["model"], shift=7.0), device=dev, dtype=BF16)
+        ddp = DistributedDataParallel(pipe, None)
+        fp32 = case["state"] == "fp32"
+        opt = DistributedOptimizer(ddp, lr=1e-5, weight_decay=1e-2, master_mode="fp32" if fp32 else "split16",
+                                   state_dtype=torch.float32 if fp32 else BF16)
+        args = types.SimpleNamespace(num_microbatches=1, comm_check_interval=1)
+        return dict(kind=kind, ddp=ddp, opt=opt, sched=OptimizerParamScheduler(opt, max_lr=1e-5), args=args, batch=_batch(case, g, dev))
+    if kind == "sample":
+        model = HunyuanVideoTransformer3DModel(_config(case, seed), tp=1, device=dev, dtype=BF16).eval()
+        b = _batch(case, g, dev)
+        x = b["latents"]
+        if case["model"] == "i2v":
+            cond = torch.zeros_like(x)
+            cond[:, :, :1] = b["first_frame_latents"]
+            m = torch.zeros_like(x[:, :1])
+            m[:, :, 0] = 1
+            x = torch.cat([x, cond, m], dim=1)
+        t = torch.rand(case["batch"], device=dev, generator=g) * 1000
+        return dict(kind=kind, model=model, x=x, t=t, text=b["prompt_embeds"], mask=b["prompt_attention_mask"],
+                    pooled=b["clip_text_embed"], guidance=torch.full((case["batch"],), 6000.0, device=dev))
+    rn = lambda *s, k=1.0: (torch.randn(*s, device=dev, generator=g) * k).to(BF16)  # noqa: E731
+    if kind == "attention":
+        B, H, S = case["batch"], case["heads"], case["seq"]
+        # q and k leave an RMSNorm and a rotation: rows of norm sqrt(128)
+        q, k, v = (rn(B, H, S, HEAD_DIM).requires_grad_() for _ in range(3))
+        mask = (case["mask_lo"], case["mask_hi"]) if case["mask_lo"] < case["mask_hi"] else None
+        return dict(kind=kind, q=q, k=k, v=v, dout=rn(B, S, H * HEAD_DIM), kv_len=case["kv_len"] or None, mask=mask)
+    if kind == "mlp":
+        B, R = case["batch"], case["rows"]
+        s = dict(x=rn(B, R, HIDDEN), shift=rn(B, HIDDEN, k=0.3), scale=rn(B, HIDDEN, k=0.3), gate=rn(B, HIDDEN, k=0.3),
+                 w1=rn(MLP, HIDDEN, k=0.02), b1=rn(MLP, k=0.1), w2=rn(HIDDEN, MLP, k=0.01), b2=rn(HIDDEN, k=0.1))
+        for t in s.values():
+            t.requires_grad_()
+        return dict(kind=kind, dout=rn(B, R, HIDDEN), **s)
+    R, C = case["rows"], case["cols"]
+    e = lambda *s: torch.empty(*s, dtype=BF16, device=dev)  # noqa: E731
+    return dict(kind=kind, rows=R, cols=C, x=rn(R, C), scale=rn(C, k=0.3), shift=rn(C, k=0.3), dy=rn(R, C),
+                w=(1 + 0.2 * torch.randn(HEAD_DIM, device=dev, generator=g)).to(BF16),
+                y=e(R, C), xn=e(R, C), rstd=torch.empty(R, device=dev), dx=e(R, C), dscale=e(C), dshift=e(C),
+                hy=e(R, C), hrstd=torch.empty(R * (C // HEAD_DIM), device=dev), hdx=e(R, C), dw=e(HEAD_DIM))
+
+
+# ------------------------------------------------------------------------------------------------ one pass
+
+def _loss(out):
+    loss = out[0].mean()
+    return loss, {"loss": loss.detach()}
+
+
+def run(s):
+    kind = s["kind"]
+    if kind == "train":
+        batch = s["batch"]
+        losses, _, _ = train_step(lambda _it, model: (model(batch), _loss), None, s["ddp"], s["opt"], s["sched"], s["args"])
+        buf = s["ddp"].buffers[0]
+        return {"loss": losses["loss"], "grads": buf.grad_data, "params": buf.param_data}
+    if kind == "sample":
+        with torch.no_grad():
+            return s["model"](s["x"], s["t"], s["text"], s["mask"], s["pooled"], s["guidance"])[0]
+    if kind == "attention":
+        o = ops.attention(s["q"], s["k"], s["v"], s["kv_len"], None, s["mask"])
+        return (o.detach(),) + torch.autograd.grad(o, (s["q"], s["k"], s["v"]), s["dout"])
+    if kind == "mlp":
+        h = ops.layernorm_modulate(s["x"], s["scale"], s["shift"])
+        h = ops.linear(ops.linear(h, s["w1"], s["b1"], "gelu"), s["w2"], s["b2"])
+        y = ops.gate_residual(s["x"], h, s["gate"])
+        wrt = [s[n] for n in ("x", "shift", "scale", "gate", "w1", "b1", "w2", "b2")]
+        return (y.detach(),) + torch.autograd.grad(y, wrt, s["dout"])
+    R, C = s["rows"], s["cols"]
+    fused_adaln.torch_launch_adaln_forward(s["y"], s["x"], s["scale"], s["shift"], s["xn"], s["rstd"], R, C)
+    fused_adaln.torch_launch_adaln_backward(s["dx"], s["dscale"], s["dshift"], s["dy"], s["xn"], s["scale"], s["rstd"], R, C)
+    n = C // HEAD_DIM
+    fused_rmsnorm.torch_launch_rms_forward(s["hy"], s["x"], s["w"], s["hrstd"], R * n, HEAD_DIM)
+    fused_rmsnorm.torch_launch_rms_backward(s["hdx"], s["dw"], s["dy"], s["x"], s["w"], s["hrstd"], R * n, HEAD_DIM)
+    return {k: s[k] for k in ("y", "xn", "rstd", "dx", "dscale", "dshift", "hy", "hrstd", "hdx", "dw")}
+
+
+# ------------------------------------------------------------------------------------------------ what a pass cannot do without
+
+def _params(c):
+    """(per-video-token, per-text-token, per-sample) parameters of the model: what each kind of row is multiplied with."""
+    h, d, s = HIDDEN, c["dual"], c["single"]
+    stream = 4 * h * h + 2 * h * MLP                       # QKV, projection, two MLP products
+    joint = 3 * h * h + h * MLP + (h + MLP) * h            # the same of a single-stream block
+    cin = 33 if c["model"] == "i2v" else 16
+    video = d * stream + s * joint + h * cin * 4 + h * 64
+    text = d * stream + s * joint + TEXT_DIM * h + 2 * (4 * h * h + 8 * h * h)
+    vec = d * 12 * h * h + s * 3 * h * h + 2 * h * h + 2 * 2 * h * h + 4 * (256 + h) * h + (POOLED_DIM + TEXT_DIM + 2 * h) * h
+    return video, text, vec
+
+
+def work(case):
+    kind = case["kind"]
+    if kind in ("train", "sample"):
+        n, t, b = _video_tokens(case), case["text"], case["batch"]
+        pv, pt, ps = _params(case)
+        lin = 2.0 * b * (n * pv + t * pt + ps)
+        att = 4.0 * b * (n + t) ** 2 * HIDDEN * (case["dual"] + case["single"])
+        h = HIDDEN
+        # weights: each dual-stream block holds one set for the video and one for the text
+        weights = case["dual"] * 2 * (4 * h * h + 2 * h * MLP) + case["single"] * (3 * h * h + h * MLP + (h + MLP) * h) + ps \
+            + h * (16 * 4 + 64 + TEXT_DIM) + 24 * h * h
+        cin = 33 if case["model"] == "i2v" else 16
+        io = 2.0 * b * (n * 4 * (cin + 16) + t * TEXT_DIM)
+        if kind == "sample":
+            return {"bytes": 2.0 * weights + io, "flops": lin + att}
+        state = 8 if case["state"] == "fp32" else 4        # moments, read and written; and the master's own part
+        master = 4 if case["state"] == "fp32" else 2
+        return {"bytes": weights * (2.0 + 2.0 + 2.0 + 2.0 * (state + master)) + io, "flops": 3.0 * lin + 3.5 * att}
+    if kind == "attention":
+        B, H, S = case["batch"], case["heads"], case["seq"]
+        keys = (case["kv_len"] or S) - (case["mask_hi"] - case["mask_lo"])
+        return {"bytes": 2.0 * B * H * S * HEAD_DIM * 8, "flops": 3.5 * 4.0 * B * H * S * keys * HEAD_DIM}
+    if kind == "mlp":
+        rows = case["batch"] * case["rows"]
+        return {"bytes": 2.0 * (4 * HIDDEN * MLP + 4 * rows * HIDDEN), "flops": 6.0 * rows * 2 * HIDDEN * MLP}
+    R, C = case["rows"], case["cols"]
+    # x, dy in; y, xn, dx, hy, hdx out; the statistics
+    return {"bytes": 2.0 * 7 * R * C + 4.0 * (R + R * (C // HEAD_DIM)), "flops": 40.0 * R * C}
+
+
+def tolerance(case):
+    """About four times what the same path on plain PyTorch bf16 operations (other summation orders, other places of
+    rounding) differs by: 4e-3 for gradients of a training step, 1.2e-3 for a prediction, 3.7e-3 for attention
+    gradients, 4.5e-3 for the MLP's, and one bf16 rounding more or less (2e-3, elementwise 8e-3) for the norms.  A
+    training step's gradient buffer spans orders of magnitude between layers: single elements differ by up to 0.8 of
+    its root mean square."""
+    return {"train": {"rel": 1.6e-2, "max": 0.99}, "sample": {"rel": 5e-3, "max": 4e-2}, "attention": {"rel": 1.5e-2, "max": 0.13},
+            "mlp": {"rel": 1.8e-2, "max": 0.25}, "norms": {"rel": 6e-3, "max": 4e-2}}[case["kind"]]
