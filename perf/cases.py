@@ -281,3 +281,63 @@ def tolerance(case):
     its root mean square."""
     return {"train": {"rel": 1.6e-2, "max": 0.99}, "sample": {"rel": 5e-3, "max": 4e-2}, "attention": {"rel": 1.5e-2, "max": 0.13},
             "mlp": {"rel": 1.8e-2, "max": 0.25}, "norms": {"rel": 6e-3, "max": 4e-2}}[case["kind"]]
+
+
+# ------------------------------------------------------------------------------------------------ the same in 64 bits
+
+def _exact_attention(s):
+    q, k, v = (s[n].detach().double() for n in "qkv")
+    B, H, S, D = q.shape
+    dout = s["dout"].double().view(B, S, H, D).transpose(1, 2)
+    dead = torch.zeros(S, dtype=torch.bool, device=q.device)
+    if s["kv_len"]:
+        dead[s["kv_len"]:] = True
+    if s["mask"]:
+        dead[s["mask"][0]:s["mask"][1]] = True
+    o, dq, dk, dv = torch.empty_like(q), torch.empty_like(q), torch.zeros_like(k), torch.zeros_like(v)
+    step = max(64, (1 << 27) // S)  # 1 GB of probabilities at a time
+    for b in range(B):
+        for h in range(H):
+            for r in range(0, S, step):
+                rows = slice(r, r + step)
+                qc, do = q[b, h, rows], dout[b, h, rows]
+                p = (qc @ k[b, h].T).mul_(D ** -0.5).masked_fill_(dead, -math.inf)
+                p = torch.softmax(p, -1)
+                o[b, h, rows] = p @ v[b, h]
+                dv[b, h] += p.T @ do
+                dp = do @ v[b, h].T
+                ds = p.mul_(dp.sub_((do * o[b, h, rows]).sum(-1, keepdim=True))).mul_(D ** -0.5)
+                dq[b, h, rows] = ds @ k[b, h]
+                dk[b, h] += ds.T @ qc
+    return o.transpose(1, 2).reshape(B, S, H * D), dq, dk, dv
+
+
+def _exact_mlp(s):
+    names = ("x", "shift", "scale", "gate", "w1", "b1", "w2", "b2")
+    p = {n: s[n].detach().double().requires_grad_() for n in names}
+    h = torch.nn.functional.layer_norm(p["x"], (HIDDEN,), eps=1e-6) * (1 + p["scale"][:, None]) + p["shift"][:, None]
+    h = torch.nn.functional.gelu(h @ p["w1"].T + p["b1"])
+    y = p["x"] + p["gate"][:, None] * (h @ p["w2"].T + p["b2"])
+    return (y.detach(),) + torch.autograd.grad(y, [p[n] for n in names], s["dout"].double())
+
+
+def _exact_norms(s):
+    x, dy, w, scale = (s[n].double() for n in ("x", "dy", "w", "scale"))
+    var, mean = torch.var_mean(x, -1, unbiased=False, keepdim=True)
+    rstd = (var + 1e-6).rsqrt()
+    xn = (x - mean) * rstd
+    g = dy * (1 + scale)
+    dx = rstd * (g - g.mean(-1, keepdim=True) - xn * (g * xn).mean(-1, keepdim=True))
+    out = dict(y=xn * (1 + scale) + s["shift"].double(), xn=xn, rstd=rstd[:, 0], dx=dx, dscale=(dy * xn).sum(0), dshift=dy.sum(0))
+    x, dy = x.view(-1, HEAD_DIM), dy.view(-1, HEAD_DIM)
+    rstd = (x.square().mean(-1, keepdim=True) + 1e-6).rsqrt()
+    xn, g = x * rstd, dy * w
+    hdx = rstd * (g - xn * (g * xn).mean(-1, keepdim=True))
+    out.update(hy=(xn * w).view(s["rows"], s["cols"]), hrstd=rstd[:, 0], hdx=hdx.view(s["rows"], s["cols"]), dw=(dy * xn).sum(0))
+    return out
+
+
+def exact(case, seed):
+    """None for the whole model: its weights and inputs take minutes in 64 bits."""
+    f = {"attention": _exact_attention, "mlp": _exact_mlp, "norms": _exact_norms}.get(case["kind"])
+    return f(prepare(case, seed)) if f else None
