@@ -20,12 +20,16 @@ constexpr int kMaxCols = 8192;
 // ---------------------------------------------------------------------------------------------
 // forward: one warp per row, the row lives in registers
 // ---------------------------------------------------------------------------------------------
-template <int VPL, bool GATE>
+// XN (drop-in fused_adaln): the normalised row is stored as well, from the registers that hold it anyway; no mean.  Bound by
+// HBM: at 32656 x 3072 it takes 95 us (600 MB, 6.3 TB/s).  Forming x_norm from x, mean and rstd with separate elementwise
+// passes took another 0.8 ms, and scaling the backward's result by rstd in two more passes as much again; the pair with
+// the RMSNorm pair went from 2122 to 417 us there, and from 143 to 46 us at 256 rows.
+template <int VPL, bool GATE, bool XN = false>
 __global__ void __launch_bounds__(256, (VPL <= 12 ? 3 : 1)) ln_mod_fwd_kernel(
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ branch,
     const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ scale,
     const __nv_bfloat16* __restrict__ shift, __nv_bfloat16* __restrict__ new_res,
-    __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out,
+    __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ xn, float* __restrict__ mean_out, float* __restrict__ rstd_out,
     long rows, int cols, long rows_per_batch, float eps) {
     // The row stays in registers as packed bf16 (4 registers per 8 elements) and is unpacked in each of the three
     // passes: that keeps the kernel under 85 registers, so three CTAs (24 warps, each with a whole row of loads in
@@ -83,7 +87,7 @@ __global__ void __launch_bounds__(256, (VPL <= 12 ? 3 : 1)) ln_mod_fwd_kernel(
         }
         const float rstd = rsqrtf(warp_sum(sq) * inv_cols + eps);
         if (lane == 0) {
-            mean_out[row] = mean;
+            if (!XN) mean_out[row] = mean;
             rstd_out[row] = rstd;
         }
 #pragma unroll
@@ -95,8 +99,12 @@ __global__ void __launch_bounds__(256, (VPL <= 12 ? 3 : 1)) ln_mod_fwd_kernel(
                 unpack8(ld8(scale + b * cols + c * 8), sc);
                 unpack8(ld8(shift + b * cols + c * 8), sh);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) o[j] = (v[j] - mean) * rstd * (1.f + sc[j]) + sh[j];
+                for (int j = 0; j < 8; ++j) {
+                    v[j] = (v[j] - mean) * rstd;
+                    o[j] = v[j] * (1.f + sc[j]) + sh[j];
+                }
                 st8(y + row * cols + c * 8, pack8(o));
+                if (XN) st8(xn + row * cols + c * 8, pack8(v));
             }
         }
     }
@@ -141,7 +149,8 @@ __device__ __forceinline__ void block_sum_batch(float* v, float* red, int parity
     for (int q = 0; q < 8; ++q) v[q] = __shfl_sync(0xffffffffu, t, q);
 }
 
-template <bool GATE, int MAXT>
+// XHAT: `x` is the normalised row itself (drop-in fused_adaln, which saves it instead of the mean); rstd still scales dx.
+template <bool GATE, int MAXT, bool XHAT = false>
 __global__ void __launch_bounds__(MAXT) ln_mod_bwd_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ dres_in,
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ branch,
@@ -176,7 +185,7 @@ __global__ void __launch_bounds__(MAXT) ln_mod_bwd_kernel(
         for (int k = 0; k < kRowBatch; ++k) {
             const bool live = r0 + k < rows_per_batch;
             const long row = b * rows_per_batch + (live ? r0 + k : r0);
-            mu[k] = mean[row];
+            mu[k] = XHAT ? 0.f : mean[row];
             rs[k] = rstd[row];
             if (active && live) {
                 pdy[k] = ld8(dy + row * cols + t * 8);
@@ -197,7 +206,7 @@ __global__ void __launch_bounds__(MAXT) ln_mod_bwd_kernel(
             if (active) {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const float xh = (xv[j] - mu[k]) * rs[k];
+                    const float xh = XHAT ? xv[j] : (xv[j] - mu[k]) * rs[k];
                     const float g = dyv[j] * sc1[j];
                     s1 += g;
                     s2 += g * xh;
@@ -219,7 +228,7 @@ __global__ void __launch_bounds__(MAXT) ln_mod_bwd_kernel(
                 unpack8(px[k], xv);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const float xh = (xv[j] - mu[k]) * rs[k];
+                    const float xh = XHAT ? xv[j] : (xv[j] - mu[k]) * rs[k];
                     d[j] = rs[k] * (dyv[j] * sc1[j] - m1 - xh * m2);
                 }
                 if (dres_in != nullptr) {
@@ -287,7 +296,7 @@ __device__ __forceinline__ void consumer_sum_batch(float* v, float* red, int par
     for (int q = 0; q < 8; ++q) v[q] = __shfl_sync(0xffffffffu, t, q);
 }
 
-template <bool GATE, int MAXT>
+template <bool GATE, int MAXT, bool XHAT = false>
 __global__ void __launch_bounds__(MAXT + 32) ln_mod_bwd_ring_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ dres_in,
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ branch,
@@ -366,7 +375,7 @@ __global__ void __launch_bounds__(MAXT + 32) ln_mod_bwd_ring_kernel(
 #pragma unroll
             for (int k = 0; k < kRowBatch; ++k) {
                 const long row = b * rows_per_batch + (k < live ? r0 + k : r0);
-                mu[k] = mean[row];
+                mu[k] = XHAT ? 0.f : mean[row];
                 rs[k] = rstd[row];
                 if (active && k < live) {
                     if (dres_in != nullptr) pup[k] = ld8(dres_in + row * cols + t * 8);
@@ -393,7 +402,7 @@ __global__ void __launch_bounds__(MAXT + 32) ln_mod_bwd_ring_kernel(
                     unpack8(ring_row(1, k), xv);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const float xh = (xv[j] - mu[k]) * rs[k];
+                        const float xh = XHAT ? xv[j] : (xv[j] - mu[k]) * rs[k];
                         const float g = dyv[j] * sc1[j];
                         s1 += g;
                         s2 += g * xh;
@@ -415,7 +424,7 @@ __global__ void __launch_bounds__(MAXT + 32) ln_mod_bwd_ring_kernel(
                     unpack8(ring_row(1, k), xv);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const float xh = (xv[j] - mu[k]) * rs[k];
+                        const float xh = XHAT ? xv[j] : (xv[j] - mu[k]) * rs[k];
                         d[j] = rs[k] * (dyv[j] * sc1[j] - m1 - xh * m2);
                     }
                     if (dres_in != nullptr) {
@@ -463,29 +472,47 @@ __global__ void __launch_bounds__(MAXT + 32) ln_mod_bwd_ring_kernel(
     }
 }
 
-// out[k][b][c] (bf16) = sum over blocks of partials[b][blk][k][c]
-__global__ void column_finalize_kernel(const float* __restrict__ partials, __nv_bfloat16* __restrict__ out0,
-                                       __nv_bfloat16* __restrict__ out1, __nv_bfloat16* __restrict__ out2, int K,
-                                       int nblk, int cols) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+// out[k][b][c] (bf16) = sum over blocks of partials[b][blk][k][c].  A CTA owns 32 columns, its kSlices warps a slice of the
+// partial rows each, so the chain of dependent loads is nblk / (4 kSlices) long: the partials sit in L2 and latency is all
+// this kernel costs: 2.5 us for 64 x 2 x 3072, where one thread per column walked the rows in 25 - 29 us.  The order is fixed
+// (deterministic).
+constexpr int kSlices = 16;
+
+__global__ void __launch_bounds__(32 * kSlices) column_finalize_kernel(const float* __restrict__ partials, __nv_bfloat16* __restrict__ out0,
+                                                                       __nv_bfloat16* __restrict__ out1, __nv_bfloat16* __restrict__ out2,
+                                                                       int K, int nblk, int cols) {
+    __shared__ float fold[kSlices][32];
+    const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+    const int c = blockIdx.x * 32 + lane;
     const int k = blockIdx.y;
     const long b = blockIdx.z;
-    if (c >= cols) return;
-    // four independent chains keep several loads in flight; the order is fixed, so the sum is deterministic
+    const bool ok = c < cols;
+    // four independent chains keep several loads in flight
     float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-    const float* p = partials + (b * nblk * K + k) * (long)cols + c;
+    const float* p = partials + (b * nblk * K + k) * (long)cols + (ok ? c : 0);
     const long step = (long)K * cols;
-    int i = 0;
-    for (; i + 3 < nblk; i += 4) {
-        s0 += p[(i + 0) * step];
-        s1 += p[(i + 1) * step];
-        s2 += p[(i + 2) * step];
-        s3 += p[(i + 3) * step];
+    int i = slice;
+    for (; i + 3 * kSlices < nblk; i += 4 * kSlices) {
+        s0 += p[i * step];
+        s1 += p[(i + kSlices) * step];
+        s2 += p[(i + 2 * kSlices) * step];
+        s3 += p[(i + 3 * kSlices) * step];
     }
-    for (; i < nblk; ++i) s0 += p[i * step];
-    const float s = (s0 + s1) + (s2 + s3);
-    __nv_bfloat16* o = k == 0 ? out0 : (k == 1 ? out1 : out2);
-    if (o != nullptr) o[b * cols + c] = __float2bfloat16(s);
+    for (; i < nblk; i += kSlices) s0 += p[i * step];
+    fold[slice][lane] = (s0 + s1) + (s2 + s3);
+    __syncthreads();
+    if (slice == 0 && ok) {
+        float s = 0.f;
+#pragma unroll
+        for (int w = 0; w < kSlices; ++w) s += fold[w][lane];
+        __nv_bfloat16* o = k == 0 ? out0 : (k == 1 ? out1 : out2);
+        if (o != nullptr) o[b * cols + c] = __float2bfloat16(s);
+    }
+}
+
+inline void launch_finalize(const float* partials, void* out0, void* out1, void* out2, int K, int nblk, int cols, int batch, cudaStream_t st) {
+    column_finalize_kernel<<<dim3((cols + 31) / 32, K, batch), 32 * kSlices, 0, st>>>(partials, (__nv_bfloat16*)out0, (__nv_bfloat16*)out1,
+                                                                                     (__nv_bfloat16*)out2, K, nblk, cols);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -806,11 +833,11 @@ extern "C" int tt_norm_status(void) {
 #define LAUNCH_FWD(VPL)                                                                                         \
     do {                                                                                                        \
         if (has_gate)                                                                                           \
-            ln_mod_fwd_kernel<VPL, true><<<grid, 256, 0, st>>>(X, BR, G, SC, SH, NR, Y, mean, rstd, rows, cols, \
-                                                               rows_per_batch, eps);                            \
+            ln_mod_fwd_kernel<VPL, true><<<grid, 256, 0, st>>>(X, BR, G, SC, SH, NR, Y, nullptr, mean, rstd,    \
+                                                               rows, cols, rows_per_batch, eps);                \
         else                                                                                                    \
-            ln_mod_fwd_kernel<VPL, false><<<grid, 256, 0, st>>>(X, BR, G, SC, SH, NR, Y, mean, rstd, rows,      \
-                                                                cols, rows_per_batch, eps);                     \
+            ln_mod_fwd_kernel<VPL, false><<<grid, 256, 0, st>>>(X, BR, G, SC, SH, NR, Y, nullptr, mean, rstd,   \
+                                                                rows, cols, rows_per_batch, eps);               \
     } while (0)
 
 extern "C" int tt_ln_mod_fwd(const void* x, const void* branch, const void* gate, const void* scale,
@@ -839,10 +866,33 @@ extern "C" int tt_ln_mod_fwd(const void* x, const void* branch, const void* gate
     return TT_OK;
 }
 
-extern "C" int tt_ln_mod_bwd(const void* dy, const void* dres_in, const void* x, const void* branch,
-                             const void* gate, const void* scale, const float* mean, const float* rstd, void* dx,
-                             void* dbranch, float* partials, void* dscale, void* dshift, void* dgate, long rows,
-                             int cols, long rows_per_batch, void* stream) {
+// fused_adaln forward: y = LN(x) (1 + scale) + shift with one modulation vector for all rows, xn = LN(x), rstd per row
+extern "C" int tt_adaln_fwd(const void* x, const void* scale, const void* shift, void* y, void* xn, float* rstd, long rows, int cols,
+                            float eps, void* stream) {
+    if (bad_cols(cols) || rows <= 0) return TT_ERR_ARG;
+    cudaStream_t st = (cudaStream_t)stream;
+    const long want = (rows + 7) / 8;
+    const int grid = (int)(want < 148L * 16 ? want : 148L * 16);
+    const int vpl = ((cols >> 3) + 31) / 32;
+#define ADALN_FWD(VPL)                                                                                                          \
+    ln_mod_fwd_kernel<VPL, false, true><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, nullptr, nullptr, (const __nv_bfloat16*)scale, \
+                                                              (const __nv_bfloat16*)shift, nullptr, (__nv_bfloat16*)y,          \
+                                                              (__nv_bfloat16*)xn, nullptr, rstd, rows, cols, rows, eps)
+    if (vpl <= 4) ADALN_FWD(4);
+    else if (vpl <= 8) ADALN_FWD(8);
+    else if (vpl <= 12) ADALN_FWD(12);
+    else if (vpl <= 16) ADALN_FWD(16);
+    else ADALN_FWD(32);
+#undef ADALN_FWD
+    TT_CHECK_LAUNCH();
+    return TT_OK;
+}
+
+namespace {
+// `xhat`: x holds normalised rows (no mean, no gate)
+int ln_mod_bwd(const void* dy, const void* dres_in, const void* x, const void* branch, const void* gate, const void* scale,
+               const float* mean, const float* rstd, void* dx, void* dbranch, float* partials, void* dscale, void* dshift, void* dgate,
+               long rows, int cols, long rows_per_batch, bool xhat, void* stream) {
     if (bad_cols(cols) || rows <= 0 || rows_per_batch <= 0 || rows % rows_per_batch) return TT_ERR_ARG;
     const bool has_gate = branch != nullptr;
     if (has_gate && (gate == nullptr || dbranch == nullptr || dgate == nullptr)) return TT_ERR_ARG;
@@ -860,16 +910,19 @@ extern "C" int tt_ln_mod_bwd(const void* dy, const void* dres_in, const void* x,
         int dev = 0, sms = 148;
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         int g = sms / batch;
+        const long row_batches = (rows_per_batch + kRowBatch - 1) / kRowBatch;      // a CTA without rows would only add a partial row
+        if (g > row_batches) g = (int)row_batches;
         if (g < 1) g = 1;
         if (g > nblk) g = nblk;
         nblk_used = g;
         const int smem = (int)(stages * stage_bytes) + 16 * stages + 256;
         const bool wide = threads > 512;
         auto kern = has_gate ? (wide ? ln_mod_bwd_ring_kernel<true, 1024> : ln_mod_bwd_ring_kernel<true, 512>)
-                             : (wide ? ln_mod_bwd_ring_kernel<false, 1024> : ln_mod_bwd_ring_kernel<false, 512>);
-        static int configured[4][64] = {{0}};
+                  : xhat   ? (wide ? ln_mod_bwd_ring_kernel<false, 1024, true> : ln_mod_bwd_ring_kernel<false, 512, true>)
+                           : (wide ? ln_mod_bwd_ring_kernel<false, 1024> : ln_mod_bwd_ring_kernel<false, 512>);
+        static int configured[6][64] = {{0}};
         if (dev < 0 || dev >= 64) dev = 0;
-        const int which = (has_gate ? 2 : 0) + (wide ? 1 : 0);
+        const int which = (has_gate ? 2 : (xhat ? 4 : 0)) + (wide ? 1 : 0);
         if (configured[which][dev] < smem) {
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return tt_record_cuda(e);
@@ -883,14 +936,17 @@ extern "C" int tt_ln_mod_bwd(const void* dy, const void* dres_in, const void* x,
         TT_CHECK_LAUNCH();
     } else {
     dim3 grid(nblk, batch);
-#define LN_BWD(G_, T_)                                                                                          \
-    ln_mod_bwd_kernel<G_, T_><<<grid, threads, 0, st>>>(                                                        \
+#define LN_BWD(...)                                                                                             \
+    ln_mod_bwd_kernel<__VA_ARGS__><<<grid, threads, 0, st>>>(                                                        \
         (const __nv_bfloat16*)dy, (const __nv_bfloat16*)dres_in, (const __nv_bfloat16*)x,                       \
         (const __nv_bfloat16*)branch, (const __nv_bfloat16*)gate, (const __nv_bfloat16*)scale, mean, rstd,      \
         (__nv_bfloat16*)dx, (__nv_bfloat16*)dbranch, partials, cols, rows_per_batch)
     if (has_gate) {
         if (threads <= 512) LN_BWD(true, 512);
         else LN_BWD(true, 1024);
+    } else if (xhat) {
+        if (threads <= 512) LN_BWD(false, 512, true);
+        else LN_BWD(false, 1024, true);
     } else {
         if (threads <= 512) LN_BWD(false, 512);
         else LN_BWD(false, 1024);
@@ -898,11 +954,27 @@ extern "C" int tt_ln_mod_bwd(const void* dy, const void* dres_in, const void* x,
     TT_CHECK_LAUNCH();
     }
     const int K = has_gate ? 3 : 2;
-    dim3 fgrid((cols + 255) / 256, K, batch);
-    column_finalize_kernel<<<fgrid, 256, 0, st>>>(partials, (__nv_bfloat16*)dscale, (__nv_bfloat16*)dshift,
-                                                  (__nv_bfloat16*)dgate, K, nblk_used, cols);
+    launch_finalize(partials, dscale, dshift, dgate, K, nblk_used, cols, batch, st);
     TT_CHECK_LAUNCH();
     return TT_OK;
+}
+
+}  // namespace
+
+extern "C" int tt_ln_mod_bwd(const void* dy, const void* dres_in, const void* x, const void* branch,
+                             const void* gate, const void* scale, const float* mean, const float* rstd, void* dx,
+                             void* dbranch, float* partials, void* dscale, void* dshift, void* dgate, long rows,
+                             int cols, long rows_per_batch, void* stream) {
+    return ln_mod_bwd(dy, dres_in, x, branch, gate, scale, mean, rstd, dx, dbranch, partials, dscale, dshift, dgate, rows, cols,
+                      rows_per_batch, false, stream);
+}
+
+// fused_adaln backward from the saved normalised rows: dx = rstd (dy (1 + scale) - mean(..) - xn mean(.. xn)), column sums of
+// dy xn and dy.  partials: 2 * cols * tt_norm_partial_blocks(rows, 1) floats
+extern "C" int tt_adaln_bwd(const void* dy, const void* xn, const void* scale, const float* rstd, void* dx, float* partials,
+                            void* dscale, void* dshift, long rows, int cols, void* stream) {
+    return ln_mod_bwd(dy, nullptr, xn, nullptr, nullptr, scale, nullptr, rstd, dx, nullptr, partials, dscale, dshift, nullptr, rows, cols,
+                      rows, true, stream);
 }
 
 extern "C" int tt_gate_residual_fwd(const void* res, const void* branch, const void* gate, void* out, long rows,
@@ -930,8 +1002,7 @@ extern "C" int tt_gate_residual_bwd(const void* dout, const void* branch, const 
         (const __nv_bfloat16*)dout, (const __nv_bfloat16*)branch, (const __nv_bfloat16*)gate, (__nv_bfloat16*)dbranch,
         partials, cols, rows_per_batch);
     TT_CHECK_LAUNCH();
-    column_finalize_kernel<<<dim3((cols + 255) / 256, 1, batch), 256, 0, st>>>(partials, (__nv_bfloat16*)dgate, nullptr,
-                                                                             nullptr, 1, nblk, cols);
+    launch_finalize(partials, dgate, nullptr, nullptr, 1, nblk, cols, batch, st);
     TT_CHECK_LAUNCH();
     return TT_OK;
 }
@@ -970,6 +1041,15 @@ extern "C" int tt_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd
 }
 
 namespace {
+// Partial rows of the RMSNorm backward, at most `limit`: a CTA of the short-row kernel takes 8 warps x 4 x (32 / lanes per
+// row) >= 32 rows at a time, and one without rows would only add zeros for the finalize pass to read.
+int rmsnorm_bwd_blocks(long rows, int cols, int limit) {
+    if (cols > 256) return limit;
+    const int nvec = cols >> 3, lpr = nvec <= 4 ? 4 : nvec <= 8 ? 8 : nvec <= 16 ? 16 : 32;
+    const long need = (rows + 32 * (32 / lpr) - 1) / (32 * (32 / lpr));
+    return (int)(need < limit ? need : limit);
+}
+
 // first pass of the RMSNorm backward into `nblk` partial rows: rows-per-warp kernel for short rows, CTA-per-row otherwise
 void launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* partials,
                         long rows, int cols, int nblk, cudaStream_t st) {
@@ -993,11 +1073,10 @@ extern "C" int tt_rmsnorm_bwd(const void* dy, const void* x, const void* w, cons
                               float* partials, void* dw, long rows, int cols, void* stream) {
     if (bad_cols(cols) || rows <= 0) return TT_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
-    const int nblk = pick_blocks(rows, 1);
+    const int nblk = rmsnorm_bwd_blocks(rows, cols, pick_blocks(rows, 1));
     launch_rmsnorm_bwd(dy, x, w, rstd, dx, partials, rows, cols, nblk, st);
     TT_CHECK_LAUNCH();
-    column_finalize_kernel<<<dim3((cols + 255) / 256, 1, 1), 256, 0, st>>>(partials, (__nv_bfloat16*)dw, nullptr, nullptr,
-                                                                         1, nblk, cols);
+    launch_finalize(partials, dw, nullptr, nullptr, 1, nblk, cols, 1, st);
     TT_CHECK_LAUNCH();
     return TT_OK;
 }
@@ -1039,13 +1118,13 @@ extern "C" int tt_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void*
     if (rc != TT_OK) return rc;
     int nblk = pick_blocks(rows, 1);
     if (nblk > TT_NOALLOC_MAX_BLOCKS) nblk = TT_NOALLOC_MAX_BLOCKS;
+    nblk = rmsnorm_bwd_blocks(rows, cols, nblk);
     cudaStream_t st = (cudaStream_t)stream;
     // every one of the nblk partial rows is fully rewritten by its block before the finalize pass reads it,
     // so nothing left behind by an earlier call can leak into this one
     launch_rmsnorm_bwd(dy, x, w, rstd, dx, partials, rows, cols, nblk, st);
     TT_CHECK_LAUNCH();
-    column_finalize_kernel<<<dim3((cols + 255) / 256, 1, 1), 256, 0, st>>>(partials, (__nv_bfloat16*)dw, nullptr, nullptr,
-                                                                         1, nblk, cols);
+    launch_finalize(partials, dw, nullptr, nullptr, 1, nblk, cols, 1, st);
     TT_CHECK_LAUNCH();
     return TT_OK;
 }

@@ -29,6 +29,11 @@ int tt_ln_mod_fwd(const void* x, const void* branch, const void* gate, const voi
 int tt_ln_mod_bwd(const void* dy, const void* dres_in, const void* x, const void* branch, const void* gate,
                   const void* scale, const float* mean, const float* rstd, void* dx, void* dbranch, float* partials,
                   void* dscale, void* dshift, void* dgate, long rows, int cols, long rows_per_batch, void* stream);
+/* the drop-in fused_adaln pair: normalised rows saved in place of the mean; partials as for tt_ln_mod_bwd with batch 1 */
+int tt_adaln_fwd(const void* x, const void* scale, const void* shift, void* y, void* xn, float* rstd, long rows, int cols,
+                 float eps, void* stream);
+int tt_adaln_bwd(const void* dy, const void* xn, const void* scale, const float* rstd, void* dx, float* partials, void* dscale,
+                 void* dshift, long rows, int cols, void* stream);
 int tt_gate_residual_fwd(const void* res, const void* branch, const void* gate, void* out, long rows, int cols,
                          long rows_per_batch, void* stream);
 int tt_gate_residual_bwd(const void* dout, const void* branch, const void* gate, void* dbranch, float* partials,

@@ -19,23 +19,29 @@ def torch_launch_adaln_forward(out, x, scale, shift, x_norm, invvar, rows: int, 
     for t, n in ((out, "out"), (x, "x"), (scale, "scale"), (shift, "shift"), (x_norm, "x_norm")):
         check(t, BF16, n)
     check(invvar, torch.float32, "invvar")
-    if x.numel() != rows * cols or scale.numel() != cols or shift.numel() != cols:
+    if x.numel() != rows * cols or scale.numel() != cols or shift.numel() != cols or x_norm.numel() != rows * cols:
         raise _lib.NativeError("shape mismatch")
-    mean = torch.empty(rows, dtype=torch.float32, device=x.device)
-    call("tt_ln_mod_fwd", ptr(x), ptr(None), ptr(None), ptr(scale), ptr(shift), ptr(None), ptr(out), ptr(mean), ptr(invvar),
-         c_long(rows), c_int(cols), c_long(rows), c_float(eps), stream())
-    x_norm.copy_(((x.float().view(rows, cols) - mean[:, None]) * invvar[:, None]).to(BF16).view_as(x_norm))
+    _check_rows(invvar, rows, cols, out)
+    call("tt_adaln_fwd", ptr(x), ptr(scale), ptr(shift), ptr(out), ptr(x_norm), ptr(invvar), c_long(rows), c_int(cols), c_float(eps),
+         stream())
+
+
+def _check_rows(invvar, rows, cols, *full):
+    """One statistic per row, and whole [rows, cols] buffers behind every pointer the kernels walk."""
+    if invvar.numel() != rows or (invvar.dim() != 1 and rows != 1):
+        raise _lib.NativeError("invvar: expected one value per row")
+    if any(t.numel() < rows * cols for t in full):
+        raise _lib.NativeError("shape mismatch")
 
 
 def torch_launch_adaln_backward(dx, dscale, dshift, dout, x_norm, scale, invvar, rows: int, cols: int):
     for t, n in ((dx, "dx"), (dscale, "dscale"), (dshift, "dshift"), (dout, "dout"), (x_norm, "x_norm"), (scale, "scale")):
         check(t, BF16, n)
     check(invvar, torch.float32, "invvar")
-    # x_norm is already normalised: feed it as the input with mean 0 and rstd 1, then apply the saved rstd
-    zeros = torch.zeros(rows, dtype=torch.float32, device=dx.device)
-    ones = torch.ones(rows, dtype=torch.float32, device=dx.device)
+    if dx.numel() != rows * cols or min(scale.numel(), dscale.numel(), dshift.numel()) < cols:
+        raise _lib.NativeError("shape mismatch")
+    _check_rows(invvar, rows, cols, dout, x_norm)
     nblk = _lib.lib().tt_norm_partial_blocks(c_long(rows), c_int(1))
     partials = torch.empty(nblk * 2 * cols, dtype=torch.float32, device=dx.device)
-    call("tt_ln_mod_bwd", ptr(dout), ptr(None), ptr(x_norm), ptr(None), ptr(None), ptr(scale), ptr(zeros), ptr(ones), ptr(dx),
-         ptr(None), ptr(partials), ptr(dscale), ptr(dshift), ptr(None), c_long(rows), c_int(cols), c_long(rows), stream())
-    dx.copy_((dx.float().view(rows, cols) * invvar[:, None]).to(BF16).view_as(dx))
+    call("tt_adaln_bwd", ptr(dout), ptr(x_norm), ptr(scale), ptr(invvar), ptr(dx), ptr(partials), ptr(dscale), ptr(dshift),
+         c_long(rows), c_int(cols), stream())

@@ -280,3 +280,30 @@ def test_flow_noise_mix_and_loss_with_gradient():
     assert _rel(pred.grad, ref_pred.grad) < 6e-3
     # same bits on a second run: the partial sums are added in a fixed order
     assert float(ops.flow_match_loss(pred.detach(), noise, lat, weight)) == float(loss)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 264), (5, 3072), (257, 3072), (593, 1024), (40, 6144), (19, 6152), (9, 8192)])
+def test_drop_in_adaln_saves_and_consumes_normalised_rows(rows, cols):
+    """Fewer rows than a batch of four, ragged row batches, the last width of the shared-memory ring (6144) and the first of
+    the register kernel.  One bf16 rounding of each output against fp64: 2^-8 relative per element, half of it in norm."""
+    from teletron_b200.legacy import fused_adaln
+    g = torch.Generator(device="cuda").manual_seed(rows * 7 + cols)
+    rn = lambda *s, k=1.0: (torch.randn(*s, device=_dev(), generator=g) * k).bfloat16()  # noqa: E731
+    x, dy, scale, shift = rn(rows, cols) * 2 + 0.5, rn(rows, cols), rn(cols, k=0.3), rn(cols, k=0.3)
+    y, xn, dx = (torch.empty_like(x) for _ in range(3))
+    rstd = torch.empty(rows, device=_dev())
+    dscale, dshift = torch.empty_like(scale), torch.empty_like(scale)
+    fused_adaln.torch_launch_adaln_forward(y, x, scale, shift, xn, rstd, rows, cols)
+    fused_adaln.torch_launch_adaln_backward(dx, dscale, dshift, dy, xn, scale, rstd, rows, cols)
+    xd, dyd, sd = x.double(), dy.double(), scale.double()
+    rs = (xd.var(-1, unbiased=False, keepdim=True) + 1e-6).rsqrt()
+    xnd = (xd - xd.mean(-1, keepdim=True)) * rs
+    assert _rel(rstd, rs[:, 0]) < 1e-6
+    assert _rel(xn, xnd) < 4e-3 and _rel(y, xnd * (1 + sd) + shift.double()) < 4e-3
+    xq, gd = xn.double(), dyd * (1 + sd)        # the backward sees the rounded rows
+    dxd = rs * (gd - gd.mean(-1, keepdim=True) - xq * (gd * xq).mean(-1, keepdim=True))
+    # cols = 8: the bracket cancels to a part of its terms, so the fp32 sums count beside the rounding
+    assert _rel(dx, dxd) < 5e-3
+    assert _rel(dscale, (dyd * xq).sum(0)) < 4e-3 and _rel(dshift, dyd.sum(0)) < 4e-3
+    with pytest.raises(Exception):
+        fused_adaln.torch_launch_adaln_forward(y, x, scale, shift, xn, rstd[:-1] if rows > 1 else rstd[:0], rows, cols)
