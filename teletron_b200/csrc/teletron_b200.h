@@ -61,6 +61,9 @@ int tt_qkv_post_bwd_peer(void* const* dq_ptrs, void* const* dk_ptrs, void* const
 /* ---- activations ---- */
 int tt_gelu_fwd(const void* u, void* y, long n, int kind, void* stream);   /* kind 0 = erf, 1 = tanh */
 int tt_gelu_bwd(const void* dy, const void* u, void* du, long n, int kind, void* stream);
+/* bias gradient: column sums of dy (kind 2), or of du = dy * gelu'(u) (kind 0 / 1), which is written as well */
+int tt_colsum_groups(long rows, int cols);
+int tt_act_bwd_colsum(const void* dy, const void* u, void* du, float* partials, void* db, long rows, int cols, int kind, void* stream);
 
 /* ---- flow matching: noise mix and weighted MSE loss (+ its gradient) ---- */
 int tt_flow_loss_blocks(void);

@@ -210,6 +210,23 @@ def _gemm_tn(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     return gemm.gemm_tn(a, b)
 
 
+def _bias_grad(du: torch.Tensor) -> torch.Tensor:
+    """Column sums of ``du [rows, cols]`` in fp32, rounded once."""
+    rows, cols = du.shape
+    if cols % 8 or not du.is_contiguous() or du.dtype != BF16 or du.data_ptr() % 16 or rows == 0:
+        return du.sum(dim=0, dtype=torch.float32).to(du.dtype)
+    db = torch.empty(cols, dtype=BF16, device=du.device)
+    _colsum(du, None, None, db, rows, cols, 2)
+    return db
+
+
+def _colsum(dy, u, du, db, rows, cols, kind):
+    groups = _lib.lib().tt_colsum_groups(c_long(rows), c_int(cols))
+    partials = torch.empty(groups * cols, dtype=torch.float32, device=dy.device) if groups > 1 else None
+    call("tt_act_bwd_colsum", ptr(dy), ptr(u), ptr(du), ptr(partials), ptr(db), c_long(rows), c_int(cols), c_int(kind), stream())
+    _lib.LAUNCHES += groups > 1      # the finalize pass
+
+
 class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, activation):
@@ -237,6 +254,7 @@ class _Linear(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
+        db = None
         if ctx.activation is None:
             x2, weight = ctx.saved_tensors
             du = dy.reshape(-1, weight.shape[0])
@@ -246,10 +264,16 @@ class _Linear(torch.autograd.Function):
             x2, weight, u = ctx.saved_tensors
             dyc = check(dy.reshape(-1, weight.shape[0]).contiguous(), BF16, "dy")
             du = torch.empty_like(u)
-            call("tt_gelu_bwd", ptr(dyc), ptr(u), ptr(du), c_long(u.numel()), c_int(_GELU_KIND[ctx.activation]), stream())
+            rows, cols = u.shape
+            if ctx.has_bias and ctx.needs_input_grad[2] and cols % 8 == 0:
+                db = torch.empty(cols, dtype=BF16, device=u.device)     # bias gradient in the same pass
+                _colsum(dyc, u, du, db, rows, cols, _GELU_KIND[ctx.activation])
+            else:
+                call("tt_gelu_bwd", ptr(dyc), ptr(u), ptr(du), c_long(u.numel()), c_int(_GELU_KIND[ctx.activation]), stream())
         dx = _gemm_nn(du, weight) if ctx.needs_input_grad[0] else None
         dw = _gemm_tn(du, x2) if ctx.needs_input_grad[1] else None
-        db = du.sum(dim=0, dtype=torch.float32).to(du.dtype) if (ctx.has_bias and ctx.needs_input_grad[2]) else None
+        if db is None and ctx.has_bias and ctx.needs_input_grad[2]:
+            db = _bias_grad(du)
         if dx is not None:
             dx = dx.view(*dy.shape[:-1], weight.shape[1])
         return dx, dw, db, None
@@ -287,7 +311,7 @@ class _LinearMerged(torch.autograd.Function):
             dw = torch.empty_like(weight)
             gemm.gemm_tn_into(du, a1, dw[:, :k1])
             gemm.gemm_tn_into(du, a2, dw[:, k1:])
-        db = du.sum(dim=0, dtype=torch.float32).to(du.dtype) if (ctx.has_bias and ctx.needs_input_grad[3]) else None
+        db = _bias_grad(du) if (ctx.has_bias and ctx.needs_input_grad[3]) else None
         return d1, d2, dw, db
 
 
@@ -361,7 +385,7 @@ class _QKVProjection(torch.autograd.Function):
                  c_long(rows), c_int(heads), c_long(rows // B), c_long(S), c_long(off), c_long(rl), c_float(eps), stream())
             dx = _gemm_nn(dqkv, ws).view(B, -1, K)
             dw = _gemm_tn(dqkv, xs2)
-            db = dqkv.sum(dim=0, dtype=torch.float32).to(BF16) if hb else None
+            db = _bias_grad(dqkv) if hb else None
             outs.append((dx, dw, db, dqw, dkw))
         (dx1, dw1, db1, dqw1, dkw1), (dx2, dw2, db2, dqw2, dkw2) = outs
         return None, None, None, None, None, dx1, dw1, db1, dqw1, dkw1, dx2, dw2, db2, dqw2, dkw2

@@ -30,6 +30,7 @@ from ..parallel.symm_mem import SymmetricHeap
 from . import _lib, gemm
 from ._lib import c_float, c_int, c_long, check, ptr, stream
 from ._lib import call as _call
+from .cuda_ops import _bias_grad
 from .gemm_tcgen05 import status_tensor
 
 BF16 = torch.bfloat16
@@ -210,7 +211,7 @@ class _FusedQKVAllToAll(torch.autograd.Function):
                 dkw.mul_(scale)
             dx = gemm.gemm_nn(dqkv, ww)
             dw = gemm.gemm_tn(dqkv, xx)
-            db = dqkv.sum(dim=0, dtype=torch.float32).to(BF16) if hb else None
+            db = _bias_grad(dqkv) if hb else None
             outs.append((dx, dw, db, dqw, dkw))
         (dx, dw, db, dqw, dkw), (dxt, dwt, dbt, dqwt, dkwt) = outs
         xs, xts = ctx.shapes
@@ -289,8 +290,8 @@ class _FusedAllToAllLinear(torch.autograd.Function):
         at_full = at if ext is None else torch.cat([at, ext], dim=1)
         dw = gemm.gemm_tn(dy2, a_full)
         dwt = gemm.gemm_tn(dyt2, at_full)
-        db = dy2.sum(0, dtype=torch.float32).to(BF16) if hb else None
-        dbt = dyt2.sum(0, dtype=torch.float32).to(BF16) if hbt else None
+        db = _bias_grad(dy2) if hb else None
+        dbt = _bias_grad(dyt2) if hbt else None
         # data gradient: each head's columns go to the head's owner (sequence -> head all-to-all fused in the epilogue)
         K = w.shape[1]
         dex = torch.empty(ws.s, K - G, dtype=BF16, device=dev) if hex_ else None
@@ -405,8 +406,8 @@ class _FusedAttentionOutProj(torch.autograd.Function):
             gemm.gemm_tn_into(dy2, ex, dw[:, G:])
         if ext is not None:
             gemm.gemm_tn_into(dyt2, ext, dwt[:, G:])
-        db = dy2.sum(0, dtype=torch.float32).to(BF16) if ctx.has[0] else None
-        dbt = dyt2.sum(0, dtype=torch.float32).to(BF16) if ctx.has[1] else None
+        db = _bias_grad(dy2) if ctx.has[0] else None
+        dbt = _bias_grad(dyt2) if ctx.has[1] else None
         # data gradient of the video rows: every head's columns are pushed to the head's owner by the GEMM epilogue
         dex = torch.empty(s, K - G, dtype=BF16, device=dev) if ex is not None else None
         ws.heap.barrier()                  # peers are done reading the previous contents of `do`
@@ -593,7 +594,7 @@ class _SPColumnLinear(torch.autograd.Function):
             call("tt_gelu_bwd", ptr(dy), ptr(u), ptr(du), c_long(u.numel()), c_int(_GELU_KIND[ctx.activation]), stream())
         dx = _gemm_rs(ctx.ws, du, w, 1) if ctx.needs_input_grad[1] else None
         dw = gemm.gemm_tn(du, xg) if ctx.needs_input_grad[2] else None
-        db = du.sum(dim=0, dtype=torch.float32).to(BF16) if (ctx.has_bias and ctx.needs_input_grad[3]) else None
+        db = _bias_grad(du) if (ctx.has_bias and ctx.needs_input_grad[3]) else None
         return None, dx, dw, db, None
 
 
@@ -615,7 +616,7 @@ class _SPRowLinear(torch.autograd.Function):
         dy = check(dy.contiguous(), BF16, "dy")
         dx, dyg = _ag_gemm(ctx.ws, dy, w, None, 1)
         dw = gemm.gemm_tn(dyg, x) if ctx.needs_input_grad[2] else None
-        db = dy.sum(dim=0, dtype=torch.float32).to(BF16) if (ctx.has_bias and ctx.needs_input_grad[3]) else None
+        db = _bias_grad(dy) if (ctx.has_bias and ctx.needs_input_grad[3]) else None
         return None, dx, dw, db
 
 

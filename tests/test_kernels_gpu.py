@@ -307,3 +307,26 @@ def test_drop_in_adaln_saves_and_consumes_normalised_rows(rows, cols):
     assert _rel(dscale, (dyd * xq).sum(0)) < 4e-3 and _rel(dshift, dyd.sum(0)) < 4e-3
     with pytest.raises(Exception):
         fused_adaln.torch_launch_adaln_forward(y, x, scale, shift, xn, rstd[:-1] if rows > 1 else rstd[:0], rows, cols)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (31, 256), (33, 264), (257, 3072), (1037, 9216), (5000, 64)])
+@pytest.mark.parametrize("act", [None, "gelu", "gelu_tanh"])
+def test_bias_gradient_column_sums(rows, cols, act):
+    """One row group and several, ragged rows and columns; with an activation the sums are those of the rounded du."""
+    from teletron_b200.ops import cuda_ops
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    dy = torch.randn(rows, cols, device=_dev(), generator=g).bfloat16()
+    db = torch.full((cols,), float("nan"), device=_dev(), dtype=torch.bfloat16)
+    if act is None:
+        cuda_ops._colsum(dy, None, None, db, rows, cols, 2)
+        du = dy
+    else:
+        u = (torch.randn(rows, cols, device=_dev(), generator=g) * 2).bfloat16()
+        du = torch.empty_like(u)
+        cuda_ops._colsum(dy, u, du, db, rows, cols, cuda_ops._GELU_KIND[act])
+        ud = u.double().requires_grad_()
+        torch.nn.functional.gelu(ud, approximate="tanh" if act == "gelu_tanh" else "none").backward(dy.double())
+        assert _rel(du, ud.grad) < 4e-3
+    want = du.double().sum(0)
+    # one bf16 rounding of the sum plus fp32 summation error, which is relative to the sum of magnitudes
+    assert ((db.double() - want).abs() <= want.abs() * 2.0 ** -8 + du.double().abs().sum(0) * 2e-6).all()
