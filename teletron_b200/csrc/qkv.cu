@@ -251,26 +251,31 @@ __global__ void __launch_bounds__(256, 3) qkv_post_bwd_kernel(
     }
 }
 
-__global__ void __launch_bounds__(1024) qkv_weight_finalize_kernel(const float* __restrict__ partials,
-                                                                   __nv_bfloat16* __restrict__ dqw,
-                                                                   __nv_bfloat16* __restrict__ dkw, int nparts) {
-    // One block (fixed summation order => deterministic).  1024 threads = 4 row groups x 256 columns; every thread
-    // keeps 8 independent loads in flight, then the 4 groups are folded through shared memory in a fixed order.
-    __shared__ float fold[4][256];
-    const int c = threadIdx.x & 255, g = threadIdx.x >> 8;
-    float acc[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) acc[u] = 0.f;
+// Sums the partial rows.  A CTA owns 16 of the 256 columns, 64 threads a column, four independent loads each, so a
+// thread's chain of dependent loads is nparts / 256 long; the fold through shared memory has a fixed order (deterministic).
+// One CTA for all columns, four threads a column, took 53 us for the 4736 rows of a whole grid: more than the pass itself
+// on a short sequence; this takes 10 us.
+constexpr int kFinCols = 16, kFinRows = 64;
+
+__global__ void __launch_bounds__(kFinCols * kFinRows) qkv_weight_finalize_kernel(const float* __restrict__ partials,
+                                                                                  __nv_bfloat16* __restrict__ dqw,
+                                                                                  __nv_bfloat16* __restrict__ dkw, int nparts) {
+    __shared__ float fold[kFinRows][kFinCols + 1];
+    const int cl = threadIdx.x % kFinCols, g = threadIdx.x / kFinCols;
+    const int c = blockIdx.x * kFinCols + cl;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
     int i = g;
-    for (; i + 28 < nparts; i += 32) {
+    for (; i + 3 * kFinRows < nparts; i += 4 * kFinRows) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) acc[u] += partials[(long)(i + 4 * u) * 256 + c];
+        for (int u = 0; u < 4; ++u) acc[u] += partials[(long)(i + u * kFinRows) * 256 + c];
     }
-    for (; i < nparts; i += 4) acc[0] += partials[(long)i * 256 + c];
-    fold[g][c] = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+    for (; i < nparts; i += kFinRows) acc[0] += partials[(long)i * 256 + c];
+    fold[g][cl] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
     __syncthreads();
     if (g == 0) {
-        const float s = (fold[0][c] + fold[1][c]) + (fold[2][c] + fold[3][c]);
+        float s = 0.f;
+#pragma unroll 8
+        for (int r = 0; r < kFinRows; ++r) s += fold[r][cl];
         if (c < D) dqw[c] = __float2bfloat16(s);
         else dkw[c - D] = __float2bfloat16(s);
     }
@@ -321,7 +326,7 @@ extern "C" int tt_qkv_post_bwd_peer(void* const* dq_ptrs, void* const* dk_ptrs, 
                                               (const __nv_bfloat16*)kw, cos_t, sin_t, (__nv_bfloat16*)dqkv, partials,
                                               rows, heads, seq_in, seq_out, out_offset, rope_len, eps);
     TT_CHECK_LAUNCH();
-    qkv_weight_finalize_kernel<<<1, 1024, 0, st>>>(partials, (__nv_bfloat16*)dqw, (__nv_bfloat16*)dkw, grid * 8);
+    qkv_weight_finalize_kernel<<<256 / kFinCols, kFinCols * kFinRows, 0, st>>>(partials, (__nv_bfloat16*)dqw, (__nv_bfloat16*)dkw, grid * 8);
     TT_CHECK_LAUNCH();
     return TT_OK;
 }
