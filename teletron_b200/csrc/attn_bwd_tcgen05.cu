@@ -131,7 +131,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint32_t acc_final = s_full + 32u;
 
     static_assert(!(KVS && TSA), "the key-stationary kernel has no free tensor-memory columns");
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int bh = blockIdx.y;
     const int b = bh / p.H, head = bh - b * p.H;
     const int r0 = blockIdx.x * BS;                                     // first stationary row
@@ -170,7 +170,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             if (!TSA) mbar_arrive_expect_tx(a_full, 2 * kTile);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -205,7 +205,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_t = idesc_bf16(BS, BC, false, false);   // T = A B^T, both K-major
             constexpr uint32_t idesc_a = idesc_bf16(BS, D, false, true);     // acc += P B, B MN-major
             // T[128 x 128] = stationary (K-major) x chunk^T (K-major): eight K = 16 steps over the head dim
@@ -470,49 +470,61 @@ done:
 
 // ---------------------------------------------------------------------------------------------------------------
 // One-pass variant: the key-stationary kernel also forms this chunk's dQ contribution, so S and dP are computed once
-// (five products per [128 x 128] tile pair instead of seven).  dS is written twice by the softmax warps: as bf16 pairs
-// into tensor memory (the A operand of dK += dS^T Q, as above) and into a shared-memory tile laid out [key][query]
-// with 128-byte swizzle, which the tensor core reads MN-major as the A operand of dQ(c) = dS(c) K.  That product lands
-// in T2 once dK(c) / dV(c) have consumed the bf16 P / dS there (the tensor core executes in issue order); the softmax
-// warps read it back and add it to an fp32 [B*H, s_pad, 128] accumulator in global memory with vector reductions
-// (every key tile of a head adds into the same rows: the order of those additions is not fixed, so dQ is reproducible
-// only to fp32 rounding).  A last elementwise kernel scales and rounds the accumulator to bf16.
+// (five products per [128 x 128] tile pair instead of seven).  bf16 P overwrites the scores in T1 and feeds dV from there.
+// dS is written twice by the softmax warps: as bf16 pairs over dP in T2 (the A operand of dK += dS^T Q) and into a
+// shared-memory tile laid out [key][query] with 128-byte swizzle, which the tensor core reads MN-major as the A operand
+// of dQ(c) = dS(c) K.  That product lands in T2 once dK(c) has consumed the bf16 dS there (the tensor core executes in
+// issue order); the softmax warps read it back and add it to an fp32 [B*H, s_pad, 128] accumulator in global memory with
+// TMA reductions (every key tile of a head adds into the same rows: the order of those additions is not fixed, so dQ is
+// reproducible only to fp32 rounding).  A last elementwise kernel scales and rounds the accumulator to bf16.
 //
-//   tensor core:  dP(c) S(c+1) ............ | dK(c) dV(c) dQ(c) | dP(c+1) S(c+2) ...
-//   softmax:      readout(c-1) | dS(c) .... | P(c+1) .......... | readout(c) | dS(c+1) ...
+//   tensor core:  dK(c) dQ(c) ..... | ............... | dP(c+1) dV(c+1) S(c+2) .. | dK(c+1) dQ(c+1) ...
+//   softmax:      P(c+1) .......... | readout dQ(c) . | (dP(c+1)) dS(c+1) ....... | P(c+2) ...
 //
-// Shared memory: K, V resident; two slots each for the streamed Q and dO; one dS tile (same 225 KB as above).
+// What bounds it is a chain through T2 and the dS tile: dS -> dK, dQ -> read-out -> the staged half leaves the dS tile ->
+// next dS (~4500 clocks a chunk; shared memory moves 480 KB a chunk, 3750 clocks at 128 bytes each, the tensor core needs
+// 2560).  So everything else is kept off it: dV takes P from T1, where it waits for nothing but the exponentials; dP(c+1) is
+// issued the moment dQ(c) has been read; S(c+2) follows dV(c+1) into T1 before dS(c+1) is through; lse and delta arrive
+// in shared memory with their chunk (from L2 they cost ~500 clocks a pass); the MMA warp issues from one elected lane
+// (200 clocks for eight products instead of 650).  24 heads x 32656 tokens: 36.2 -> 33.1 ms, 3 heads x 119056: 62.5 -> 56.4.
+//
+// Shared memory: K, V resident; two slots each for the streamed Q (with the chunk's lse) and dO (with its delta); one dS tile.
 constexpr int kFRing = 2;
-constexpr int kFSmemBytes = (2 + 2 * kFRing + 1) * kTile + 256 + 1024;
+constexpr int kFStatBytes = 2 * BC * 4;      // lse and delta of one chunk
+constexpr int kFSmemBytes = (2 + 2 * kFRing + 1) * kTile + 256 /* barriers, flags */ + kFRing * kFStatBytes;
 
-// TMA reduction shared -> global: adds the [32 x 32] fp32 box at `smem_src` (128-byte swizzle) into the tensor at (x, y)
-__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* tmap, uint32_t smem_src, int x, int y) {
-    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                     (uint64_t)tmap),
-                 "r"(smem_src), "r"(x), "r"(y)
+// dQ accumulator: per 128-query chunk two halves (column groups 0, 1 and 2, 3) of 32 KB, each the byte image of its staging
+// buffer: [quad][group & 1][lane] rows of 32 floats whose 16-byte pieces are XOR-swizzled by the lane.  The accumulator is
+// scratch that only dq_finish_kernel reads, so its layout is free, and with this one a half leaves as one contiguous bulk
+// reduction.  It drains at 25 bytes per clock and SM, as tensor boxes do, so 64 KB a chunk take 2600 clocks; red.v4 straight from
+// registers is no faster (27) and holds up the softmax warps' other accesses (39.8 ms at 24 heads x 32656 against 36.4).
+constexpr int kHalfFloats = 64 * 128;
+__device__ __forceinline__ void bulk_reduce_add(float* dst, uint32_t smem_src, uint32_t bytes) {
+    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(smem_src), "r"(bytes)
                  : "memory");
 }
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read_but_last() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 constexpr int kFThreads = kThreads + 32;     // one more warp: issues the dQ reductions and waits for them
 __global__ void __launch_bounds__(kFThreads, 1)
 attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                      const __grid_constant__ CUtensorMap tmDQ, const BwdParams p) {
-    extern __shared__ uint8_t smem_raw[];
-    __shared__ volatile int abort_flag;
-    __shared__ uint32_t tmem_base_slot;
+                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO, const BwdParams p) {
+    // 226 KB of the 227 a CTA can have: the tiles' 1024-byte alignment comes from the declaration, without slack
+    extern __shared__ __align__(1024) uint8_t fused_smem[];
+    volatile int& abort_flag = *reinterpret_cast<volatile int*>(fused_smem + (2 + 2 * kFRing + 1) * kTile + 248);
+    uint32_t& tmem_base_slot = *reinterpret_cast<uint32_t*>(fused_smem + (2 + 2 * kFRing + 1) * kTile + 252);
 
-    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t base = smem_u32(fused_smem);
+    if (base & 1023u) {
+        if (threadIdx.x == 0) atomicExch(p.status, TT_ERR_ARG);
+        return;
+    }
     const uint32_t sA1 = base;                       // K tile
     const uint32_t sA2 = base + kTile;               // V tile
     const uint32_t sRing1 = base + 2 * kTile;        // Q chunks
     const uint32_t sRing2 = sRing1 + kFRing * kTile; // dO chunks
     const uint32_t sDS = sRing2 + kFRing * kTile;    // dS of the current chunk, [key][query] bf16
     const uint32_t bars = sDS + kTile;
+    const uint32_t sStat = bars + 256u;              // per slot: lse [128], delta [128]
     const uint32_t a_full = bars;
     auto b1_full = [&](int s) { return bars + 8u * (1 + s); };
     auto b1_empty = [&](int s) { return bars + 8u * (1 + kFRing + s); };
@@ -520,8 +532,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     auto b2_empty = [&](int s) { return bars + 8u * (1 + 3 * kFRing + s); };
     const uint32_t s_full = bars + 8u * (1 + 4 * kFRing);
     const uint32_t dp_full = s_full + 8u;
-    const uint32_t p_ready = s_full + 16u;
-    const uint32_t ds_ready = s_full + 24u;
+    const uint32_t p_ready = s_full + 16u;           // every softmax warp has written P over its part of S in T1
+    const uint32_t ds_ready = s_full + 24u;          // dS is in T2 and in the dS tile
     const uint32_t dq_full = s_full + 32u;           // T2 holds dQ(c)
     const uint32_t dq_read = s_full + 40u;           // every softmax warp has read dQ(c) out of T2
     const uint32_t acc_final = s_full + 48u;
@@ -529,7 +541,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const uint32_t staged_a = s_full + 64u;          // column groups 0, 1 of dQ(c) are in the dS tile
     const uint32_t staged_b = s_full + 72u;          // column groups 2, 3 of dQ(c) are in chunk c's dO slot
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int bh = blockIdx.y;
     const int b = bh / p.H, head = bh - b * p.H;
     const int r0 = blockIdx.x * BS;                  // first key of this CTA
@@ -546,7 +558,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             mbar_init(b1_full(s), 1);
             mbar_init(b1_empty(s), 1);
             mbar_init(b2_full(s), 1);
-            mbar_init(b2_empty(s), 2);     // dV(c) has read the slot + the dQ half staged in it afterwards has left
+            mbar_init(b2_empty(s), 2);     // dV(c), dP(c) have read the slot + the dQ half staged in it afterwards has left
         }
         mbar_init(s_full, 1);
         mbar_init(dp_full, 1);
@@ -573,7 +585,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_arrive_expect_tx(a_full, 2 * kTile);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -585,12 +597,17 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 const uint32_t wpar = ((uint32_t)(c / kFRing) & 1u) ^ 1u;
                 if (!mbar_wait(b1_empty(s), wpar, &abort_flag)) goto done;
                 TT_STAMPF(15);
-                mbar_arrive_expect_tx(b1_full(s), kTile);
+                // the rows of the statistics are `pitch` (a multiple of 64) long: the last chunk may have half of them
+                const uint32_t stat_bytes = 4u * (uint32_t)min(BC, p.pitch - chunk_of(c) * BC);
+                const long stat_at = (long)bh * p.pitch + chunk_of(c) * BC;
+                mbar_arrive_expect_tx(b1_full(s), kTile + stat_bytes);
+                bulk_load_1d(sStat + s * kFStatBytes, p.lse + stat_at, stat_bytes, b1_full(s));
 #pragma unroll
                 for (int h = 0; h < 2; ++h) tma_load_3d(sRing1 + s * kTile + h * kSlab, &tmQ, b1_full(s), h * 64, chunk_of(c) * BC, bh);
                 if (!mbar_wait(b2_empty(s), wpar, &abort_flag)) goto done;
                 TT_STAMPF(14);
-                mbar_arrive_expect_tx(b2_full(s), kTile);
+                mbar_arrive_expect_tx(b2_full(s), kTile + stat_bytes);
+                bulk_load_1d(sStat + s * kFStatBytes + BC * 4, p.delta + stat_at, stat_bytes, b2_full(s));
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
                     tma_load_4d(sRing2 + s * kTile + h * kSlab, &tmDO, b2_full(s), h * 64, head, chunk_of(c) * BC, b);
@@ -598,7 +615,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_t = idesc_bf16(BS, BC, false, false);   // T = A B^T, both K-major
             constexpr uint32_t idesc_a = idesc_bf16(BS, D, false, true);     // acc += (tensor-memory A) B, B MN-major
             constexpr uint32_t idesc_q = idesc_bf16(BC, D, true, true);      // dQ = dS K: both operands MN-major
@@ -625,42 +642,52 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             tc_fence_after();
             issue_t(kT2, sA2, sRing2);
             umma_commit(dp_full);
+            if (!mbar_wait(p_ready, 0, &abort_flag)) goto done;
+            tc_fence_after();
+            issue_acc(kAccV, kT1, sRing2, true);
+            umma_commit(b2_empty(0));
+            if (n_chunks > 1) {
+                if (!mbar_wait(b1_full(1 % kFRing), (uint32_t)(1 / kFRing) & 1u, &abort_flag)) goto done;
+                tc_fence_after();
+                issue_t(kT1, sA1, sRing1 + (1 % kFRing) * kTile);
+                umma_commit(s_full);
+            }
             for (int c = 0; c < n_chunks; ++c) {
                 const uint32_t par = (uint32_t)c & 1u;
                 const bool more = c + 1 < n_chunks;
                 const int slot = c % kFRing, nslot = (c + 1) % kFRing;
                 const uint32_t npar = (uint32_t)((c + 1) / kFRing) & 1u;
                 TT_STAMPF(0);
-                if (!mbar_wait(p_ready, par, &abort_flag)) goto done;              // S(c) has been read: T1 is free
+                if (!mbar_wait(ds_ready, par, &abort_flag)) goto done;             // dS in T2 and in shared memory
                 TT_STAMPF(1);
                 tc_fence_after();
-                if (more) {
-                    if (!mbar_wait(b1_full(nslot), npar, &abort_flag)) goto done;
-                    tc_fence_after();
-                    issue_t(kT1, sA1, sRing1 + nslot * kTile);                     // S(c+1)
-                    umma_commit(s_full);
-                }
-                if (!mbar_wait(ds_ready, par, &abort_flag)) goto done;             // P, dS in T2; dS in shared memory
-                TT_STAMPF(2);
-                tc_fence_after();
-                issue_acc(kAccK, kT2 + 16, sRing1 + slot * kTile, c == 0);          // dK += dS^T Q
+                issue_acc(kAccK, kT2, sRing1 + slot * kTile, c == 0);               // dK += dS^T Q
                 umma_commit(b1_empty(slot));
-                issue_acc(kAccV, kT2, sRing2 + slot * kTile, c == 0);               // dV += P^T dO
-                umma_commit(b2_empty(slot));
 #pragma unroll
                 for (int kk = 0; kk < BS / 16; ++kk)                                // dQ(c) = dS K over the 128 keys, into T2
                     umma_bf16_ss(tmem + kT2, smem_desc_sw128(sDS + kk * 2048, kSlab, 1024),
                                  smem_desc_sw128(sA1 + kk * 2048, kSlab, 1024), idesc_q, kk ? 1u : 0u);
                 umma_commit(dq_full);
-                TT_STAMPF(3);
                 if (more) {
-                    if (!mbar_wait(dq_read, par, &abort_flag)) goto done;          // dQ(c) is in registers: T2 is free
-                    TT_STAMPF(4);
                     if (!mbar_wait(b2_full(nslot), npar, &abort_flag)) goto done;
                     TT_STAMPF(10);
+                    if (!mbar_wait(dq_read, par, &abort_flag)) goto done;          // dQ(c) is in registers: T2 is free
+                    TT_STAMPF(4);
                     tc_fence_after();
-                    issue_t(kT2, sA2, sRing2 + nslot * kTile);                     // dP(c+1)
+                    issue_t(kT2, sA2, sRing2 + nslot * kTile);                     // dP(c+1): heads the chain to dS(c+1)
                     umma_commit(dp_full);
+                    if (!mbar_wait(p_ready, par ^ 1u, &abort_flag)) goto done;      // P(c+1) in T1
+                    TT_STAMPF(2);
+                    tc_fence_after();
+                    issue_acc(kAccV, kT1, sRing2 + nslot * kTile, false);           // dV += P^T dO
+                    umma_commit(b2_empty(nslot));
+                    TT_STAMPF(3);
+                    if (c + 2 < n_chunks) {                                        // S(c+2): T1 is free once dV(c+1) has read P
+                        if (!mbar_wait(b1_full(slot), (uint32_t)((c + 2) / kFRing) & 1u, &abort_flag)) goto done;
+                        tc_fence_after();
+                        issue_t(kT1, sA1, sRing1 + slot * kTile);
+                        umma_commit(s_full);
+                    }
                 }
             }
             umma_commit(acc_final);
@@ -668,33 +695,25 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     } else if (warp == 2 + 4 * kGroups) {
         // ------------------------------------------------------------ dQ reductions
         // dQ(c) is staged by the softmax warps in two halves of eight [32 x 32] fp32 boxes: column groups 0, 1 in the dS
-        // tile (idle until the next chunk's dS is stored), groups 2, 3 in chunk c's dO slot (dV(c) has consumed it; the
+        // tile (idle until the next chunk's dS is stored), groups 2, 3 in chunk c's dO slot (dV(c) and dP(c) have consumed it; the
         // producer refills it only after this thread has released it).  The first half is issued first, so it leaves
         // first; both drain while the next chunk is computed.  A thread of its own waits for the TMA unit, so that no
         // softmax warp ever does.
-        if (lane == 0) {
+        if (elect_one()) {
             for (int c = 0; c < n_chunks; ++c) {
                 const uint32_t par = (uint32_t)c & 1u;
-                const int yrow = bh * p.s_pad + chunk_of(c) * BC;
+                float* acc = p.dq_acc + ((long)bh * p.s_pad + chunk_of(c) * BC) * D;
                 if (!mbar_wait(staged_a, par, &abort_flag)) goto done;
                 TT_STAMPF(11);
-#ifndef TT_FUSED_NO_RED
-#pragma unroll
-                for (int g = 0; g < 8; ++g) tma_reduce_add_2d(&tmDQ, sDS + ((uint32_t)g << 12), (g & 1) * kCols, yrow + (g >> 1) * 32);
-#endif
+                bulk_reduce_add(acc, sDS, kHalfFloats * 4);
                 bulk_commit();
                 if (!mbar_wait(staged_b, par, &abort_flag)) goto done;
-#ifndef TT_FUSED_NO_RED
-                const uint32_t slot = sRing2 + (uint32_t)(c % kFRing) * kTile;
-#pragma unroll
-                for (int g = 0; g < 8; ++g)
-                    tma_reduce_add_2d(&tmDQ, slot + ((uint32_t)g << 12), (2 + (g & 1)) * kCols, yrow + (g >> 1) * 32);
-#endif
+                bulk_reduce_add(acc + kHalfFloats, sRing2 + (uint32_t)(c % kFRing) * kTile, kHalfFloats * 4);
                 bulk_commit();
-                bulk_wait_read_but_last();
+                bulk_wait_read<1>();
                 TT_STAMPF(12);
                 mbar_arrive(stage_done);
-                bulk_wait_read();
+                bulk_wait_read<0>();
                 TT_STAMPF(13);
                 mbar_arrive(b2_empty(c % kFRing));
             }
@@ -708,7 +727,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const int row = r0 + srow;
         const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
         const float c_log2 = p.scale * kLog2e;
-        const bool row_live = row < p.kv_len && !(row >= p.mask_lo && row < p.mask_hi);
+        const uint32_t live_mask = row < p.kv_len && !(row >= p.mask_lo && row < p.mask_hi) ? 0xffffffffu : 0u;
         const uint32_t t1 = tmem + lane_sel + kT1 + part * kCols, t2 = tmem + lane_sel + kT2 + part * kCols;
         // this thread's 64 bytes of the dS tile: row srow of slab (part >> 1), 16-byte chunks 4 (part & 1) + 0..3, swizzled
         const uint32_t ds_row = sDS + (uint32_t)(part >> 1) * kSlab + (uint32_t)srow * 128u;
@@ -717,29 +736,32 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         // this warp's 4 KB of the dQ staging: groups 0, 1 in the dS tile, groups 2, 3 in the chunk's dO slot
         const uint32_t stage_off = ((uint32_t)(quad * 2 + (part & 1)) << 12) + (uint32_t)lane * 128u;
 
+        // statistics of columns [8 i', 8 i' + 4) ... of this thread's 32 columns of chunk c (columns beyond the padded row: `pad`)
+        auto stat4 = [&](int c, int which, int i, float pad) {
+            float4 v;
+            const uint32_t a = sStat + (uint32_t)(c % kFRing) * kFStatBytes + (uint32_t)(which * BC + part * kCols + i * 4) * 4u;
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+            return chunk_of(c) * BC + part * kCols < p.pitch ? v : make_float4(pad, pad, pad, pad);
+        };
         auto p_pass = [&](int c) -> bool {
-            const int col0 = chunk_of(c) * BC + part * kCols;
-            const bool cols_ok = col0 < p.pitch;
-            const float4* lse4 = reinterpret_cast<const float4*>(p.lse + (long)bh * p.pitch + col0);
+            if (!mbar_wait(b1_full(c % kFRing), (uint32_t)(c / kFRing) & 1u, &abort_flag)) return false;      // lse(c)
             if (!mbar_wait(s_full, (uint32_t)c & 1u, &abort_flag)) return false;
             tc_fence_after();
             uint32_t a[32];
             tmem_ld_32x32(t1, a);
-            float4 lq[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) lq[i] = cols_ok ? __ldg(lse4 + i) : make_float4(INFINITY, INFINITY, INFINITY, INFINITY);
+            float4 lv;
             tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-                const float4 lv = lq[i >> 1];
-                const float2 l2 = (i & 1) ? make_float2(lv.z * kLog2e, lv.w * kLog2e) : make_float2(lv.x * kLog2e, lv.y * kLog2e);
+                if ((i & 1) == 0) lv = stat4(c, 0, i >> 1, INFINITY);
+                const float2 nl2 = __fmul2_rn((i & 1) ? make_float2(lv.z, lv.w) : make_float2(lv.x, lv.y), make_float2(-kLog2e, -kLog2e));
                 const float2 x = __ffma2_rn(make_float2(__uint_as_float(a[2 * i]), __uint_as_float(a[2 * i + 1])),
-                                            make_float2(c_log2, c_log2), make_float2(-l2.x, -l2.y));
-                float2 pr = make_float2(exp2f(x.x), exp2f(x.y));
-                if (!row_live) pr = make_float2(0.f, 0.f);
-                const __nv_bfloat162 pb = __floats2bfloat162_rn(pr.x, pr.y);
-                pk[i] = *reinterpret_cast<const uint32_t*>(&pb);
+                                            make_float2(c_log2, c_log2), nl2);
+                const __nv_bfloat162 pb = __floats2bfloat162_rn(exp2f(x.x), exp2f(x.y));
+                pk[i] = *reinterpret_cast<const uint32_t*>(&pb) & live_mask;     // masked keys: 0, whatever their score
             }
+            tmem_st_32x16(t1, pk);             // bf16 P over the scores just read: the A operand of dV += P^T dO
+            tmem_st_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(p_ready);
@@ -749,10 +771,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (!p_pass(0)) goto done;
         for (int c = 0; c < n_chunks; ++c) {
             const uint32_t par = (uint32_t)c & 1u;
-            const int col0 = chunk_of(c) * BC + part * kCols;
-            const bool cols_ok = col0 < p.pitch;
-            const float4* del4 = reinterpret_cast<const float4*>(p.delta + (long)bh * p.pitch + col0);
             // ---- dS(c) from dP(c) and the P kept in registers
+            if (!mbar_wait(b2_full(c % kFRing), (uint32_t)(c / kFRing) & 1u, &abort_flag)) goto done;            // delta(c)
             if (!mbar_wait(dp_full, par, &abort_flag)) goto done;
             if (threadIdx.x == 64) TT_STAMPF(5);
             tc_fence_after();
@@ -760,23 +780,20 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             {
                 uint32_t g[32];
                 tmem_ld_32x32(t2, g);
-                float4 dq4[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) dq4[i] = cols_ok ? __ldg(del4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 dv;
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const float4 dv = dq4[i >> 1];
+                    if ((i & 1) == 0) dv = stat4(c, 1, i >> 1, 0.f);
                     const float2 d2 = (i & 1) ? make_float2(dv.z, dv.w) : make_float2(dv.x, dv.y);
                     const float2 pr = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[i]));
-                    const float2 dp = make_float2(__uint_as_float(g[2 * i]) - d2.x, __uint_as_float(g[2 * i + 1]) - d2.y);
+                    const float2 dp = __ffma2_rn(d2, make_float2(-1.f, -1.f), make_float2(__uint_as_float(g[2 * i]), __uint_as_float(g[2 * i + 1])));
                     const float2 ds = __fmul2_rn(pr, dp);
                     const __nv_bfloat162 db = __floats2bfloat162_rn(ds.x, ds.y);
                     dk[i] = *reinterpret_cast<const uint32_t*>(&db);
                 }
             }
-            tmem_st_32x16(t2, pk);
-            tmem_st_32x16(t2 + 16, dk);
+            tmem_st_32x16(t2, dk);
             // the dS tile doubles as a staging buffer of the previous chunk's dQ read-out: wait until that has left
             if (c > 0 && !mbar_wait(stage_done, (uint32_t)(c - 1) & 1u, &abort_flag)) goto done;
 #pragma unroll
@@ -805,6 +822,9 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(dq_read);
+            // groups 2, 3 leave the shared-memory write path to groups 0, 1 first: the half in the dS tile is the one the next
+            // chunk waits for, so it is complete, and on its way out, as early as possible
+            if (part >= 2 && !mbar_wait(staged_a, par, &abort_flag)) goto done;
             {
                 const uint32_t mine = (part < 2 ? sDS : sRing2 + (uint32_t)(c % kFRing) * kTile) + stage_off;
 #pragma unroll
@@ -864,8 +884,12 @@ __global__ void __launch_bounds__(256) dq_finish_kernel(const float* __restrict_
         const long rowi = i / (D / 8);
         const int c8 = (int)(i - rowi * (D / 8));
         const long bhi = rowi / S, s = rowi - bhi * S;
-        const float4* src = reinterpret_cast<const float4*>(acc + (bhi * s_pad + s) * D + c8 * 8);
-        const float4 x = __ldg(src), y = __ldg(src + 1);
+        // row r of its chunk, columns [8 c8, 8 c8 + 8): 16-byte pieces 2 (c8 & 3) and 2 (c8 & 3) + 1 of group c8 >> 2
+        const int r = (int)(s & (BC - 1)), lane = r & 31, grp = c8 >> 2;
+        const float4* src = reinterpret_cast<const float4*>(acc + (bhi * s_pad + s - r) * D + (grp >> 1) * kHalfFloats +
+                                                            (((r >> 5) * 2 + (grp & 1)) << 10) + lane * 32);
+        const int j = (c8 & 3) * 2;
+        const float4 x = __ldg(src + (j ^ (lane & 7))), y = __ldg(src + ((j + 1) ^ (lane & 7)));
         float o[8] = {x.x * scale, x.y * scale, x.z * scale, x.w * scale, y.x * scale, y.y * scale, y.z * scale, y.w * scale};
         tt::st8(dq + rowi * D + c8 * 8, tt::pack8(o));
     }
@@ -979,18 +1003,6 @@ extern "C" int tt_attn_bwd_fused(const void* q, const void* k, const void* v, co
         if (e != cudaSuccess) return tt_record_cuda(e);
         configured_dev[dev] = true;
     }
-    CUtensorMap tdq;      // fp32 [B*H*s_pad, 128], boxes of 32 rows x 32 columns (128 bytes), 128-byte swizzle
-    {
-        tt_encode_tiled_fn enc = tt_get_encode_tiled();
-        if (enc == nullptr) return TT_ERR_CUDA;
-        cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)(BH * (uint64_t)s_pad)};
-        cuuint64_t strides[1] = {(cuuint64_t)D * sizeof(float)};
-        cuuint32_t box[2] = {32, 32};
-        cuuint32_t estr[2] = {1, 1};
-        if (enc(&tdq, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, dq_acc, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return TT_ERR_ARG;
-    }
     cudaError_t e = cudaMemsetAsync(dq_acc, 0, BH * (uint64_t)s_pad * D * sizeof(float), st);
     if (e != cudaSuccess) return tt_record_cuda(e);
     const long nwork = (long)B * S * H;
@@ -1018,7 +1030,7 @@ extern "C" int tt_attn_bwd_fused(const void* q, const void* k, const void* v, co
 #endif
     p.out1 = (__nv_bfloat16*)dv;
     p.out2 = (__nv_bfloat16*)dk;
-    attn_bwd_fused_kernel<<<dim3((S + BS - 1) / BS, (unsigned)BH), kFThreads, kFSmemBytes, st>>>(tq_s, tk_s, tv_s, tdo_s, tdq, p);
+    attn_bwd_fused_kernel<<<dim3((S + BS - 1) / BS, (unsigned)BH), kFThreads, kFSmemBytes, st>>>(tq_s, tk_s, tv_s, tdo_s, p);
     TT_CHECK_LAUNCH();
     const long n8 = (long)BH * S * (D / 8);
     long blocks = (n8 + 255) / 256;

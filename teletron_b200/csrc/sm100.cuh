@@ -14,6 +14,19 @@ namespace sm100 {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// One lane of a converged warp.  Unlike `lane == 0` this tells the compiler that the branch is taken by a single thread, so
+// the operands of the tensor-core and TMA instructions inside stay in uniform registers instead of being moved there before
+// every instruction.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(p));
+    return p != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -88,6 +101,39 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t smem_dst, const void* gmem
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_dst),
                  "l"(gmem_src), "r"(bytes), "r"(bar)
                  : "memory");
+}
+// 2-D tiled store shared -> global (rows and columns beyond the tensor are clipped; coordinates are never negative)
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* tmap, uint32_t smem_src, int c0, int c1) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"((uint64_t)tmap), "r"(smem_src),
+                 "r"(c0), "r"(c1)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// at most N of this thread's bulk groups have not been read out of shared memory yet
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+// Epilogue store of one warp's 32 rows x 64 columns of bf16 through a 4 KB box in shared memory (1024-byte aligned, 128-byte
+// rows, 16-byte pieces XOR-swizzled by row as SWIZZLE_128B expects; lane = row).  `o(g, f)` yields columns [8 g, 8 g + 8).
+template <typename F>
+__device__ __forceinline__ void store_box_32x64(uint32_t box, const CUtensorMap* tmap, int col, int row, int lane, F&& o) {
+    // two boxes per warp: the group before last, which used this one, has been read
+    if (lane == 0) bulk_wait_read<1>();
+    __syncwarp();
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+        const uint4 u = o(g);
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(box + (uint32_t)lane * 128u + (uint32_t)((g ^ (lane & 7)) << 4)), "r"(u.x),
+                     "r"(u.y), "r"(u.z), "r"(u.w)
+                     : "memory");
+    }
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) {
+        tma_store_2d(tmap, box, col, row);
+        bulk_commit();
+    }
 }
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {
     asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)tmap) : "memory");

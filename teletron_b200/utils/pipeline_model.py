@@ -5,8 +5,8 @@ The kernel has five kinds of actors that only meet at mbarriers: the TMA-issuing
 softmax warps (modelled as two groups of eight: column groups 0, 1 and 2, 3), the thread that issues and awaits the dQ
 reductions, and the two asynchronous units they feed - the tensor core, which executes what it is given in issue order
 and signals through commits, and the TMA unit, whose pending copies may complete in any order.  Buffers are reused
-aggressively: T1 holds S, T2 holds dP, then bf16 P / dS, then dQ; the dS tile and each chunk's dO slot double as staging
-buffers for the reductions.  The model gives every buffer a content tag and the set of readers that still need it, and
+aggressively: T1 holds S, then bf16 P; T2 holds dP, then bf16 dS, then dQ; the dS tile and each chunk's dO slot double as
+staging buffers for the reductions.  The model gives every buffer a content tag and the set of readers that still need it, and
 reports
 
 * a read that finds something else than the tag it expects,
@@ -50,9 +50,9 @@ def _tc_effect(op: Tuple, n: int):
     if kind == "dP":
         return ([("KV", "KV", None), (f"do{s}", ("dO", c), "dP")], [("T2a", ("dP", c), {"smA"}), ("T2b", ("dP", c), {"smB"})], [])
     if kind == "dK":
-        return ([("T2a", ("PdS", c), "dK"), ("T2b", ("PdS", c), "dK"), (f"q{s}", ("Q", c), "dK")], [], [])
+        return ([("T2a", ("dS", c), "dK"), ("T2b", ("dS", c), "dK"), (f"q{s}", ("Q", c), "dK")], [], [])
     if kind == "dV":
-        return ([("T2a", ("PdS", c), "dV"), ("T2b", ("PdS", c), "dV"), (f"do{s}", ("dO", c), "dV")], [], [])
+        return ([("T1a", ("P", c), "dV"), ("T1b", ("P", c), "dV"), (f"do{s}", ("dO", c), "dV")], [], [])
     if kind == "dQ":
         return ([("dsA", ("dS", c), "dQ"), ("dsB", ("dS", c), "dQ"), ("KV", "KV", None)],
                 [("T2a", ("dQ", c), {"smA"}), ("T2b", ("dQ", c), {"smB"})], [])
@@ -65,9 +65,9 @@ def _tma_effect(op: Tuple):
     if kind == "loadKV":
         return ([], [("KV", "KV", set())], [("a_full", 1)])
     if kind == "loadQ":
-        return ([], [(f"q{s}", ("Q", c), {"S", "dK"})], [(f"b1_full{s}", 1)])
+        return ([], [(f"q{s}", ("Q", c), {"S", "dK"}), (f"lse{s}", ("lse", c), {"smA", "smB"})], [(f"b1_full{s}", 1)])
     if kind == "loadDO":
-        return ([], [(f"do{s}", ("dO", c), {"dP", "dV"})], [(f"b2_full{s}", 1)])
+        return ([], [(f"do{s}", ("dO", c), {"dP", "dV"}), (f"delta{s}", ("delta", c), {"smA", "smB"})], [(f"b2_full{s}", 1)])
     if kind == "redA":
         return ([("dsA", ("stage", c), "redA"), ("dsB", ("stage", c), "redA")], [], [])
     if kind == "redB":
@@ -87,19 +87,25 @@ def _producer(n: int) -> List[Tuple]:
 
 def _mma(n: int, v: Variant) -> List[Tuple]:
     ops: List[Tuple] = [("wait", "a_full", 0), ("wait", "b1_full0", 0), ("tc", ("S", 0)), ("tc", ("commit", "s_full")),
-                        ("wait", "b2_full0", 0), ("tc", ("dP", 0)), ("tc", ("commit", "dp_full"))]
+                        ("wait", "b2_full0", 0), ("tc", ("dP", 0)), ("tc", ("commit", "dp_full")), ("wait", "p_ready", 0),
+                        ("tc", ("dV", 0)), ("tc", ("commit", "b2_empty0"))]
+
+    def scores(c):
+        s = c % RING
+        return [("wait", f"b1_full{s}", (c // RING) & 1), ("tc", ("S", c)), ("tc", ("commit", "s_full"))] if c < n else []
+
+    ops += scores(1)
     for c in range(n):
         par, more = c & 1, c + 1 < n
         s, ns, npar = c % RING, (c + 1) % RING, ((c + 1) // RING) & 1
-        ops.append(("wait", "p_ready", par))
+        ops += [("wait", "ds_ready", par), ("tc", ("dK", c)), ("tc", ("commit", f"b1_empty{s}")), ("tc", ("dQ", c)),
+                ("tc", ("commit", "dq_full"))]
         if more:
-            ops += [("wait", f"b1_full{ns}", npar), ("tc", ("S", c + 1)), ("tc", ("commit", "s_full"))]
-        ops += [("wait", "ds_ready", par), ("tc", ("dK", c)), ("tc", ("commit", f"b1_empty{s}")), ("tc", ("dV", c)),
-                ("tc", ("commit", f"b2_empty{s}")), ("tc", ("dQ", c)), ("tc", ("commit", "dq_full"))]
-        if more:
+            ops.append(("wait", f"b2_full{ns}", npar))
             if v.wait_dq_read:
                 ops.append(("wait", "dq_read", par))
-            ops += [("wait", f"b2_full{ns}", npar), ("tc", ("dP", c + 1)), ("tc", ("commit", "dp_full"))]
+            ops += [("tc", ("dP", c + 1)), ("tc", ("commit", "dp_full")), ("wait", "p_ready", par ^ 1), ("tc", ("dV", c + 1)),
+                    ("tc", ("commit", f"b2_empty{ns}"))] + scores(c + 2)
     ops.append(("tc", ("commit", "acc_final")))
     return ops
 
@@ -109,12 +115,14 @@ def _softmax(n: int, g: str, v: Variant) -> List[Tuple]:
     me, t1, t2, ds = "sm" + g, "T1" + g.lower(), "T2" + g.lower(), "ds" + g
 
     def p_pass(c):
-        return [("wait", "s_full", c & 1), ("read", t1, ("S", c), me), ("arrive", "p_ready", 8)]
+        return [("wait", f"b1_full{c % RING}", (c // RING) & 1), ("wait", "s_full", c & 1), ("read", f"lse{c % RING}", ("lse", c), me),
+                ("read", t1, ("S", c), me), ("write", t1, ("P", c), ("dV",)), ("arrive", "p_ready", 8)]
 
     ops: List[Tuple] = p_pass(0)
     for c in range(n):
         par = c & 1
-        ops += [("wait", "dp_full", par), ("read", t2, ("dP", c), me), ("write", t2, ("PdS", c), ("dK", "dV"))]
+        ops += [("wait", f"b2_full{c % RING}", (c // RING) & 1), ("wait", "dp_full", par), ("read", f"delta{c % RING}", ("delta", c), me),
+                ("read", t2, ("dP", c), me), ("write", t2, ("dS", c), ("dK",))]
         if c > 0 and v.wait_stage_done:
             ops.append(("wait", "stage_done", (c - 1) & 1))
         ops += [("write", ds, ("dS", c), ("dQ",)), ("arrive", "ds_ready", 8)]
@@ -124,7 +132,7 @@ def _softmax(n: int, g: str, v: Variant) -> List[Tuple]:
         if g == "A":       # column groups 0, 1 stage in the dS tile (all of it), groups 2, 3 in chunk c's dO slot
             ops += [("write", "dsA", ("stage", c), ("redA",)), ("write", "dsB", ("stage", c), ("redA",)), ("arrive", "staged_a", 8)]
         else:
-            ops += [("write", f"do{c % RING}", ("stage", c), ("redB",)), ("arrive", "staged_b", 8)]
+            ops += [("wait", "staged_a", par), ("write", f"do{c % RING}", ("stage", c), ("redB",)), ("arrive", "staged_b", 8)]
     ops.append(("wait", "acc_final", 0))
     return ops
 
@@ -163,7 +171,7 @@ def explore(chunks: int = 3, variant: Variant = Variant(), max_states: int = 3_0
     counts = _barriers()
     bar_names = sorted(counts)
     bidx = {b: i for i, b in enumerate(bar_names)}
-    buf_names = ["KV", "T1a", "T1b", "T2a", "T2b", "dsA", "dsB"] + [f"q{s}" for s in range(RING)] + [f"do{s}" for s in range(RING)]
+    buf_names = ["KV", "T1a", "T1b", "T2a", "T2b", "dsA", "dsB"] + [f"{b}{s}" for b in ("q", "do", "lse", "delta") for s in range(RING)]
     fidx = {b: i for i, b in enumerate(buf_names)}
     violations = set()
 
