@@ -71,6 +71,7 @@ struct GemmParams {
     const float* cos_t;
     const float* sin_t;
     float eps;
+    int tma_store;          // EPI 0 - 4, local C with whole 32-row groups per segment: the epilogue stores through tmC / tmAux
     int rope_len, heads_per_rank, s_in, s_out, out_off, only_local;
     int coalesce;           // pushed tiles: stage each warp's 32 x 128 block in shared memory, store whole 256-byte rows
     __nv_bfloat16* peer_q[TT_MAX_PEERS];
@@ -85,7 +86,8 @@ struct Cfg {
     static constexpr int kBBytes = BN * BK * 2;
     static constexpr int kStageBytes = kABytes + kBBytes;
     static constexpr int kTmemCols = 2 * BN;
-    static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /* alignment slack */ + 256 /* barriers */;
+    static constexpr int kEpiBytes = 4 * 8192;      // epilogue staging: 8 KB per warp
+    static constexpr int kSmemBytes = kStages * kStageBytes + kEpiBytes + 1024 /* alignment slack */ + 256 /* barriers */;
 };
 
 template <int EPI>
@@ -108,7 +110,8 @@ __device__ __forceinline__ void st_release(int* p, int v) {
 
 template <int BN, bool A_MN, bool B_MN, int EPI, bool STAGE = false>
 __global__ void __launch_bounds__(STAGE ? kThreads + 128 : kThreads, 1)
-gemm_kernel(const __grid_constant__ TmapArray tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
+gemm_kernel(const __grid_constant__ TmapArray tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
+            const __grid_constant__ CUtensorMap tmAux, const GemmParams p) {
     using C = Cfg<BN>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ volatile int abort_flag;
@@ -116,14 +119,14 @@ gemm_kernel(const __grid_constant__ TmapArray tmA, const __grid_constant__ CUten
 
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
-    const uint32_t bar_base = base + C::kStages * C::kStageBytes;
+    const uint32_t epi_stage = base + C::kStages * C::kStageBytes;       // 4 epilogue warps x 8 KB
+    const uint32_t bar_base = epi_stage + C::kEpiBytes;
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
     auto empty_bar = [&](int s) { return bar_base + 8u * (C::kStages + s); };
     auto tfull_bar = [&](int b) { return bar_base + 8u * (2 * C::kStages + b); };
     auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * C::kStages + 2 + b); };
-    const uint32_t epi_stage = bar_base + 256u;      // coalesced peer stores: 4 warps x 8 KB (only when launched with room for it)
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         abort_flag = 0;
         for (int s = 0; s < C::kStages; ++s) {
@@ -168,7 +171,7 @@ gemm_kernel(const __grid_constant__ TmapArray tmA, const __grid_constant__ CUten
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
@@ -236,7 +239,7 @@ gemm_kernel(const __grid_constant__ TmapArray tmA, const __grid_constant__ CUten
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_bf16(BM, BN, A_MN, B_MN);
             int stage = 0;
             uint32_t phase = 0;
@@ -492,6 +495,35 @@ gemm_kernel(const __grid_constant__ TmapArray tmA, const __grid_constant__ CUten
                         }
                         store_block_coalesced(v, d, min(128, p.N - colb));
                     }
+                } else if (EPI <= 4 && p.tma_store) {
+                    const int row0 = seg * p.seg_rows + m0 + quad * 32;
+                    const uint32_t box = epi_stage + (uint32_t)(warp - 2) * 8192u;
+                    if (m0 + quad * 32 < p.seg_rows)
+#pragma unroll 1
+                    for (int c = 0; c < BN / 64; ++c) {
+                        const int col0 = n0 + c * 64;
+                        if (col0 >= p.N || row0 >= p.M) break;
+                        uint32_t r[64];
+                        tmem_ld_32x32(tacc + c * 64, r);
+                        tmem_ld_32x32(tacc + c * 64 + 32, r + 32);
+                        tmem_ld_wait();
+                        auto packed = [&](int g, bool pre) -> uint4 {
+                            const int col = col0 + g * 8;
+                            float bv[8], uv[8], o[8];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) bv[j] = uv[j] = 0.f;
+                            if (EPI <= 2 && p.bias != nullptr && col + 8 <= p.N) tt::unpack8(tt::ld8(p.bias + col), bv);
+                            if (EPI >= 3 && row_ok && col + 8 <= p.N) tt::unpack8(tt::ld8(arow + col), uv);
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                o[j] = pre ? __uint_as_float(r[g * 8 + j]) + bv[j] : epi_apply<EPI>(__uint_as_float(r[g * 8 + j]), bv[j], uv[j]);
+                            const tt::bf16x8 pk = tt::pack8(o);
+                            return *reinterpret_cast<const uint4*>(&pk);
+                        };
+                        if (EPI == 1 || EPI == 2) store_box_32x64(box, &tmAux, col0, row0, lane, [&](int g) { return packed(g, true); });
+                        store_box_32x64(box + ((EPI == 1 || EPI == 2 || (c & 1)) ? 4096u : 0u), &tmC, col0, row0, lane,
+                                        [&](int g) { return packed(g, false); });
+                    }
                 } else
 #pragma unroll 1
                 for (int c = 0; c < BN / 32; ++c) {
@@ -525,6 +557,7 @@ gemm_kernel(const __grid_constant__ TmapArray tmA, const __grid_constant__ CUten
             __syncwarp();
             if (lane == 0) mbar_arrive(tempty_bar(buf));
         }
+        if (lane == 0) bulk_wait_read<0>();        // the boxes outlive the copies that read them
     }
 
 done:
@@ -542,12 +575,20 @@ done:
 }
 
 template <int BN, bool A_MN, bool B_MN, int EPI, bool STAGE = false>
-int launch(const TmapArray& tmA, const CUtensorMap& tmB, const GemmParams& p, int sms, cudaStream_t st) {
+int launch(const TmapArray& tmA, const CUtensorMap& tmB, GemmParams p, int sms, cudaStream_t st) {
     using C = Cfg<BN>;
+    CUtensorMap tmC, tmAux;
+    memset(&tmC, 0, sizeof(tmC));
+    memset(&tmAux, 0, sizeof(tmAux));
+    // 32-row boxes may run past the last row of the tensor, where they are clipped, but not into another segment
+    p.tma_store = EPI <= 4 && p.store_mode == 0 && (p.n_seg == 1 || p.seg_rows % 32 == 0);
+    if (p.tma_store) {
+        int rc = tt_make_tmap_2d(&tmC, p.C, (uint64_t)p.M, (uint64_t)p.N, (uint64_t)p.ldc, 32, 64);
+        if (rc == TT_OK && (EPI == 1 || EPI == 2)) rc = tt_make_tmap_2d(&tmAux, p.aux, (uint64_t)p.M, (uint64_t)p.N, (uint64_t)p.ldc, 32, 64);
+        if (rc != TT_OK) return rc;
+    }
     auto kern = gemm_kernel<BN, A_MN, B_MN, EPI, STAGE>;
-    // staging for the coalesced peer stores (4 epilogue warps x 8 KB), only when that variant is selected
-    const bool staged_stores = EPI == 6 || EPI == 5;
-    const int smem = C::kSmemBytes + (staged_stores ? 4 * 8192 : 0);
+    const int smem = C::kSmemBytes;
     // the attribute belongs to the device's context: remembered per device, not per process
     static int configured[64] = {0};
     int dev = 0;
@@ -559,7 +600,7 @@ int launch(const TmapArray& tmA, const CUtensorMap& tmB, const GemmParams& p, in
     }
     const int tiles = p.tiles_m * p.tiles_n;
     const int grid = tiles < sms ? tiles : sms;
-    kern<<<grid, STAGE ? kThreads + 128 : kThreads, smem, st>>>(tmA, tmB, p);
+    kern<<<grid, STAGE ? kThreads + 128 : kThreads, smem, st>>>(tmA, tmB, tmC, tmAux, p);
     TT_CHECK_LAUNCH();
     return TT_OK;
 }
