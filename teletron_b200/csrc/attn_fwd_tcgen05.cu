@@ -9,6 +9,11 @@
 // (S = Q K^T with both operands from shared memory; O += P V with P read from tensor memory and V fed
 // as an MN-major shared-memory operand, so V is never transposed), warps 2-5 softmax of tile 0,
 // warps 6-9 softmax of tile 1 (one query row per thread).
+// What bounds it: per 128 keys and tile pair the tensor core, shared memory (Q, K, V operand reads and TMA writes at 128 bytes
+// per clock) and the special-function unit (16 exponentials per clock) each need 2048 clocks, so what counts is the
+// chain S -> softmax -> P V -> next S of a tile: the other tile covers only as much of it as it is itself busy.  Hence S is
+// read from tensor memory once, whole; the new maximum is found while the first exponentials run; and P V starts
+// when half of P is there.  24 heads x 32656 tokens: 11.1 -> 9.6 ms, 3 heads x 119056: 20.9 -> 17.9.
 // The running row maximum is only raised when it grows by more than 2^8 ("lazy rescale"), so O is
 // corrected in tensor memory on rare iterations only.
 //
@@ -75,10 +80,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     auto v_full = [&](int s) { return bars + 8u * (5 + s); };
     auto v_empty = [&](int s) { return bars + 8u * (7 + s); };
     auto s_full = [&](int t) { return bars + 8u * (9 + t); };
-    auto p_full = [&](int t) { return bars + 8u * (11 + t); };
-    const uint32_t o_final = bars + 8u * 13;
+    auto p_half = [&](int t, int h) { return bars + 8u * (11 + 2 * t + h); };     // keys [64 h, 64 h + 64) of P are in place
+    const uint32_t o_final = bars + 8u * 15;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int bh = blockIdx.y;                  // batch * H + head
     const int q0 = blockIdx.x * (2 * BQ);       // first query row of this CTA
     const int n_kv = (p.kv_len + BKV - 1) / BKV;
@@ -92,7 +97,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             mbar_init(v_full(s), 1);
             mbar_init(v_empty(s), 1);
             mbar_init(s_full(s), 1);
-            mbar_init(p_full(s), 4);
+            mbar_init(p_half(s, 0), 4);
+            mbar_init(p_half(s, 1), 4);
         }
         mbar_init(o_final, 1);
         fence_barrier_init();
@@ -112,7 +118,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_arrive_expect_tx(q_full, 2 * kTileBytes);
 #pragma unroll
             for (int t = 0; t < 2; ++t)
@@ -133,7 +139,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_s = idesc_bf16(BQ, BKV, false, false);   // S = Q K^T: both K-major
             constexpr uint32_t idesc_o = idesc_bf16(BQ, D, false, true);      // O += P V: V is MN-major
             auto issue_s = [&](int t, int stage) {
@@ -146,10 +152,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 }
                 umma_commit(s_full(t));
             };
-            auto issue_o = [&](int t, int stage, bool accumulate) {
+            auto issue_o = [&](int t, int stage, int half, bool accumulate) {
                 const uint32_t b = sV + stage * kTileBytes;
 #pragma unroll
-                for (int kk = 0; kk < BKV / 16; ++kk) {
+                for (int k4 = 0; k4 < BKV / 32; ++k4) {
+                    const int kk = half * (BKV / 32) + k4;
                     // P: 16 bf16 keys = 8 TMEM columns per step; V: 16 key rows = 2048 B per step, dims slabs 16 KB apart
                     umma_bf16_ts(tmem + 256 + t * 128, tmem + t * 128 + kk * 8, smem_desc_sw128(b + kk * 2048, kSlab, 1024),
                                  idesc_o, (accumulate || kk) ? 1u : 0u);
@@ -169,17 +176,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 const int s1 = (j + 1) & 1;
                 const uint32_t ph1 = (uint32_t)((j + 1) >> 1) & 1u;
                 if (!mbar_wait(v_full(s), ph, &abort_flag)) goto done;
-                if (!mbar_wait(p_full(0), pph, &abort_flag)) goto done;
-                tc_fence_after();
-                issue_o(0, s, j > 0);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (!mbar_wait(p_half(0, h), pph, &abort_flag)) goto done;
+                    tc_fence_after();
+                    issue_o(0, s, h, j > 0);
+                }
                 if (more) {
                     if (!mbar_wait(k_full(s1), ph1, &abort_flag)) goto done;
                     tc_fence_after();
                     issue_s(0, s1);
                 }
-                if (!mbar_wait(p_full(1), pph, &abort_flag)) goto done;
-                tc_fence_after();
-                issue_o(1, s, j > 0);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (!mbar_wait(p_half(1, h), pph, &abort_flag)) goto done;
+                    tc_fence_after();
+                    issue_o(1, s, h, j > 0);
+                }
                 umma_commit(v_empty(s));
                 if (more) {
                     issue_s(1, s1);
@@ -209,76 +222,79 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             const int lo = p.mask_lo - j * BKV, hi = p.mask_hi - j * BKV;      // and columns [lo, hi) of this tile
             const bool full_tile = valid >= BKV && (lo >= hi || hi <= 0 || lo >= BKV);
 #endif
-            // pass 1: row maximum (3-input max, four independent chains)
-            float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+            // The whole row of S goes into registers at once, which frees its TMEM columns for P.
+            uint32_t r[BKV];
 #pragma unroll
-            for (int c = 0; c < BKV / 32; ++c) {
-                uint32_t r[32];
-                tmem_ld_32x32(tS + c * 32, r);
-                tmem_ld_wait();
-                if (!full_tile) {
+            for (int c = 0; c < BKV / 32; ++c) tmem_ld_32x32(tS + c * 32, r + c * 32);
+            tmem_ld_wait();
+            if (!full_tile) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        if (c * 32 + i >= valid || (c * 32 + i >= lo && c * 32 + i < hi)) r[i] = 0xff800000u;      // -inf
-                }
-#pragma unroll
-                for (int i = 0; i < 32; i += 8) {
-                    mx0 = max3(mx0, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
-                    mx1 = max3(mx1, __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
-                    mx2 = max3(mx2, __uint_as_float(r[i + 4]), __uint_as_float(r[i + 5]));
-                    mx3 = max3(mx3, __uint_as_float(r[i + 6]), __uint_as_float(r[i + 7]));
-                }
+                for (int i = 0; i < BKV; ++i)
+                    if (i >= valid || (i >= lo && i < hi)) r[i] = 0xff800000u;      // -inf
             }
-            const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale_log2;
-            // lazy rescale of the accumulator
-            const bool grow = mx > m + kRescaleThreshold || j == 0;
-            if (j > 0 && __any_sync(0xffffffffu, grow)) {
-                const float alpha = grow ? exp2f(m - mx) : 1.f;
-                l *= alpha;
-#pragma unroll 1
-                for (int c = 0; c < D / 16; ++c) {
-                    uint32_t r[16];
-                    tmem_ld_32x16(tO + c * 16, r);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-                    tmem_st_32x16(tO + c * 16, r);
-                }
-                tmem_st_wait();
-            }
-            if (grow) m = mx;
-            // pass 2: P = exp2(s * scale - m) with packed fp32x2 arithmetic, row sum, bf16 pack, store over S
+            // 32 columns: P = exp2(s * scale - m) with packed fp32x2 arithmetic, row sum, bf16 pack, store over S
             const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
-            const float2 nm2 = make_float2(-m, -m);
             float2 sum2a = make_float2(0.f, 0.f), sum2b = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int c = 0; c < BKV / 32; ++c) {
-                uint32_t r[32];
-                tmem_ld_32x32(tS + c * 32, r);
-                tmem_ld_wait();
+            auto exp_cols = [&](int c) {
+                const float nm = m == -INFINITY ? 0.f : -m;         // no key seen so far: the scores are -inf and P is 0
+                const float2 nm2 = make_float2(nm, nm);
                 uint32_t pk[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const float2 x = __ffma2_rn(make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), sc2, nm2);
-                    float2 e = make_float2(exp2f(x.x), exp2f(x.y));
-                    if (!full_tile) {
-                        const int c0 = c * 32 + 2 * i;
-                        if (c0 >= valid || (c0 >= lo && c0 < hi)) e.x = 0.f;
-                        if (c0 + 1 >= valid || (c0 + 1 >= lo && c0 + 1 < hi)) e.y = 0.f;
-                    }
+                    const float2 x = __ffma2_rn(make_float2(__uint_as_float(r[c * 32 + 2 * i]), __uint_as_float(r[c * 32 + 2 * i + 1])), sc2, nm2);
+                    const float2 e = make_float2(exp2f(x.x), exp2f(x.y));
                     if (i & 1) sum2b = __fadd2_rn(sum2b, e);
                     else sum2a = __fadd2_rn(sum2a, e);
                     const __nv_bfloat162 b2 = __floats2bfloat162_rn(e.x, e.y);
                     pk[i] = *reinterpret_cast<const uint32_t*>(&b2);
                 }
                 tmem_st_32x16(tS + c * 16, pk);
+            };
+            // The first 32 exponentials use the running maximum as it stands, so that they keep the special-function unit
+            // busy while the row's new maximum (3-input max, four independent chains) is found; in the rare tile whose maximum
+            // grows by more than the threshold they are redone after the accumulator has been rescaled.
+            exp_cols(0);
+            float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < BKV; i += 8) {
+                mx0 = max3(mx0, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+                mx1 = max3(mx1, __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+                mx2 = max3(mx2, __uint_as_float(r[i + 4]), __uint_as_float(r[i + 5]));
+                mx3 = max3(mx3, __uint_as_float(r[i + 6]), __uint_as_float(r[i + 7]));
             }
-            const float sum = (sum2a.x + sum2a.y) + (sum2b.x + sum2b.y);
-            l += sum;
+            const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale_log2;
+            const bool grow = mx > m + kRescaleThreshold;           // always for the first visible key (m = -inf)
+            if (__any_sync(0xffffffffu, grow)) {
+                if (j > 0) {
+                    const float alpha = grow ? exp2f(m - mx) : 1.f;
+                    l *= alpha;
+#pragma unroll 1
+                    for (int c = 0; c < D / 16; ++c) {
+                        uint32_t o[16];
+                        tmem_ld_32x16(tO + c * 16, o);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        tmem_st_32x16(tO + c * 16, o);
+                    }
+                    tmem_st_wait();
+                }
+                if (grow) m = mx;
+                sum2a = sum2b = make_float2(0.f, 0.f);
+                exp_cols(0);
+            }
+            exp_cols(1);
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(p_full(t));
+            if (lane == 0) mbar_arrive(p_half(t, 0));               // P V over the first 64 keys can start
+            exp_cols(2);
+            exp_cols(3);
+            l += (sum2a.x + sum2a.y) + (sum2b.x + sum2b.y);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_half(t, 1));
         }
         // epilogue: O / l -> bf16, token-major store; log-sum-exp for the backward pass
         if (!mbar_wait(o_final, 0, &abort_flag)) goto done;

@@ -133,3 +133,24 @@ def test_forward_and_backward_are_bitwise_reproducible(bwd_variant):
                 else:
                     assert torch.equal(a, b)
     check_status()
+
+
+@pytest.mark.parametrize("S,kv_len,mask,ramp", [(640, None, (0, 200), 1.0), (900, 777, (0, 256), 6.0), (1100, 1090, (300, 520), 6.0),
+                                                (129, None, None, 1.0), (2049, None, None, 8.0)])
+def test_forward_running_maximum_with_masked_tiles(S, kv_len, mask, ramp):
+    """The first exponentials of a tile use the maximum before it: a first tile without a visible key, maxima that keep
+    growing (the redo path) before, inside and after masked tiles, and a last tile of one key."""
+    from teletron_b200.ops import attn_tcgen05 as A
+    from teletron_b200.ops import reference
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q = torch.randn(1, 2, S, 128, device="cuda", generator=g).bfloat16()
+    k = (torch.randn(1, 2, S, 128, device="cuda", generator=g) * torch.linspace(0.3, ramp, S, device="cuda").view(1, 1, S, 1)).bfloat16()
+    v = torch.randn(1, 2, S, 128, device="cuda", generator=g).bfloat16()
+    out, lse, *_ = A.forward(q, k, v, kv_len, None, mask)
+    ref = reference.attention(q.double(), k.double(), v.double(), kv_len, None, mask)
+    assert _rel(out, ref) < 1.2e-2
+    s = q.double() @ k.double().transpose(-1, -2) / math.sqrt(128)
+    s[..., kv_len or S:] = float("-inf")
+    if mask:
+        s[..., mask[0]:mask[1]] = float("-inf")
+    torch.testing.assert_close(lse[..., :S].double(), s.logsumexp(-1), rtol=1e-4, atol=1e-3)
