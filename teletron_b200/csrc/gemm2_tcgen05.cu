@@ -14,6 +14,10 @@
 //   tempty[b] in the leader: the four epilogue warps of both CTAs arrive (8 arrivals) once a buffer has been drained.
 // Tensor memory is allocated and freed by warp 1 of both CTAs (cta_group::2), the free after a cluster barrier.
 //
+// Split-K (tt_gemm2_bf16_splitk): a product with few tiles and a long K leaves most pairs idle, so the k-blocks of a tile are
+// shared by `splits` pairs; each writes its fp32 accumulator to its own slice of a scratch buffer (EPI 7) and a second kernel
+// adds the slices in a fixed order and applies the epilogue.
+//
 // Layouts and epilogues are those of gemm_tcgen05.cu (nt / nn / tn; bias, GELU erf / tanh with pre-activation,
 // GELU backward).  In the reference these products are TransformerEngine -> cuBLASLt calls
 // (teletron/models/dit/dit_attention.py:65-104, dit_layerspec.py:266-298, 438-445).
@@ -49,6 +53,8 @@ struct Params2 {
     __nv_bfloat16* aux;
     int* status;
     int tiles_m, tiles_n;       // in 256 x 256 tiles
+    int splits, kb_split;       // k-block ranges per tile, and their length
+    int part_rows;              // rows of one split's slice of the scratch buffer (M rounded up to whole 32-row boxes)
 };
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -150,9 +156,12 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_slot;
 
-    const int num_tiles = p.tiles_m * p.tiles_n;
+    const int num_tiles = p.tiles_m * p.tiles_n * p.splits;       // units of work: (tile, k-block range)
     const int kblocks = (p.K + BK - 1) / BK;
-    auto tile_coords = [&](int t, int& m0, int& n0) {
+    auto k_first = [&](int u) { return (u % p.splits) * p.kb_split; };
+    auto k_end = [&](int u) { return min(kblocks, (u % p.splits + 1) * p.kb_split); };
+    auto tile_coords = [&](int u, int& m0, int& n0) {
+        const int t = u / p.splits;
         const int per_group = kGroupM * p.tiles_n;
         const int g = t / per_group;
         const int first_m = g * kGroupM;
@@ -171,7 +180,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                 int m0, n0;
                 tile_coords(t, m0, n0);
                 const int am = m0 + (int)rank * BMH, bn = n0 + (int)rank * BNH;
-                for (int kb = 0; kb < kblocks; ++kb) {
+                const int kb1 = k_end(t);
+                for (int kb = k_first(t); kb < kb1; ++kb) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1u, &abort_flag)) goto done;
                     const uint32_t sa = base + stage * kStageBytes;
                     const uint32_t sb = sa + kABytes;
@@ -209,7 +219,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                 if (!mbar_wait(tempty_bar(buf), acc_phase ^ 1u, &abort_flag)) goto done;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
-                for (int kb = 0; kb < kblocks; ++kb) {
+                const int kb0 = k_first(t), kb1 = k_end(t);
+                for (int kb = kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(full_bar(stage), phase, &abort_flag)) goto done;
                     tc_fence_after();
                     const uint32_t sa = base + stage * kStageBytes;
@@ -218,7 +229,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                     for (int kk = 0; kk < BK / 16; ++kk) {
                         const uint64_t da = A_MN ? smem_desc_sw128(sa + kk * 2048, 8192, 1024) : smem_desc_sw128(sa + kk * 32, 16, 1024);
                         const uint64_t db = B_MN ? smem_desc_sw128(sb + kk * 2048, 8192, 1024) : smem_desc_sw128(sb + kk * 32, 16, 1024);
-                        umma2_bf16_ss(d_tmem, da, db, idesc, (kb | kk) ? 1u : 0u);
+                        umma2_bf16_ss(d_tmem, da, db, idesc, (kb > kb0 || kk) ? 1u : 0u);
                     }
                     umma2_commit_both(empty_bar(stage));        // frees this stage in both CTAs when the MMAs retire
                     if (++stage == kStages) {
@@ -244,11 +255,24 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
             const int row = row0 + lane;
             const bool row_ok = row < p.M;
             const uint32_t tacc = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * BN);
-            const __nv_bfloat16* arow = (EPI >= 3) ? p.aux + (long)row * p.ldc : nullptr;
+            const __nv_bfloat16* arow = (EPI == 3 || EPI == 4) ? p.aux + (long)row * p.ldc : nullptr;
             // Through shared memory and the TMA unit: a lane holds a row, so direct 16-byte stores touch 32 rows per instruction and
             // the epilogue of a tile, not its products, set the pace of short-K products (12288 x 3072 x 256, 75 MB written: 43.8 us direct, 25.2 us this way; 32656 x 12288 x 3072:
             // 1676 and 1625 us).
             const uint32_t box = epi_stage + (uint32_t)(warp - 2) * 8192u;
+            if (EPI == 7) {
+                const int prow = (t % p.splits) * p.part_rows + row0;
+#pragma unroll 1
+                for (int c = 0; c < BN / 32; ++c) {
+                    const int col0 = n0 + c * 32;
+                    if (col0 >= p.N || row0 >= p.M) break;
+                    uint32_t r[32];
+                    tmem_ld_32x32(tacc + c * 32, r);
+                    tmem_ld_wait();
+                    store_box_32x64(box + ((c & 1) ? 4096u : 0u), &tmC, col0, prow, lane,
+                                    [&](int g) { return make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]); });
+                }
+            } else
 #pragma unroll 1
             for (int c = 0; c < BN / 64; ++c) {
                 const int col0 = n0 + c * 64;
@@ -308,7 +332,7 @@ int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& t
         if (e != cudaSuccess) return tt_record_cuda(e);
         configured[dev] = true;
     }
-    const int tiles = p.tiles_m * p.tiles_n;
+    const int tiles = p.tiles_m * p.tiles_n * p.splits;
     int pairs = sms / 2;
     if (pairs > tiles) pairs = tiles;
     if (pairs < 1) pairs = 1;
@@ -317,20 +341,51 @@ int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& t
     return TT_OK;
 }
 
-}  // namespace
+// out = epilogue(sum of the splits' slices): 8 columns per thread, slices added in order
+template <int EPI>
+__global__ void __launch_bounds__(256) splitk_finish_kernel(const float* __restrict__ part, int splits, long slice, int M, int N, long ldc,
+                                                           const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ aux,
+                                                           __nv_bfloat16* __restrict__ C) {
+    const int nvec = N >> 3;
+    const long total = (long)M * nvec;
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+        const long row = i / nvec;
+        const int col = (int)(i - row * nvec) * 8;
+        const float* src = part + row * N + col;
+        float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int s = 0; s < splits; ++s) {
+            const float4 x = __ldcs(reinterpret_cast<const float4*>(src + s * slice)), y = __ldcs(reinterpret_cast<const float4*>(src + s * slice) + 1);
+            a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w;
+            a[4] += y.x; a[5] += y.y; a[6] += y.z; a[7] += y.w;
+        }
+        float bv[8], uv[8], o[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) bv[j] = uv[j] = 0.f;
+        if (EPI <= 2 && bias != nullptr) tt::unpack8(tt::ld8(bias + col), bv);
+        if (EPI >= 3) tt::unpack8(tt::ld8(aux + row * ldc + col), uv);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = epi2<EPI>(a[j], bv[j], uv[j]);
+        if (EPI == 1 || EPI == 2) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a[j] += bv[j];
+            tt::st8(aux + row * ldc + col, tt::pack8(a));
+        }
+        tt::st8(C + row * ldc + col, tt::pack8(o));
+    }
+}
 
-// Same contract as tt_gemm_bf16 (gemm_tcgen05.cu); returns TT_ERR_ARG for shapes this kernel does not take, so that the
-// caller can fall back to the single-CTA kernel.
-extern "C" int tt_gemm2_bf16(const void* a, const void* b, void* c, const void* bias, void* aux, int M, int N, int K,
-                             long lda, long ldb, long ldc, int a_mn, int b_mn, int epi, int* status, void* stream) {
+// What both entry points take: the operands' tensor maps and the parameters common to whole and split products.
+int prepare2(const void* a, const void* b, void* c, const void* bias, void* aux, int M, int N, int K, long lda, long ldb, long ldc, int a_mn,
+             int b_mn, int epi, int* status, CUtensorMap& tmA, CUtensorMap& tmB, Params2& p, int& sms) {
     if (M <= 0 || N <= 0 || K <= 0 || (N & 7) || (K & 7) || (ldc & 7) || status == nullptr) return TT_ERR_ARG;
     if (a_mn && (M & 7)) return TT_ERR_ARG;
     if (epi < 0 || epi > 4 || (epi != 0 && aux == nullptr)) return TT_ERR_ARG;
     if (((uintptr_t)c & 15) || (bias && ((uintptr_t)bias & 15)) || (aux && ((uintptr_t)aux & 15))) return TT_ERR_ARG;
     if (a_mn && !b_mn) return TT_ERR_ARG;
-    int dev = 0, sms = 148;
+    int dev = 0;
+    sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    CUtensorMap tmA, tmB, tmC, tmAux;
     int rc;
     if (!a_mn) rc = tt_make_tmap_2d(&tmA, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BMH, BK);
     else rc = tt_make_tmap_2d(&tmA, a, (uint64_t)K, (uint64_t)M, (uint64_t)lda, 64, 64);
@@ -338,10 +393,6 @@ extern "C" int tt_gemm2_bf16(const void* a, const void* b, void* c, const void* 
     if (!b_mn) rc = tt_make_tmap_2d(&tmB, b, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, BNH, BK);
     else rc = tt_make_tmap_2d(&tmB, b, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, 64, 64);
     if (rc != TT_OK) return rc;
-    if ((rc = tt_make_tmap_2d(&tmC, c, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64)) != TT_OK) return rc;
-    tmAux = tmC;
-    if ((epi == 1 || epi == 2) && (rc = tt_make_tmap_2d(&tmAux, aux, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64)) != TT_OK) return rc;
-    Params2 p;
     memset(&p, 0, sizeof(p));
     p.M = M; p.N = N; p.K = K;
     p.C = (__nv_bfloat16*)c;
@@ -351,6 +402,24 @@ extern "C" int tt_gemm2_bf16(const void* a, const void* b, void* c, const void* 
     p.status = status;
     p.tiles_m = (M + 255) / 256;
     p.tiles_n = (N + 255) / 256;
+    p.splits = 1;
+    p.kb_split = (K + BK - 1) / BK;
+    return TT_OK;
+}
+
+}  // namespace
+
+// Same contract as tt_gemm_bf16 (gemm_tcgen05.cu); returns TT_ERR_ARG for shapes this kernel does not take, so that the
+// caller can fall back to the single-CTA kernel.
+extern "C" int tt_gemm2_bf16(const void* a, const void* b, void* c, const void* bias, void* aux, int M, int N, int K,
+                             long lda, long ldb, long ldc, int a_mn, int b_mn, int epi, int* status, void* stream) {
+    CUtensorMap tmA, tmB, tmC, tmAux;
+    Params2 p;
+    int sms, rc;
+    if ((rc = prepare2(a, b, c, bias, aux, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, status, tmA, tmB, p, sms)) != TT_OK) return rc;
+    if ((rc = tt_make_tmap_2d(&tmC, c, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64)) != TT_OK) return rc;
+    tmAux = tmC;
+    if ((epi == 1 || epi == 2) && (rc = tt_make_tmap_2d(&tmAux, aux, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64)) != TT_OK) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     const bool amn = a_mn != 0, bmn = b_mn != 0;
 #define GO(A_, B_, E_) return launch2<A_, B_, E_>(tmA, tmB, tmC, tmAux, p, sms, st)
@@ -367,4 +436,38 @@ extern "C" int tt_gemm2_bf16(const void* a, const void* b, void* c, const void* 
     }
 #undef GO
     return TT_ERR_ARG;
+}
+
+// The product with its k-blocks shared by `splits` pairs per tile.  scratch: fp32, splits * roundup(M, 32) * N entries.
+extern "C" int tt_gemm2_bf16_splitk(const void* a, const void* b, void* c, const void* bias, void* aux, int M, int N, int K, long lda, long ldb,
+                                    long ldc, int a_mn, int b_mn, int epi, int splits, float* scratch, int* status, void* stream) {
+    CUtensorMap tmA, tmB, tmC;
+    Params2 p;
+    int sms, rc;
+    if ((rc = prepare2(a, b, c, bias, aux, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, status, tmA, tmB, p, sms)) != TT_OK) return rc;
+    if (splits < 1 || splits > p.kb_split || scratch == nullptr || ((uintptr_t)scratch & 15)) return TT_ERR_ARG;
+    const int kblocks = p.kb_split;
+    p.kb_split = (kblocks + splits - 1) / splits;
+    p.splits = (kblocks + p.kb_split - 1) / p.kb_split;           // no empty range
+    p.part_rows = (M + 31) / 32 * 32;
+    if ((rc = tt_make_tmap_2d_f32(&tmC, scratch, (uint64_t)p.part_rows * p.splits, (uint64_t)N, (uint64_t)N, 32, 32)) != TT_OK) return rc;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (!a_mn && !b_mn) rc = launch2<false, false, 7>(tmA, tmB, tmC, tmC, p, sms, st);
+    else if (!a_mn) rc = launch2<false, true, 7>(tmA, tmB, tmC, tmC, p, sms, st);
+    else rc = launch2<true, true, 7>(tmA, tmB, tmC, tmC, p, sms, st);
+    if (rc != TT_OK) return rc;
+    const long want = ((long)M * (N >> 3) + 255) / 256;
+    const int grid = (int)(want < 148L * 8 ? want : 148L * 8);
+    const long slice = (long)p.part_rows * N;
+#define FIN(E_)                                                                                                          \
+    splitk_finish_kernel<E_><<<grid, 256, 0, st>>>(scratch, p.splits, slice, M, N, ldc, (const __nv_bfloat16*)bias,        \
+                                                   (__nv_bfloat16*)aux, (__nv_bfloat16*)c)
+    if (epi == 0) FIN(0);
+    else if (epi == 1) FIN(1);
+    else if (epi == 2) FIN(2);
+    else if (epi == 3) FIN(3);
+    else FIN(4);
+#undef FIN
+    TT_CHECK_LAUNCH();
+    return TT_OK;
 }

@@ -248,6 +248,9 @@ tt_encode_tiled_fn tt_get_encode_tiled();
 // 2-D bf16 tensor [rows, cols] (cols contiguous, row pitch `ld` elements), box [box_rows, box_cols], 128B swizzle.
 int tt_make_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
                     uint32_t box_cols);
+// The same for fp32 (box_cols * 4 <= 128).
+int tt_make_tmap_2d_f32(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
+                        uint32_t box_cols);
 // 3-D bf16 tensor [d2, d1, d0] (d0 contiguous), box [1, box1, box0], 128B swizzle.
 int tt_make_tmap_3d(CUtensorMap* out, const void* base, uint64_t d2, uint64_t d1, uint64_t d0, uint64_t stride1,
                     uint64_t stride2, uint32_t box1, uint32_t box0);

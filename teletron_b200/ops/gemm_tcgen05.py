@@ -12,6 +12,7 @@ into :class:`teletron_b200.ops._lib.CommTimeoutError` (the CUDA context stays us
 
 from __future__ import annotations
 
+import functools
 import os
 from typing import Dict, Optional, Tuple
 
@@ -26,11 +27,35 @@ _LAYOUTS = {"nt": (0, 0), "nn": (0, 1), "tn": (1, 1)}
 # TELETRON_B200_GEMM_2CTA=0 keeps everything on the single-CTA kernel
 PAIR_KERNEL = os.environ.get("TELETRON_B200_GEMM_2CTA", "1") != "0"
 PAIR_MIN_TILES = 74
-COUNTERS = {"pair": 0, "single": 0}
+COUNTERS = {"pair": 0, "single": 0, "split": 0}
 
 
 def use_pair_kernel(M: int, N: int) -> bool:
     return PAIR_KERNEL and ((M + 255) // 256) * ((N + 255) // 256) >= PAIR_MIN_TILES
+
+
+@functools.lru_cache(maxsize=4096)
+def _plan(M: int, N: int, K: int) -> Tuple[bool, int]:
+    """``(pair, splits)`` for a product with fewer than PAIR_MIN_TILES 256 x 256 tiles.
+
+    Costs in microseconds as measured over M = 40 .. 1280, N = 3072 .. 12288, K = 3072 .. 15360 with weights from HBM: a
+    64-wide k-block of a wave of 128 x 128 tiles (148 of them, one an SM) takes 0.22 us, 0.26 when waves follow one another
+    (32 KB through L2 per SM set the pace); a wave of 74 pair tiles takes 0.30 (four times the tile on twice the SMs: the
+    tensor core does); a split product adds a second launch and one write and read of its fp32 slices.  Examples, single /
+    pair / best split: 256 x 3072 x 12288 45.7 / 62.2 / 25.5 (6 splits); 256 x 12288 x 3072 28.1 / 23.0 / 29.0;
+    256 x 9216 x 3072 17.4 / 22.0 / 21.6; 1024 x 3072 x 12288 85.8 / 67.8 / 61.1 (3); 512 x 3072 x 4096 18.8 / 25.9 / 18.8."""
+    kb, t1, t2 = (K + 63) // 64, ((M + 127) // 128) * ((N + 127) // 128), ((M + 255) // 256) * ((N + 255) // 256)
+    waves = (t1 + 147) // 148
+    best = (4 + waves * kb * (0.22 if waves == 1 else 0.26), False, 1)
+    for s in range(1, min(16, kb // 4) + 1):
+        cost = 5 + ((t2 * s + 73) // 74) * ((kb + s - 1) // s) * 0.30
+        if s > 1:
+            cost += 5 + 0.13e-6 * (s * ((M + 31) // 32 * 32) * N * 8)
+        if cost < best[0]:
+            best = (cost, True, s)
+    return best[1:]
+
+
 _STATUS: Dict[torch.device, torch.Tensor] = {}
 
 
@@ -90,7 +115,16 @@ def gemm(a: torch.Tensor, b: torch.Tensor, layout: str, bias: Optional[torch.Ten
             raise _lib.NativeError("epilogue 3/4 needs a contiguous [M, N] pre-activation tensor")
     if bias is not None:
         bias = _lib.check(bias.contiguous(), BF16, "bias")
-    pair = use_pair_kernel(M, N)
+    pair, splits = use_pair_kernel(M, N), 1
+    if PAIR_KERNEL and not pair:
+        pair, splits = _plan(M, N, K)
+    if splits > 1:
+        COUNTERS["split"] += 1
+        scratch = torch.empty(splits * ((M + 31) // 32 * 32) * N, dtype=torch.float32, device=a.device)
+        call("tt_gemm2_bf16_splitk", ptr(a), ptr(b), ptr(c), ptr(bias), ptr(aux), c_int(M), c_int(N), c_int(K), c_long(a.stride(0)),
+             c_long(b.stride(0)), c_long(c.stride(0)), c_int(a_mn), c_int(b_mn), c_int(epi), c_int(splits), ptr(scratch),
+             ptr(status_tensor(a.device)), stream())
+        return (c, aux) if epi in (1, 2) else c
     COUNTERS["pair" if pair else "single"] += 1
     call("tt_gemm2_bf16" if pair else "tt_gemm_bf16", ptr(a), ptr(b), ptr(c), ptr(bias), ptr(aux), c_int(M), c_int(N), c_int(K), c_long(a.stride(0)),
          c_long(b.stride(0)), c_long(c.stride(0)), c_int(a_mn), c_int(b_mn), c_int(epi), ptr(status_tensor(a.device)),

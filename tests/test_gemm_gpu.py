@@ -179,3 +179,40 @@ def test_cta_pair_kernel_epilogues():
         G.check_status()
     finally:
         G.PAIR_KERNEL, G.PAIR_MIN_TILES = old
+
+
+@pytest.mark.parametrize("M,N,K,splits", [(33, 72, 512, 2), (256, 264, 4104, 6), (130, 520, 1032, 5), (520, 136, 2056, 16), (8, 8, 264, 2)])
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+def test_split_k(M, N, K, splits, layout, monkeypatch):
+    """Ragged rows, columns and k-blocks (a last range shorter than the others, ranges that would be empty), every epilogue
+    the layout has, an output window, and the same bits twice."""
+    from teletron_b200.ops import gemm_tcgen05 as G
+    if layout == "tn" and M % 8:
+        pytest.skip("tn needs M % 8 == 0")
+    monkeypatch.setattr(G, "_plan", lambda *a: (True, splits))
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = _mk((K, M) if layout == "tn" else (M, K), g)
+    b = _mk((N, K) if layout == "nt" else (K, N), g, 0.05)
+    ref = (a.double().t() if layout == "tn" else a.double()) @ (b.double().t() if layout == "nt" else b.double())
+    before = G.COUNTERS["split"]
+    guard = torch.full((M + 2, N + 16), -777.0, device="cuda", dtype=torch.bfloat16)
+    c = G.gemm(a, b, layout, out=guard[1:M + 1, 8:N + 8])
+    assert G.COUNTERS["split"] == before + 1
+    assert _rel(c, ref) < 3e-3                   # one bf16 rounding (2^-9 relative, 1.7e-3 in norm) and fp32 sums
+    guard[1:M + 1, 8:N + 8] = -777.0
+    assert bool((guard == -777.0).all())
+    assert torch.equal(G.gemm(a, b, layout), G.gemm(a, b, layout))
+    if layout == "nt":
+        bias = _mk((N,), g)
+        assert _rel(G.gemm(a, b, "nt", bias), ref + bias.double()) < 3e-3
+        for epi, approx in ((1, "none"), (2, "tanh")):
+            y, u = G.gemm(a, b, "nt", bias, epi=epi)
+            assert _rel(u, ref + bias.double()) < 3e-3
+            assert _rel(y, torch.nn.functional.gelu(ref + bias.double(), approximate=approx)) < 4e-3
+    elif layout == "nn":
+        aux = _mk((M, N), g)
+        for epi, approx in ((3, "none"), (4, "tanh")):
+            ud = aux.double().requires_grad_()
+            torch.nn.functional.gelu(ud, approximate=approx).backward(ref)
+            assert _rel(G.gemm(a, b, "nn", epi=epi, aux=aux), ud.grad) < 4e-3
+    G.check_status()
