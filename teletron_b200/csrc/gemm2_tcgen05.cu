@@ -18,6 +18,9 @@
 // shared by `splits` pairs; each writes its fp32 accumulator to its own slice of a scratch buffer (EPI 7) and a second kernel
 // adds the slices in a fixed order and applies the epilogue.
 //
+// Two A operands (tt_gemm2_bf16_two): [a | a2] B^T with the K columns from k1 on taken from a second tensor, so that the
+// single-stream block's [attention | MLP] never has to be concatenated.
+//
 // Layouts and epilogues are those of gemm_tcgen05.cu (nt / nn / tn; bias, GELU erf / tanh with pre-activation,
 // GELU backward).  In the reference these products are TransformerEngine -> cuBLASLt calls
 // (teletron/models/dit/dit_attention.py:65-104, dit_layerspec.py:266-298, 438-445).
@@ -54,6 +57,7 @@ struct Params2 {
     int* status;
     int tiles_m, tiles_n;       // in 256 x 256 tiles
     int splits, kb_split;       // k-block ranges per tile, and their length
+    int k1;                     // K columns >= k1 come from the second A tensor (a multiple of BK, or >= K: there is none)
     int part_rows;              // rows of one split's slice of the scratch buffer (M rounded up to whole 32-row boxes)
 };
 
@@ -113,7 +117,7 @@ __device__ __forceinline__ float epi2(float acc, float b, float u) {
 template <bool A_MN, bool B_MN, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
-             const __grid_constant__ CUtensorMap tmAux, const Params2 p) {
+             const __grid_constant__ CUtensorMap tmAux, const __grid_constant__ CUtensorMap tmA2, const Params2 p) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ volatile int abort_flag;
     __shared__ uint32_t tmem_base_slot;
@@ -188,7 +192,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                     if (rank == 0) mbar_arrive_expect_tx(full_bar(stage), 2 * kStageBytes);      // both CTAs' bytes
                     const int k0 = kb * BK;
                     if (!A_MN) {
-                        tma_load_2d_pair(sa, &tmA, full_bar(stage), k0, am);
+                        const bool second = k0 >= p.k1;
+                        tma_load_2d_pair(sa, second ? &tmA2 : &tmA, full_bar(stage), second ? k0 - p.k1 : k0, am);
                     } else {
 #pragma unroll
                         for (int j = 0; j < BMH / 64; ++j) tma_load_2d_pair(sa + j * 8192, &tmA, full_bar(stage), am + 64 * j, k0);
@@ -322,7 +327,8 @@ done:
 }
 
 template <bool A_MN, bool B_MN, int EPI>
-int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmAux, const Params2& p, int sms, cudaStream_t st) {
+int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmAux, const CUtensorMap& tmA2,
+            const Params2& p, int sms, cudaStream_t st) {
     auto kern = gemm2_kernel<A_MN, B_MN, EPI>;
     static bool configured[64] = {false};
     int dev = 0;
@@ -336,7 +342,7 @@ int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& t
     int pairs = sms / 2;
     if (pairs > tiles) pairs = tiles;
     if (pairs < 1) pairs = 1;
-    kern<<<2 * pairs, kThreads, kSmemBytes, st>>>(tmA, tmB, tmC, tmAux, p);      // cluster shape comes from __cluster_dims__
+    kern<<<2 * pairs, kThreads, kSmemBytes, st>>>(tmA, tmB, tmC, tmAux, tmA2, p);      // cluster shape comes from __cluster_dims__
     TT_CHECK_LAUNCH();
     return TT_OK;
 }
@@ -375,24 +381,29 @@ __global__ void __launch_bounds__(256) splitk_finish_kernel(const float* __restr
     }
 }
 
-// What both entry points take: the operands' tensor maps and the parameters common to whole and split products.
-int prepare2(const void* a, const void* b, void* c, const void* bias, void* aux, int M, int N, int K, long lda, long ldb, long ldc, int a_mn,
-             int b_mn, int epi, int* status, CUtensorMap& tmA, CUtensorMap& tmB, Params2& p, int& sms) {
+// The product of every entry point.  a2 (or nullptr) supplies the K columns from k1 on; splits > 1 needs `scratch`.
+int run2(const void* a, const void* a2, int k1, long lda2, const void* b, void* c, const void* bias, void* aux, int M, int N, int K, long lda,
+         long ldb, long ldc, int a_mn, int b_mn, int epi, int splits, float* scratch, int* status, void* stream) {
     if (M <= 0 || N <= 0 || K <= 0 || (N & 7) || (K & 7) || (ldc & 7) || status == nullptr) return TT_ERR_ARG;
     if (a_mn && (M & 7)) return TT_ERR_ARG;
     if (epi < 0 || epi > 4 || (epi != 0 && aux == nullptr)) return TT_ERR_ARG;
     if (((uintptr_t)c & 15) || (bias && ((uintptr_t)bias & 15)) || (aux && ((uintptr_t)aux & 15))) return TT_ERR_ARG;
     if (a_mn && !b_mn) return TT_ERR_ARG;
-    int dev = 0;
-    sms = 148;
+    if (a2 != nullptr && (a_mn || k1 <= 0 || k1 >= K || (k1 % BK))) return TT_ERR_ARG;
+    const int kblocks = (K + BK - 1) / BK;
+    if (splits < 1 || splits > kblocks || (splits > 1 && (scratch == nullptr || ((uintptr_t)scratch & 15)))) return TT_ERR_ARG;
+    int dev = 0, sms = 148, rc;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int rc;
-    if (!a_mn) rc = tt_make_tmap_2d(&tmA, a, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BMH, BK);
+    CUtensorMap tmA, tmA2, tmB, tmC, tmAux;
+    if (!a_mn) rc = tt_make_tmap_2d(&tmA, a, (uint64_t)M, (uint64_t)(a2 != nullptr ? k1 : K), (uint64_t)lda, BMH, BK);
     else rc = tt_make_tmap_2d(&tmA, a, (uint64_t)K, (uint64_t)M, (uint64_t)lda, 64, 64);
     if (rc != TT_OK) return rc;
+    tmA2 = tmA;
+    if (a2 != nullptr && (rc = tt_make_tmap_2d(&tmA2, a2, (uint64_t)M, (uint64_t)(K - k1), (uint64_t)lda2, BMH, BK)) != TT_OK) return rc;
     if (!b_mn) rc = tt_make_tmap_2d(&tmB, b, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, BNH, BK);
     else rc = tt_make_tmap_2d(&tmB, b, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, 64, 64);
     if (rc != TT_OK) return rc;
+    Params2 p;
     memset(&p, 0, sizeof(p));
     p.M = M; p.N = N; p.K = K;
     p.C = (__nv_bfloat16*)c;
@@ -402,59 +413,35 @@ int prepare2(const void* a, const void* b, void* c, const void* bias, void* aux,
     p.status = status;
     p.tiles_m = (M + 255) / 256;
     p.tiles_n = (N + 255) / 256;
-    p.splits = 1;
-    p.kb_split = (K + BK - 1) / BK;
-    return TT_OK;
-}
-
-}  // namespace
-
-// Same contract as tt_gemm_bf16 (gemm_tcgen05.cu); returns TT_ERR_ARG for shapes this kernel does not take, so that the
-// caller can fall back to the single-CTA kernel.
-extern "C" int tt_gemm2_bf16(const void* a, const void* b, void* c, const void* bias, void* aux, int M, int N, int K,
-                             long lda, long ldb, long ldc, int a_mn, int b_mn, int epi, int* status, void* stream) {
-    CUtensorMap tmA, tmB, tmC, tmAux;
-    Params2 p;
-    int sms, rc;
-    if ((rc = prepare2(a, b, c, bias, aux, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, status, tmA, tmB, p, sms)) != TT_OK) return rc;
-    if ((rc = tt_make_tmap_2d(&tmC, c, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64)) != TT_OK) return rc;
-    tmAux = tmC;
-    if ((epi == 1 || epi == 2) && (rc = tt_make_tmap_2d(&tmAux, aux, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64)) != TT_OK) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
-    const bool amn = a_mn != 0, bmn = b_mn != 0;
-#define GO(A_, B_, E_) return launch2<A_, B_, E_>(tmA, tmB, tmC, tmAux, p, sms, st)
-    if (!amn && !bmn) {
-        if (epi == 0) GO(false, false, 0);
-        if (epi == 1) GO(false, false, 1);
-        if (epi == 2) GO(false, false, 2);
-    } else if (!amn && bmn) {
-        if (epi == 0) GO(false, true, 0);
-        if (epi == 3) GO(false, true, 3);
-        if (epi == 4) GO(false, true, 4);
-    } else if (amn && bmn) {
-        if (epi == 0) GO(true, true, 0);
-    }
-#undef GO
-    return TT_ERR_ARG;
-}
-
-// The product with its k-blocks shared by `splits` pairs per tile.  scratch: fp32, splits * roundup(M, 32) * N entries.
-extern "C" int tt_gemm2_bf16_splitk(const void* a, const void* b, void* c, const void* bias, void* aux, int M, int N, int K, long lda, long ldb,
-                                    long ldc, int a_mn, int b_mn, int epi, int splits, float* scratch, int* status, void* stream) {
-    CUtensorMap tmA, tmB, tmC;
-    Params2 p;
-    int sms, rc;
-    if ((rc = prepare2(a, b, c, bias, aux, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, status, tmA, tmB, p, sms)) != TT_OK) return rc;
-    if (splits < 1 || splits > p.kb_split || scratch == nullptr || ((uintptr_t)scratch & 15)) return TT_ERR_ARG;
-    const int kblocks = p.kb_split;
+    p.k1 = a2 != nullptr ? k1 : K;
     p.kb_split = (kblocks + splits - 1) / splits;
     p.splits = (kblocks + p.kb_split - 1) / p.kb_split;           // no empty range
     p.part_rows = (M + 31) / 32 * 32;
-    if ((rc = tt_make_tmap_2d_f32(&tmC, scratch, (uint64_t)p.part_rows * p.splits, (uint64_t)N, (uint64_t)N, 32, 32)) != TT_OK) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    if (!a_mn && !b_mn) rc = launch2<false, false, 7>(tmA, tmB, tmC, tmC, p, sms, st);
-    else if (!a_mn) rc = launch2<false, true, 7>(tmA, tmB, tmC, tmC, p, sms, st);
-    else rc = launch2<true, true, 7>(tmA, tmB, tmC, tmC, p, sms, st);
+    const bool amn = a_mn != 0, bmn = b_mn != 0;
+    if (splits == 1) {
+        if ((rc = tt_make_tmap_2d(&tmC, c, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64)) != TT_OK) return rc;
+        tmAux = tmC;
+        if ((epi == 1 || epi == 2) && (rc = tt_make_tmap_2d(&tmAux, aux, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64)) != TT_OK) return rc;
+#define GO(A_, B_, E_) return launch2<A_, B_, E_>(tmA, tmB, tmC, tmAux, tmA2, p, sms, st)
+        if (!amn && !bmn) {
+            if (epi == 0) GO(false, false, 0);
+            if (epi == 1) GO(false, false, 1);
+            if (epi == 2) GO(false, false, 2);
+        } else if (!amn && bmn) {
+            if (epi == 0) GO(false, true, 0);
+            if (epi == 3) GO(false, true, 3);
+            if (epi == 4) GO(false, true, 4);
+        } else if (amn && bmn) {
+            if (epi == 0) GO(true, true, 0);
+        }
+#undef GO
+        return TT_ERR_ARG;
+    }
+    if ((rc = tt_make_tmap_2d_f32(&tmC, scratch, (uint64_t)p.part_rows * p.splits, (uint64_t)N, (uint64_t)N, 32, 32)) != TT_OK) return rc;
+    if (!amn && !bmn) rc = launch2<false, false, 7>(tmA, tmB, tmC, tmC, tmA2, p, sms, st);
+    else if (!amn) rc = launch2<false, true, 7>(tmA, tmB, tmC, tmC, tmA2, p, sms, st);
+    else rc = launch2<true, true, 7>(tmA, tmB, tmC, tmC, tmA2, p, sms, st);
     if (rc != TT_OK) return rc;
     const long want = ((long)M * (N >> 3) + 255) / 256;
     const int grid = (int)(want < 148L * 8 ? want : 148L * 8);
@@ -470,4 +457,26 @@ extern "C" int tt_gemm2_bf16_splitk(const void* a, const void* b, void* c, const
 #undef FIN
     TT_CHECK_LAUNCH();
     return TT_OK;
+}
+
+}  // namespace
+
+// Same contract as tt_gemm_bf16 (gemm_tcgen05.cu); returns TT_ERR_ARG for shapes this kernel does not take, so that the
+// caller can fall back to the single-CTA kernel.
+extern "C" int tt_gemm2_bf16(const void* a, const void* b, void* c, const void* bias, void* aux, int M, int N, int K,
+                             long lda, long ldb, long ldc, int a_mn, int b_mn, int epi, int* status, void* stream) {
+    return run2(a, nullptr, 0, 0, b, c, bias, aux, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, 1, nullptr, status, stream);
+}
+
+// The product with its k-blocks shared by `splits` pairs per tile.  scratch: fp32, splits * roundup(M, 32) * N entries.
+extern "C" int tt_gemm2_bf16_splitk(const void* a, const void* b, void* c, const void* bias, void* aux, int M, int N, int K, long lda, long ldb,
+                                    long ldc, int a_mn, int b_mn, int epi, int splits, float* scratch, int* status, void* stream) {
+    return run2(a, nullptr, 0, 0, b, c, bias, aux, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, splits, scratch, status, stream);
+}
+
+// c = [a | a2] b^T + bias: a [M, k1] (k1 a multiple of 64), a2 [M, K - k1], b [N, K]; splits and scratch as above.
+extern "C" int tt_gemm2_bf16_two(const void* a, const void* a2, const void* b, void* c, const void* bias, int M, int N, int K, int k1, long lda,
+                                 long lda2, long ldb, long ldc, int splits, float* scratch, int* status, void* stream) {
+    if (a2 == nullptr) return TT_ERR_ARG;
+    return run2(a, a2, k1, lda2, b, c, bias, nullptr, M, N, K, lda, ldb, ldc, 0, 0, 0, splits, scratch, status, stream);
 }

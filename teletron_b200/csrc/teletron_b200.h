@@ -93,6 +93,8 @@ int tt_gemm2_bf16(const void* a, const void* b, void* c, const void* bias, void*
 int tt_gemm2_bf16_splitk(const void* a, const void* b, void* c, const void* bias, void* aux, int M, int N, int K, long lda,
                          long ldb, long ldc, int a_mn, int b_mn, int epi, int splits, float* scratch, int* status,
                          void* stream);
+int tt_gemm2_bf16_two(const void* a, const void* a2, const void* b, void* c, const void* bias, int M, int N, int K, int k1,
+                      long lda, long lda2, long ldb, long ldc, int splits, float* scratch, int* status, void* stream);
 
 /* pushed tiles (tt_gemm_comm_bf16 store modes 1 / 2): 1 = staged stores of whole 256-byte rows (default), 0 = 16 bytes per thread */
 void tt_set_coalesced_peer_stores(int on);

@@ -421,15 +421,16 @@ class SingleAttention(nn.Module):
         self.k_layernorm = RMSNorm(head_dim, eps, tp > 1, **kw)
 
     def forward(self, h, text_len, cos, sin, pad, kv_valid_len, in_region: bool = False):
+        """Token-major ``[B, S + T, heads * head_dim]``, video tokens first."""
         if not in_region:
             h = M.copy_to_tensor_model_parallel_region(h, ps.get_tensor_model_parallel_group())
         s = h.shape[1] - text_len
         q, k, v = ops.qkv_projection(h, self.linear_qkv.weight, self.linear_qkv.bias, self.q_layernorm.weight,
                                      self.k_layernorm.weight, cos, sin, self.heads_local, self.eps, rope_len=s)
         if ps.get_context_parallel_world_size() == 1:
-            return _joint_attention(q, k, v, text_len, kv_valid_len)
-        return _ulysses_attention(q[:, :, :s], k[:, :, :s], v[:, :, :s], q[:, :, s:], k[:, :, s:], v[:, :, s:],
-                                  pad, kv_valid_len)
+            return ops.attention(q, k, v, kv_valid_len=None if kv_valid_len is None else s + kv_valid_len)
+        return torch.cat(_ulysses_attention(q[:, :, :s], k[:, :, :s], v[:, :, :s], q[:, :, s:], k[:, :, s:], v[:, :, s:],
+                                            pad, kv_valid_len), dim=1)
 
 
 # ---------------------------------------------------------------------------------------------
@@ -505,8 +506,8 @@ class HunyuanSingleDiTLayer(nn.Module):
         if _use_fused(hn, self.self_attention.head_dim):
             proj = self._attention_and_projection_fused(hn, mlp, T, cos, sin, pad, kv_valid_len, in_region=sp)
         else:
-            attn, c_attn = self.self_attention(hn, T, cos, sin, pad, kv_valid_len, in_region=sp)
-            proj = self.proj_out.forward_merged(torch.cat([attn, c_attn], dim=1), mlp, row_splits=splits)
+            attn = self.self_attention(hn, T, cos, sin, pad, kv_valid_len, in_region=sp)
+            proj = self.proj_out.forward_merged(attn, mlp, row_splits=splits)
         h = ops.gate_residual(h, proj, gate)
         return M.split_tokens(h, h.shape[1] - T_own)
 

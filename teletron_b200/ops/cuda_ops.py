@@ -281,8 +281,9 @@ class _Linear(torch.autograd.Function):
 
 class _LinearMerged(torch.autograd.Function):
     """``y = cat([x1, x2], -1) @ weight^T + bias`` for the single-stream block's merged projection (attention output and
-    MLP activation side by side).  The forward concatenates once and runs one GEMM; the backward never forms the
-    concatenated gradient: each input's gradient comes from its own GEMM against a column slice of the weight (a strided
+    MLP activation side by side).  The forward's GEMM takes its K columns from the two tensors where they are (concatenated
+    first only if their seam does not suit the kernel: 1 GB written and read again per block at 32656 tokens); the backward
+    never forms the concatenated gradient: each input's gradient comes from its own GEMM against a column slice of the weight (a strided
     B operand), and each half of the weight gradient is written into its column slice of ``dW``, so no strided slice
     of a ``[tokens, k1 + k2]`` gradient has to be copied to make it contiguous."""
 
@@ -290,7 +291,12 @@ class _LinearMerged(torch.autograd.Function):
     def forward(ctx, x1, x2, weight, bias):
         k1, k2 = x1.shape[-1], x2.shape[-1]
         a1, a2 = x1.reshape(-1, k1), x2.reshape(-1, k2)
-        y = _gemm_nt(torch.cat([a1, a2], dim=1), weight, bias)
+        from . import gemm, gemm_tcgen05
+        if gemm.get_backend() != "cublas" and gemm_tcgen05.two_supported(a1, a2, weight):
+            gemm.COUNTERS["tcgen05"] += 1
+            y = gemm_tcgen05.gemm_two(a1, a2, weight, bias)
+        else:
+            y = _gemm_nt(torch.cat([a1, a2], dim=1), weight, bias)
         ctx.save_for_backward(a1, a2, weight)
         ctx.has_bias = bias is not None
         ctx.lead = x1.shape[:-1]

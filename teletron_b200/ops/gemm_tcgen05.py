@@ -130,3 +130,25 @@ def gemm(a: torch.Tensor, b: torch.Tensor, layout: str, bias: Optional[torch.Ten
          c_long(b.stride(0)), c_long(c.stride(0)), c_int(a_mn), c_int(b_mn), c_int(epi), ptr(status_tensor(a.device)),
          stream())
     return (c, aux) if epi in (1, 2) else c
+
+
+def two_supported(a: torch.Tensor, a2: torch.Tensor, b: torch.Tensor) -> bool:
+    """``[a | a2] @ b.T`` without the concatenation: the seam has to lie between two 64-wide k-blocks."""
+    return (PAIR_KERNEL and a2.dtype == BF16 and a2.is_cuda and _rowmajor(a2) and a.dim() == 2 and a.shape[0] == a2.shape[0]
+            and a.shape[1] % 64 == 0 and a2.shape[1] % 8 == 0 and a2.shape[1] > 0 and a.shape[1] + a2.shape[1] == b.shape[1]
+            and supported(a, b[:, :a.shape[1]], "nt"))
+
+
+def gemm_two(a: torch.Tensor, a2: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Always on the CTA-pair kernel: what the single-CTA kernel gains on a short product is less than the concatenation costs."""
+    (M, k1), N, K = a.shape, b.shape[0], b.shape[1]
+    c = torch.empty(M, N, dtype=BF16, device=a.device)
+    if bias is not None:
+        bias = _lib.check(bias.contiguous(), BF16, "bias")
+    splits = 1 if use_pair_kernel(M, N) else _plan(M, N, K)[1]
+    COUNTERS["pair" if splits == 1 else "split"] += 1
+    scratch = None if splits == 1 else torch.empty(splits * ((M + 31) // 32 * 32) * N, dtype=torch.float32, device=a.device)
+    call("tt_gemm2_bf16_two", ptr(a), ptr(a2), ptr(b), ptr(c), ptr(bias), c_int(M), c_int(N), c_int(K), c_int(k1), c_long(a.stride(0)),
+         c_long(a2.stride(0)), c_long(b.stride(0)), c_long(c.stride(0)), c_int(splits), ptr(scratch), ptr(status_tensor(a.device)), stream())
+    _lib.LAUNCHES += splits > 1      # the pass over the slices
+    return c

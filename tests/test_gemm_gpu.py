@@ -216,3 +216,21 @@ def test_split_k(M, N, K, splits, layout, monkeypatch):
             torch.nn.functional.gelu(ud, approximate=approx).backward(ref)
             assert _rel(G.gemm(a, b, "nn", epi=epi, aux=aux), ud.grad) < 4e-3
     G.check_status()
+
+
+@pytest.mark.parametrize("M,k1,k2,N,splits", [(300, 64, 72, 264, 1), (1031, 384, 1536, 768, 1), (8, 128, 64, 8, 1), (257, 320, 2040, 136, 4)])
+def test_two_operands_side_by_side(M, k1, k2, N, splits, monkeypatch):
+    """``[a | a2] @ b.T`` from two tensors (one of them a strided view): the seam inside a split's range, ragged ends, with
+    the same k order as the concatenated product and therefore the same bits when that takes the same kernel."""
+    from teletron_b200.ops import gemm_tcgen05 as G
+    monkeypatch.setattr(G, "_plan", lambda *a: (True, splits))
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a, wide, b, bias = _mk((M, k1), g), _mk((M, k2 + 16), g), _mk((N, k1 + k2), g, 0.05), _mk((N,), g)
+    a2 = wide[:, 8:8 + k2]
+    assert G.two_supported(a, a2, b)
+    c = G.gemm_two(a, a2, b, bias)
+    cat = torch.cat([a, a2], dim=1)
+    assert _rel(c, cat.double() @ b.double().t() + bias.double()) < 3e-3
+    assert torch.equal(c, G.gemm(cat, b, "nt", bias))
+    assert not G.two_supported(a[:, :k1 - 8], a2, b[:, 8:])
+    G.check_status()
