@@ -12,8 +12,7 @@
 //
 // Both run the same pipeline.  Stationary operands [128 x 128] are loaded once; streamed chunks are 128 rows,
 // held in two TMA rings (three slots for the operand that the score product needs early and dK / dQ needs last,
-// two for the other).  Chunks of 128 keep every MMA at N = 128: an N = 64 instruction was measured to take as long
-// as an N = 128 one on this part.  T1 and T2 are single-buffered in tensor memory; the overlap comes from keeping P
+// two for the other).  Chunks of 128 keep every MMA at N = 128, which takes 64 clocks; an N = 64 one takes 49.  T1 and T2 are single-buffered in tensor memory; the overlap comes from keeping P
 // in registers between the two softmax passes, so that T1 is free for the next chunk's scores while dS is formed:
 //
 //   tensor core:  S(c+1) ......... | dK(c) dV(c) dP(c+1) | S(c+2) ........ | dK(c+1) ...
@@ -103,8 +102,8 @@ __global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restr
 }
 
 // TSA (query-stationary only): the stationary operands Q and dO live in tensor memory (bf16 pairs, columns [384, 512),
-// free in that kernel) instead of shared memory, so the score-type products become TS instructions.  An SS instruction
-// with N = 128 was measured at ~128 clocks on this part, a TS one at ~84.
+// free in that kernel) instead of shared memory, so the score-type products become TS instructions and read half the
+// shared memory (both forms issue at 64 clocks for N = 128).
 template <bool KVS, bool TSA = false>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
