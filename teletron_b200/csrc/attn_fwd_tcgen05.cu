@@ -265,6 +265,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale_log2;
             const bool grow = mx > m + kRescaleThreshold;           // always for the first visible key (m = -inf)
             if (__any_sync(0xffffffffu, grow)) {
+                tmem_st_wait();         // the stores that are about to be repeated have landed: the second ones win
                 if (j > 0) {
                     const float alpha = grow ? exp2f(m - mx) : 1.f;
                     l *= alpha;
