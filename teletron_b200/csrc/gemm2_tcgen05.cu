@@ -248,6 +248,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
     } else {
         // ------------------------------------------------------------ epilogue (warps 2..5 of each CTA: its 128 rows)
         const int quad = warp & 3;
+        uint32_t nbox = 0;       // boxes alternate across tiles too: a tile may store an odd number of them
         int it = 0;
         for (int t = pair; t < num_tiles; t += n_pairs, ++it) {
             int m0, n0;
@@ -274,7 +275,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                     uint32_t r[32];
                     tmem_ld_32x32(tacc + c * 32, r);
                     tmem_ld_wait();
-                    store_box_32x64(box + ((c & 1) ? 4096u : 0u), &tmC, col0, prow, lane,
+                    store_box_32x64(box + 4096u * (nbox++ & 1u), &tmC, col0, prow, lane,
                                     [&](int g) { return make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]); });
                 }
             } else
@@ -299,8 +300,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                     const tt::bf16x8 pk = tt::pack8(o);
                     return *reinterpret_cast<const uint4*>(&pk);
                 };
-                if (EPI == 1 || EPI == 2) store_box_32x64(box, &tmAux, col0, row0, lane, [&](int g) { return packed(g, true); });
-                store_box_32x64(box + ((EPI == 1 || EPI == 2 || (c & 1)) ? 4096u : 0u), &tmC, col0, row0, lane,
+                if (EPI == 1 || EPI == 2) store_box_32x64(box + 4096u * (nbox++ & 1u), &tmAux, col0, row0, lane, [&](int g) { return packed(g, true); });
+                store_box_32x64(box + 4096u * (nbox++ & 1u), &tmC, col0, row0, lane,
                                 [&](int g) { return packed(g, false); });
             }
             tc_fence_before();

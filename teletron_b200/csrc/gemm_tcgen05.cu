@@ -333,6 +333,7 @@ gemm_kernel(const __grid_constant__ TmapArray tmA, const __grid_constant__ CUten
             }
             __syncwarp();       // the staging block is reused by the next call
         };
+        uint32_t nbox = 0;       // boxes alternate across tiles too: a tile may store an odd number of them
         int it = 0;
         for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
             int seg, m0, n0;
@@ -520,8 +521,8 @@ gemm_kernel(const __grid_constant__ TmapArray tmA, const __grid_constant__ CUten
                             const tt::bf16x8 pk = tt::pack8(o);
                             return *reinterpret_cast<const uint4*>(&pk);
                         };
-                        if (EPI == 1 || EPI == 2) store_box_32x64(box, &tmAux, col0, row0, lane, [&](int g) { return packed(g, true); });
-                        store_box_32x64(box + ((EPI == 1 || EPI == 2 || (c & 1)) ? 4096u : 0u), &tmC, col0, row0, lane,
+                        if (EPI == 1 || EPI == 2) store_box_32x64(box + 4096u * (nbox++ & 1u), &tmAux, col0, row0, lane, [&](int g) { return packed(g, true); });
+                        store_box_32x64(box + 4096u * (nbox++ & 1u), &tmC, col0, row0, lane,
                                         [&](int g) { return packed(g, false); });
                     }
                 } else

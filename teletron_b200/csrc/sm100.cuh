@@ -118,7 +118,7 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 // rows, 16-byte pieces XOR-swizzled by row as SWIZZLE_128B expects; lane = row).  `o(g, f)` yields columns [8 g, 8 g + 8).
 template <typename F>
 __device__ __forceinline__ void store_box_32x64(uint32_t box, const CUtensorMap* tmap, int col, int row, int lane, F&& o) {
-    // two boxes per warp: the group before last, which used this one, has been read
+    // the caller alternates between two boxes: the group before last, which used this one, has been read
     if (lane == 0) bulk_wait_read<1>();
     __syncwarp();
 #pragma unroll

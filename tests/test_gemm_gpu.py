@@ -234,3 +234,20 @@ def test_two_operands_side_by_side(M, k1, k2, N, splits, monkeypatch):
     assert torch.equal(c, G.gemm(cat, b, "nt", bias))
     assert not G.two_supported(a[:, :k1 - 8], a2, b[:, 8:])
     G.check_status()
+
+
+@pytest.mark.parametrize("M,N,K,pair", [(40005, 64, 64, False), (40005, 72, 72, False), (30005, 320, 64, True), (700, 264, 64, True)])
+def test_epilogue_boxes_over_many_tiles(M, N, K, pair, monkeypatch):
+    """Short products with an odd number of 64-column boxes a tile, several tiles a CTA: the two staging boxes of a warp
+    alternate over tile boundaries, also when the pre-activation is stored beside the output."""
+    from teletron_b200.ops import gemm_tcgen05 as G
+    monkeypatch.setattr(G, "use_pair_kernel", lambda *a: pair)
+    monkeypatch.setattr(G, "_plan", lambda *a: (pair, 1))
+    g = torch.Generator(device="cuda").manual_seed(N)
+    a, w, bias = _mk((M, K), g), _mk((N, K), g, 0.05), _mk((N,), g)
+    ref = a.float() @ w.float().t() + bias.float()
+    for _ in range(3):
+        assert _rel(G.gemm(a, w, "nt", bias), ref) < 3e-3
+        y, u = G.gemm(a, w, "nt", bias, epi=1)
+        assert _rel(u, ref) < 3e-3 and _rel(y, torch.nn.functional.gelu(ref)) < 4e-3
+    G.check_status()
