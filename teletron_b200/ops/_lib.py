@@ -53,6 +53,14 @@ def _load() -> Optional[ctypes.CDLL]:
         _err = str(e)
         return None
     lib.tt_last_cuda_error.restype = ctypes.c_char_p
+    # The GEMM entry points are called hundreds of times a step: with declared argument types they take plain integers, which
+    # spares a ctypes object per argument (the wrappers of the other calls are accepted as well).  The text MLP and a 512 x 512
+    # image's sampling step, which wait for the host, took 2 - 4 % longer without.
+    vp, ci, cl = ctypes.c_void_p, ctypes.c_int, ctypes.c_long
+    for name in ("tt_gemm_bf16", "tt_gemm2_bf16"):
+        getattr(lib, name).argtypes = [vp] * 5 + [ci] * 3 + [cl] * 3 + [ci] * 3 + [vp] * 2
+    lib.tt_gemm2_bf16_splitk.argtypes = [vp] * 5 + [ci] * 3 + [cl] * 3 + [ci] * 4 + [vp] * 3
+    lib.tt_gemm2_bf16_two.argtypes = [vp] * 5 + [ci] * 4 + [cl] * 4 + [ci] + [vp] * 3
     _lib = lib
     return lib
 
@@ -81,12 +89,16 @@ _CUR_DEVICE = getattr(torch._C, "_cuda_getDevice", None)
 
 
 def stream() -> ctypes.c_void_p:
+    return ctypes.c_void_p(raw_stream())
+
+
+def raw_stream() -> int:
     """The current CUDA stream of the current device as a raw handle.  Every native call asks for it, so it goes
     through the two C entry points directly: ``torch.cuda.current_stream()`` resolves its device argument through
     ``device_count()``, which was measured at ~45 us per call (0.7 s over 15 700 native calls of six training steps)."""
     if _RAW_STREAM is not None and _CUR_DEVICE is not None:
-        return ctypes.c_void_p(_RAW_STREAM(_CUR_DEVICE()))
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _RAW_STREAM(_CUR_DEVICE())
+    return torch.cuda.current_stream().cuda_stream
 
 
 def check(t: torch.Tensor, dtype: torch.dtype, name: str, device: Optional[torch.device] = None, align: int = 16) -> torch.Tensor:
@@ -156,7 +168,7 @@ class phase:
 def call(fn_name: str, *args) -> None:
     """Invoke ``tt_<fn_name>`` and raise on a non-zero status."""
     global LAUNCHES
-    fn = getattr(lib(), fn_name)
+    fn = getattr(_lib if _lib is not None else lib(), fn_name)
     if _PROFILE is not None:
         with phase(fn_name):
             rc = fn(*args)

@@ -12,7 +12,7 @@ from typing import Optional
 
 import torch
 
-from . import _lib
+from . import _lib, gemm, gemm_tcgen05
 from ._lib import c_float, c_int, c_long, call, check, ptr, stream
 
 BF16 = torch.bfloat16
@@ -194,19 +194,16 @@ def rmsnorm(x, weight, eps=1e-6):
 
 def _gemm_nt(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``a [M, K] @ b [N, K]^T (+ bias)``."""
-    from . import gemm
     return gemm.gemm_nt(a, b, bias)
 
 
 def _gemm_nn(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     """``a [M, K] @ b [K, N]``."""
-    from . import gemm
     return gemm.gemm_nn(a, b)
 
 
 def _gemm_tn(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     """``a [K, M]^T @ b [K, N]`` (weight gradients)."""
-    from . import gemm
     return gemm.gemm_tn(a, b)
 
 
@@ -237,7 +234,6 @@ class _Linear(torch.autograd.Function):
         if activation is not None and _FUSE_GELU_EPILOGUE:
             # bias + GELU in the GEMM epilogue: the accumulator is activated in fp32 and the kernel writes both the
             # activated output and the bf16 pre-activation that the backward needs
-            from . import gemm, gemm_tcgen05
             if gemm.get_backend() != "cublas" and gemm_tcgen05.supported(x2, weight, "nt"):
                 gemm.COUNTERS["tcgen05"] += 1
                 y, u = gemm_tcgen05.gemm(x2, weight, "nt", bias, epi=1 + _GELU_KIND[activation])
@@ -291,7 +287,6 @@ class _LinearMerged(torch.autograd.Function):
     def forward(ctx, x1, x2, weight, bias):
         k1, k2 = x1.shape[-1], x2.shape[-1]
         a1, a2 = x1.reshape(-1, k1), x2.reshape(-1, k2)
-        from . import gemm, gemm_tcgen05
         if gemm.get_backend() != "cublas" and gemm_tcgen05.two_supported(a1, a2, weight):
             gemm.COUNTERS["tcgen05"] += 1
             y = gemm_tcgen05.gemm_two(a1, a2, weight, bias)
@@ -304,7 +299,6 @@ class _LinearMerged(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        from . import gemm
         a1, a2, weight = ctx.saved_tensors
         k1 = a1.shape[1]
         du = dy.reshape(-1, weight.shape[0])

@@ -19,6 +19,8 @@ from typing import Optional
 
 import torch
 
+from . import gemm_tcgen05
+
 _BACKEND = os.environ.get("TELETRON_B200_GEMM", "auto")
 COUNTERS = {"tcgen05": 0, "cublas": 0}
 
@@ -37,7 +39,6 @@ def get_backend() -> str:
 def _native(a: torch.Tensor, b: torch.Tensor, layout: str, bias: Optional[torch.Tensor]):
     if _BACKEND == "cublas":
         return None
-    from . import gemm_tcgen05
     if not gemm_tcgen05.supported(a, b, layout):
         if _BACKEND == "tcgen05":
             raise RuntimeError(f"tcgen05 GEMM does not take {layout} {tuple(a.shape)} x {tuple(b.shape)}")
@@ -77,7 +78,6 @@ def gemm_tn(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
 def gemm_tn_into(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """``out[:] = a.T @ b`` where ``out`` may be a column slice of a larger row-major matrix."""
     if _BACKEND != "cublas":
-        from . import gemm_tcgen05
         if gemm_tcgen05.supported(a, b, "tn") and out.stride(1) == 1 and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0:
             COUNTERS["tcgen05"] += 1
             gemm_tcgen05.gemm(a, b, "tn", out=out)

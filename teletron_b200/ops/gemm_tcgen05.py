@@ -19,7 +19,7 @@ from typing import Dict, Optional, Tuple
 import torch
 
 from . import _lib
-from ._lib import c_int, c_long, call, ptr, stream
+from ._lib import call
 
 BF16 = torch.bfloat16
 _LAYOUTS = {"nt": (0, 0), "nn": (0, 1), "tn": (1, 1)}
@@ -78,7 +78,10 @@ def check_status(device: Optional[torch.device] = None) -> None:
 
 
 def _rowmajor(t: torch.Tensor) -> bool:
-    return t.dim() == 2 and t.stride(1) == 1 and t.stride(0) >= t.shape[1] and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+    if t.dim() != 2:
+        return False
+    s0, s1 = t.stride()
+    return s1 == 1 and s0 >= t.shape[1] and s0 % 8 == 0 and t.data_ptr() % 16 == 0
 
 
 def _dims(a: torch.Tensor, b: torch.Tensor, layout: str) -> Tuple[int, int, int]:
@@ -107,9 +110,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, layout: str, bias: Optional[torch.Ten
     """Returns ``C`` (and the pre-activation tensor for ``epi`` 1 / 2)."""
     M, N, K = _dims(a, b, layout)
     a_mn, b_mn = _LAYOUTS[layout]
-    c = out if out is not None else torch.empty(M, N, dtype=BF16, device=a.device)
+    dev = a.device
+    c = out if out is not None else torch.empty(M, N, dtype=BF16, device=dev)
     if epi in (1, 2):
-        aux = torch.empty(M, N, dtype=BF16, device=a.device)
+        aux = torch.empty(M, N, dtype=BF16, device=dev)
     elif epi in (3, 4):
         if aux is None or aux.shape != (M, N) or not aux.is_contiguous():
             raise _lib.NativeError("epilogue 3/4 needs a contiguous [M, N] pre-activation tensor")
@@ -118,17 +122,15 @@ def gemm(a: torch.Tensor, b: torch.Tensor, layout: str, bias: Optional[torch.Ten
     pair, splits = use_pair_kernel(M, N), 1
     if PAIR_KERNEL and not pair:
         pair, splits = _plan(M, N, K)
+    args = (a.data_ptr(), b.data_ptr(), c.data_ptr(), None if bias is None else bias.data_ptr(), None if aux is None else aux.data_ptr(),
+            M, N, K, a.stride(0), b.stride(0), c.stride(0), a_mn, b_mn, epi)
     if splits > 1:
         COUNTERS["split"] += 1
-        scratch = torch.empty(splits * ((M + 31) // 32 * 32) * N, dtype=torch.float32, device=a.device)
-        call("tt_gemm2_bf16_splitk", ptr(a), ptr(b), ptr(c), ptr(bias), ptr(aux), c_int(M), c_int(N), c_int(K), c_long(a.stride(0)),
-             c_long(b.stride(0)), c_long(c.stride(0)), c_int(a_mn), c_int(b_mn), c_int(epi), c_int(splits), ptr(scratch),
-             ptr(status_tensor(a.device)), stream())
-        return (c, aux) if epi in (1, 2) else c
-    COUNTERS["pair" if pair else "single"] += 1
-    call("tt_gemm2_bf16" if pair else "tt_gemm_bf16", ptr(a), ptr(b), ptr(c), ptr(bias), ptr(aux), c_int(M), c_int(N), c_int(K), c_long(a.stride(0)),
-         c_long(b.stride(0)), c_long(c.stride(0)), c_int(a_mn), c_int(b_mn), c_int(epi), ptr(status_tensor(a.device)),
-         stream())
+        scratch = torch.empty(splits * ((M + 31) // 32 * 32) * N, dtype=torch.float32, device=dev)
+        call("tt_gemm2_bf16_splitk", *args, splits, scratch.data_ptr(), status_tensor(dev).data_ptr(), _lib.raw_stream())
+    else:
+        COUNTERS["pair" if pair else "single"] += 1
+        call("tt_gemm2_bf16" if pair else "tt_gemm_bf16", *args, status_tensor(dev).data_ptr(), _lib.raw_stream())
     return (c, aux) if epi in (1, 2) else c
 
 
@@ -148,7 +150,8 @@ def gemm_two(a: torch.Tensor, a2: torch.Tensor, b: torch.Tensor, bias: Optional[
     splits = 1 if use_pair_kernel(M, N) else _plan(M, N, K)[1]
     COUNTERS["pair" if splits == 1 else "split"] += 1
     scratch = None if splits == 1 else torch.empty(splits * ((M + 31) // 32 * 32) * N, dtype=torch.float32, device=a.device)
-    call("tt_gemm2_bf16_two", ptr(a), ptr(a2), ptr(b), ptr(c), ptr(bias), c_int(M), c_int(N), c_int(K), c_int(k1), c_long(a.stride(0)),
-         c_long(a2.stride(0)), c_long(b.stride(0)), c_long(c.stride(0)), c_int(splits), ptr(scratch), ptr(status_tensor(a.device)), stream())
+    call("tt_gemm2_bf16_two", a.data_ptr(), a2.data_ptr(), b.data_ptr(), c.data_ptr(), None if bias is None else bias.data_ptr(), M, N, K, k1,
+         a.stride(0), a2.stride(0), b.stride(0), c.stride(0), splits, None if scratch is None else scratch.data_ptr(),
+         status_tensor(a.device).data_ptr(), _lib.raw_stream())
     _lib.LAUNCHES += splits > 1      # the pass over the slices
     return c
