@@ -52,7 +52,10 @@ struct AttnParams {
     int kv_len;           // keys >= kv_len are masked
     int mask_lo, mask_hi; // keys in [mask_lo, mask_hi) are masked as well (padded text tokens that are not the sequence tail)
     int H;                // heads (for the output layout)
-    float scale_log2;     // softmax scale * log2(e)
+    // softmax scale * log2(e) = pre_scale * scale_log2.  A masked score is -inf before scale_log2 is applied, and the row maximum is
+    // taken there too, so scale_log2 has to be positive: a scale of zero or below goes into pre_scale whole (scale_log2 = 1),
+    // which multiplies the scores first; a positive one leaves pre_scale at 1.
+    float scale_log2, pre_scale;
     int* status;
     // Ulysses head -> sequence all-to-all fused into the epilogue (batch 1): besides the local copy, every output row
     // is stored into the gathered buffer [text_len + s_local, dest_ld] of the rank that owns that token (text rows,
@@ -227,6 +230,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
             for (int c = 0; c < BKV / 32; ++c) tmem_ld_32x32(tS + c * 32, r + c * 32);
             tmem_ld_wait();
+            if (p.pre_scale != 1.f) {
+#pragma unroll
+                for (int i = 0; i < BKV; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * p.pre_scale);
+            }
             if (!full_tile) {
 #pragma unroll
                 for (int i = 0; i < BKV; ++i)
@@ -408,7 +415,8 @@ static int attn_fwd_launch(const void* q, const void* k, const void* v, void* ou
     p.mask_lo = mask_lo;
     p.mask_hi = mask_lo < mask_hi ? mask_hi : mask_lo;
     p.H = H;
-    p.scale_log2 = scale * 1.4426950408889634f;
+    p.pre_scale = scale > 0.f ? 1.f : scale * 1.4426950408889634f;
+    p.scale_log2 = scale > 0.f ? scale * 1.4426950408889634f : 1.f;
     p.status = status;
     p.push = peer_out != nullptr ? 1 : 0;
     p.n_peers = n_peers;

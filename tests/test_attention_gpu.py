@@ -107,6 +107,28 @@ def test_masked_key_range_forward_and_backward(S, kv_len, mask, bwd_variant):
     assert float(v.grad[:, :, mask[0]:mask[1]].float().abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("S,kv_len,mask", [(256, None, None), (300, None, None), (700, 650, None), (384, None, (0, 128)), (640, 600, (100, 300))])
+@pytest.mark.parametrize("scale", [0.0, -0.05, -0.6])
+def test_scale_of_zero_and_below(S, kv_len, mask, scale, bwd_variant):
+    """Masked keys stay out whatever the scale's sign is: with tiles that are whole, ragged, partly and wholly masked (the
+    first one, too), and with scores (-0.6) whose range is beyond what exp2 takes without the running maximum."""
+    from teletron_b200 import ops
+    from teletron_b200.ops import reference
+    from teletron_b200.ops.gemm_tcgen05 import check_status
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v = (torch.randn(1, 2, S, 128, device="cuda", generator=g).bfloat16().requires_grad_() for _ in range(3))
+    d = torch.randn(1, S, 256, device="cuda", generator=g).bfloat16()
+    o = ops.attention(q, k, v, kv_len, scale, mask)
+    o.backward(d)
+    check_status()
+    refs = [t.detach().double().requires_grad_() for t in (q, k, v)]
+    ro = reference.attention(*refs, kv_len, scale, mask)
+    ro.backward(d.double())
+    assert _rel(o, ro) < 1.2e-2
+    for a, r in zip((q, k, v), refs):
+        assert _rel(a.grad, r.grad) < 2e-2
+
+
 def test_forward_and_backward_are_bitwise_reproducible(bwd_variant):
     """The forward, dK and dV have a fixed accumulation order in both variants; so has dQ in the two-kernel split:
     repeated launches on the same inputs give the same bits (also a cheap detector of ordering races between the
