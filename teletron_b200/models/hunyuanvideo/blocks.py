@@ -420,17 +420,19 @@ class SingleAttention(nn.Module):
         self.q_layernorm = RMSNorm(head_dim, eps, tp > 1, **kw)
         self.k_layernorm = RMSNorm(head_dim, eps, tp > 1, **kw)
 
-    def forward(self, h, text_len, cos, sin, pad, kv_valid_len, in_region: bool = False):
-        """Token-major ``[B, S + T, heads * head_dim]``, video tokens first."""
+    def forward(self, h, text_len, cos, sin, pad, kv_valid_len, in_region: bool = False, joined: bool = False):
+        """Token-major ``(video [B, S, heads * head_dim], text [B, T, ...])``; with ``joined`` the two as one tensor, video tokens
+        first, which on a single context-parallel rank is what attention writes anyway."""
         if not in_region:
             h = M.copy_to_tensor_model_parallel_region(h, ps.get_tensor_model_parallel_group())
         s = h.shape[1] - text_len
         q, k, v = ops.qkv_projection(h, self.linear_qkv.weight, self.linear_qkv.bias, self.q_layernorm.weight,
                                      self.k_layernorm.weight, cos, sin, self.heads_local, self.eps, rope_len=s)
         if ps.get_context_parallel_world_size() == 1:
-            return ops.attention(q, k, v, kv_valid_len=None if kv_valid_len is None else s + kv_valid_len)
-        return torch.cat(_ulysses_attention(q[:, :, :s], k[:, :, :s], v[:, :, :s], q[:, :, s:], k[:, :, s:], v[:, :, s:],
-                                            pad, kv_valid_len), dim=1)
+            o = ops.attention(q, k, v, kv_valid_len=None if kv_valid_len is None else s + kv_valid_len)
+            return o if joined else M.split_tokens(o, s)
+        o = _ulysses_attention(q[:, :, :s], k[:, :, :s], v[:, :, :s], q[:, :, s:], k[:, :, s:], v[:, :, s:], pad, kv_valid_len)
+        return torch.cat(o, dim=1) if joined else o
 
 
 # ---------------------------------------------------------------------------------------------
@@ -506,7 +508,7 @@ class HunyuanSingleDiTLayer(nn.Module):
         if _use_fused(hn, self.self_attention.head_dim):
             proj = self._attention_and_projection_fused(hn, mlp, T, cos, sin, pad, kv_valid_len, in_region=sp)
         else:
-            attn = self.self_attention(hn, T, cos, sin, pad, kv_valid_len, in_region=sp)
+            attn = self.self_attention(hn, T, cos, sin, pad, kv_valid_len, in_region=sp, joined=True)
             proj = self.proj_out.forward_merged(attn, mlp, row_splits=splits)
         h = ops.gate_residual(h, proj, gate)
         return M.split_tokens(h, h.shape[1] - T_own)

@@ -483,6 +483,17 @@ def test_linear_merged_matches_linear_of_the_concatenation():
     assert x1.grad.shape == x1.shape and x2.grad.shape == x2.shape and w.grad.shape == w.shape
 
 
+def test_single_attention_returns_video_and_text_apart():
+    """The module's result is the pair of streams; joined, it is their concatenation."""
+    from teletron_b200.models.hunyuanvideo.blocks import SingleAttention
+    g = torch.Generator().manual_seed(2)
+    sa = SingleAttention(64, 2, 32, 1, 1e-6)
+    h = torch.randn(2, 11, 64, generator=g)
+    res = sa(h, 4, None, None, None, 3)
+    assert isinstance(res, tuple) and [tuple(t.shape) for t in res] == [(2, 7, 64), (2, 4, 64)]
+    torch.testing.assert_close(torch.cat(res, 1), sa(h, 4, None, None, None, 3, joined=True))
+
+
 def test_read_video_decodes_a_container_file_with_opencv(tmp_path):
     """Without ``decord`` the dataset decodes ``.mp4`` / ``.avi`` clips through OpenCV: frame count, requested indices
     (wrapping past the end) and RGB channel order."""
