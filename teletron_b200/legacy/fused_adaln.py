@@ -40,6 +40,8 @@ def torch_launch_adaln_backward(dx, dscale, dshift, dout, x_norm, scale, invvar,
     check(invvar, torch.float32, "invvar")
     if dx.numel() != rows * cols or min(scale.numel(), dscale.numel(), dshift.numel()) < cols:
         raise _lib.NativeError("shape mismatch")
+    if invvar.shape == (1,) and rows > 1:
+        invvar = invvar.repeat(rows)        # one statistic for all rows
     _check_rows(invvar, rows, cols, dout, x_norm)
     nblk = _lib.lib().tt_norm_partial_blocks(c_long(rows), c_int(1))
     partials = torch.empty(nblk * 2 * cols, dtype=torch.float32, device=dx.device)

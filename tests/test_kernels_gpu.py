@@ -309,6 +309,20 @@ def test_drop_in_adaln_saves_and_consumes_normalised_rows(rows, cols):
         fused_adaln.torch_launch_adaln_forward(y, x, scale, shift, xn, rstd[:-1] if rows > 1 else rstd[:0], rows, cols)
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 264), (12, 264), (9, 8192)])
+def test_drop_in_adaln_backward_takes_one_statistic_for_all_rows(rows, cols):
+    """An ``invvar`` of one element is spread over the rows, as an elementwise product does."""
+    from teletron_b200.legacy import fused_adaln
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    dy, xn, scale = (torch.randn(*s, device=_dev(), generator=g).bfloat16() for s in ((rows, cols), (rows, cols), (cols,)))
+    res = []
+    for rstd in (torch.tensor([1.7], device=_dev()), torch.full((rows,), 1.7, device=_dev())):
+        dx, dscale, dshift = torch.empty_like(dy), torch.empty_like(scale), torch.empty_like(scale)
+        fused_adaln.torch_launch_adaln_backward(dx, dscale, dshift, dy, xn, scale, rstd, rows, cols)
+        res.append((dx, dscale, dshift))
+    assert all(torch.equal(a, b) for a, b in zip(*res))
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 8), (31, 256), (33, 264), (257, 3072), (1037, 9216), (5000, 64)])
 @pytest.mark.parametrize("act", [None, "gelu", "gelu_tanh"])
 def test_bias_gradient_column_sums(rows, cols, act):
