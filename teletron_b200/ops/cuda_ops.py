@@ -11,6 +11,7 @@ import os
 from typing import Optional
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib, gemm, gemm_tcgen05
 from ._lib import c_float, c_int, c_long, call, check, ptr, stream
@@ -207,10 +208,16 @@ def _gemm_tn(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     return gemm.gemm_tn(a, b)
 
 
+def _transformed(t: torch.Tensor) -> bool:
+    """``t`` is differentiated again (``create_graph``), batched (``is_grads_batched``) or may carry a forward-mode tangent: what
+    a kernel writes through raw pointers has no part in that."""
+    return (torch.is_grad_enabled() and t.requires_grad) or forward_ad._current_level >= 0 or not torch._C._has_storage(t)
+
+
 def _bias_grad(du: torch.Tensor) -> torch.Tensor:
     """Column sums of ``du [rows, cols]`` in fp32, rounded once."""
     rows, cols = du.shape
-    if cols % 8 or not du.is_contiguous() or du.dtype != BF16 or du.data_ptr() % 16 or rows == 0:
+    if _transformed(du) or cols % 8 or not du.is_contiguous() or du.dtype != BF16 or du.data_ptr() % 16 or rows == 0:
         return du.sum(dim=0, dtype=torch.float32).to(du.dtype)
     db = torch.empty(cols, dtype=BF16, device=du.device)
     _colsum(du, None, None, db, rows, cols, 2)

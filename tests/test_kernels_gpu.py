@@ -344,3 +344,24 @@ def test_bias_gradient_column_sums(rows, cols, act):
     want = du.double().sum(0)
     # one bf16 rounding of the sum plus fp32 summation error, which is relative to the sum of magnitudes
     assert ((db.double() - want).abs() <= want.abs() * 2.0 ** -8 + du.double().abs().sum(0) * 2e-6).all()
+
+
+@pytest.mark.parametrize("merged", [False, True])
+def test_bias_gradient_of_transformed_gradients(merged):
+    """A bias gradient that is differentiated again, batched or given a tangent is an ordinary sum over the rows."""
+    import torch.autograd.forward_ad as fwd
+    from teletron_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rn = lambda *s: torch.randn(*s, device=_dev(), generator=g).bfloat16()  # noqa: E731
+    x, w, b = rn(32, 128), rn(256, 128), rn(256).requires_grad_()
+    y = ops.linear_merged(x[:, :64], x[:, 64:], w, b) if merged else ops.linear(x, w, b)
+    dy = rn(32, 256).requires_grad_()
+    (gb,) = torch.autograd.grad(y, b, dy, create_graph=True)
+    (gg,) = torch.autograd.grad(gb, dy, torch.ones_like(gb))
+    assert torch.equal(gg, torch.ones_like(dy))
+    (gb,) = torch.autograd.grad(y, b, torch.stack([dy, 2 * dy]).detach(), is_grads_batched=True, retain_graph=True)
+    ref = dy.detach().double().sum(0)
+    assert _rel(gb[0], ref) < 4e-3 and torch.equal(gb[1], 2 * gb[0])
+    with fwd.dual_level():
+        (gb,) = torch.autograd.grad(y, b, fwd.make_dual(dy.detach(), torch.ones_like(dy)), retain_graph=True)
+        assert torch.equal(fwd.unpack_dual(gb).tangent, torch.full_like(b, 32.0))
