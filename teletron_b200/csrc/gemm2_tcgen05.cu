@@ -329,18 +329,16 @@ done:
 
 template <bool A_MN, bool B_MN, int EPI>
 int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmAux, const CUtensorMap& tmA2,
-            const Params2& p, int sms, cudaStream_t st) {
+            const Params2& p, const tt_device_info& on, cudaStream_t st) {
     auto kern = gemm2_kernel<A_MN, B_MN, EPI>;
     static bool configured[64] = {false};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-    if (!configured[dev]) {
+    if (!configured[on.dev]) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
         if (e != cudaSuccess) return tt_record_cuda(e);
-        configured[dev] = true;
+        configured[on.dev] = true;
     }
     const int tiles = p.tiles_m * p.tiles_n * p.splits;
-    int pairs = sms / 2;
+    int pairs = on.sms / 2;
     if (pairs > tiles) pairs = tiles;
     if (pairs < 1) pairs = 1;
     kern<<<2 * pairs, kThreads, kSmemBytes, st>>>(tmA, tmB, tmC, tmAux, tmA2, p);      // cluster shape comes from __cluster_dims__
@@ -393,8 +391,8 @@ int run2(const void* a, const void* a2, int k1, long lda2, const void* b, void* 
     if (a2 != nullptr && (a_mn || k1 <= 0 || k1 >= K || (k1 % BK))) return TT_ERR_ARG;
     const int kblocks = (K + BK - 1) / BK;
     if (splits < 1 || splits > kblocks || (splits > 1 && (scratch == nullptr || ((uintptr_t)scratch & 15)))) return TT_ERR_ARG;
-    int dev = 0, sms = 148, rc;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const tt_device_info on = tt_device();
+    int rc;
     CUtensorMap tmA, tmA2, tmB, tmC, tmAux;
     if (!a_mn) rc = tt_make_tmap_2d(&tmA, a, (uint64_t)M, (uint64_t)(a2 != nullptr ? k1 : K), (uint64_t)lda, BMH, BK);
     else rc = tt_make_tmap_2d(&tmA, a, (uint64_t)K, (uint64_t)M, (uint64_t)lda, 64, 64);
@@ -424,7 +422,7 @@ int run2(const void* a, const void* a2, int k1, long lda2, const void* b, void* 
         if ((rc = tt_make_tmap_2d(&tmC, c, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64)) != TT_OK) return rc;
         tmAux = tmC;
         if ((epi == 1 || epi == 2) && (rc = tt_make_tmap_2d(&tmAux, aux, (uint64_t)M, (uint64_t)N, (uint64_t)ldc, 32, 64)) != TT_OK) return rc;
-#define GO(A_, B_, E_) return launch2<A_, B_, E_>(tmA, tmB, tmC, tmAux, tmA2, p, sms, st)
+#define GO(A_, B_, E_) return launch2<A_, B_, E_>(tmA, tmB, tmC, tmAux, tmA2, p, on, st)
         if (!amn && !bmn) {
             if (epi == 0) GO(false, false, 0);
             if (epi == 1) GO(false, false, 1);
@@ -440,9 +438,9 @@ int run2(const void* a, const void* a2, int k1, long lda2, const void* b, void* 
         return TT_ERR_ARG;
     }
     if ((rc = tt_make_tmap_2d_f32(&tmC, scratch, (uint64_t)p.part_rows * p.splits, (uint64_t)N, (uint64_t)N, 32, 32)) != TT_OK) return rc;
-    if (!amn && !bmn) rc = launch2<false, false, 7>(tmA, tmB, tmC, tmC, tmA2, p, sms, st);
-    else if (!amn) rc = launch2<false, true, 7>(tmA, tmB, tmC, tmC, tmA2, p, sms, st);
-    else rc = launch2<true, true, 7>(tmA, tmB, tmC, tmC, tmA2, p, sms, st);
+    if (!amn && !bmn) rc = launch2<false, false, 7>(tmA, tmB, tmC, tmC, tmA2, p, on, st);
+    else if (!amn) rc = launch2<false, true, 7>(tmA, tmB, tmC, tmC, tmA2, p, on, st);
+    else rc = launch2<true, true, 7>(tmA, tmB, tmC, tmC, tmA2, p, on, st);
     if (rc != TT_OK) return rc;
     const long want = ((long)M * (N >> 3) + 255) / 256;
     const int grid = (int)(want < 148L * 8 ? want : 148L * 8);

@@ -628,18 +628,20 @@ int dispatch(bool a_mn, bool b_mn, int epi, const TmapArray& tmA, const CUtensor
 
 int g_sms[64] = {0};
 
-int sm_count() {
+int sm_count() { return tt_device().sms; }
+
+}  // namespace
+
+tt_device_info tt_device() {
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return {0, 148};
     if (g_sms[dev] == 0) {
         int n = 0;
         if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
         g_sms[dev] = n;
     }
-    return g_sms[dev];
+    return {dev, g_sms[dev]};
 }
-
-}  // namespace
 
 // ---------------------------------------------------------------------------------------------
 // tensor-map helpers (shared with the attention kernels)

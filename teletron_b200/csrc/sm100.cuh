@@ -245,6 +245,12 @@ typedef CUresult (*tt_encode_tiled_fn)(CUtensorMap*, CUtensorMapDataType, cuuint
                                        CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 tt_encode_tiled_fn tt_get_encode_tiled();
 
+// The current device (0 if it cannot be told or lies beyond the per-device tables of 64) and its SM count, which is asked for
+// once per device.
+struct tt_device_info {
+    int dev, sms;
+};
+tt_device_info tt_device();
 // 2-D bf16 tensor [rows, cols] (cols contiguous, row pitch `ld` elements), box [box_rows, box_cols], 128B swizzle.
 int tt_make_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
                     uint32_t box_cols);
