@@ -28,6 +28,8 @@ _LAYOUTS = {"nt": (0, 0), "nn": (0, 1), "tn": (1, 1)}
 PAIR_KERNEL = os.environ.get("TELETRON_B200_GEMM_2CTA", "1") != "0"
 PAIR_MIN_TILES = 74
 COUNTERS = {"pair": 0, "single": 0, "split": 0}
+# What a split product takes the host to issue: a scratch allocation and a second launch on top of the 12.4 us of the others.
+SPLIT_ISSUE_US = 17.5
 
 
 def use_pair_kernel(M: int, N: int) -> bool:
@@ -43,11 +45,17 @@ def _plan(M: int, N: int, K: int) -> Tuple[bool, int]:
     (32 KB through L2 per SM set the pace); a wave of 74 pair tiles takes 0.30 (four times the tile on twice the SMs: the
     tensor core does); a split product adds a second launch and one write and read of its fp32 slices.  Examples, single /
     pair / best split: 256 x 3072 x 12288 45.7 / 62.2 / 25.5 (6 splits); 256 x 12288 x 3072 28.1 / 23.0 / 29.0;
-    256 x 9216 x 3072 17.4 / 22.0 / 21.6; 1024 x 3072 x 12288 85.8 / 67.8 / 61.1 (3); 512 x 3072 x 4096 18.8 / 25.9 / 18.8."""
+    256 x 9216 x 3072 17.4 / 22.0 / 21.6; 1024 x 3072 x 12288 85.8 / 67.8 / 61.1 (3); 512 x 3072 x 4096 18.8 / 25.9 / 18.8.  cuBLAS
+    takes 21.8, 18.9, 14.7, 55.3 and 13.1 for these, and 8.0 where the best here is 14.0 (256 x 3072 x 3072).
+
+    A product that is through before a split one could be issued is not split: 40 x 3072 x 3072 would take 11.6 us instead of
+    12.6, but calls in a row one every 17.5 us instead of every 12.6."""
     kb, t1, t2 = (K + 63) // 64, ((M + 127) // 128) * ((N + 127) // 128), ((M + 255) // 256) * ((N + 255) // 256)
     waves = (t1 + 147) // 148
     best = (4 + waves * kb * (0.22 if waves == 1 else 0.26), False, 1)
     for s in range(1, min(16, kb // 4) + 1):
+        if s == 2 and best[0] < SPLIT_ISSUE_US:
+            break
         cost = 5 + ((t2 * s + 73) // 74) * ((kb + s - 1) // s) * 0.30
         if s > 1:
             cost += 5 + 0.13e-6 * (s * ((M + 31) // 32 * 32) * N * 8)

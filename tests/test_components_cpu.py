@@ -494,6 +494,24 @@ def test_single_attention_returns_video_and_text_apart():
     torch.testing.assert_close(torch.cat(res, 1), sa(h, 4, None, None, None, 3, joined=True))
 
 
+def test_plan_of_small_products():
+    """Which kernel a product with few tiles takes: the documented choices, and what holds for any size."""
+    from teletron_b200.ops import gemm_tcgen05 as G
+    plan = G._plan.__wrapped__
+    for shape, want in {(256, 3072, 12288): (True, 6), (256, 12288, 3072): (True, 1), (256, 9216, 3072): (False, 1),
+                        (1024, 3072, 12288): (True, 3), (512, 3072, 4096): (False, 1), (40, 3072, 12288): (True, 6),
+                        (40, 3072, 3072): (False, 1), (1, 8, 8): (False, 1)}.items():
+        assert plan(*shape) == want, shape
+    for M in (1, 8, 33, 256, 300, 1024, 4000):
+        for N in (8, 64, 264, 3072, 12288):
+            for K in (8, 64, 72, 192, 256, 520, 3072, 15360, 60000):
+                if ((M + 255) // 256) * ((N + 255) // 256) >= G.PAIR_MIN_TILES:
+                    continue
+                pair, splits = plan(M, N, K)
+                assert 1 <= splits <= max(1, (K + 63) // 64) and (pair or splits == 1), (M, N, K)
+                assert splits * ((M + 31) // 32 * 32) * N * 4 <= 1 << 29, (M, N, K)       # the scratch of a split product
+
+
 def test_read_video_decodes_a_container_file_with_opencv(tmp_path):
     """Without ``decord`` the dataset decodes ``.mp4`` / ``.avi`` clips through OpenCV: frame count, requested indices
     (wrapping past the end) and RGB channel order."""
