@@ -244,6 +244,34 @@ def test_all_gather_gemm_and_gemm_reduce_scatter(coalesced):
     _lib.lib().tt_set_coalesced_peer_stores(ctypes.c_int(1))
 
 
+@pytest.mark.parametrize("rows", [328, 352, 384, 32])     # segments of no whole, of whole 32-row boxes, of whole tiles, of one box
+@pytest.mark.parametrize("epi", [0, 1, 2])
+def test_all_gather_gemm_stores_stay_in_their_segment(rows, epi):
+    """Segments of a multiple of 32 rows are stored as 32-row boxes, which must end where the segment does: every 32-row block
+    is compared by itself, and what lies behind the last segment is untouched."""
+    c_float, c_int, c_long, call, ptr, stream, check_status, status_tensor = _imports()
+    gen = torch.Generator(device="cuda").manual_seed(rows + epi)
+    n, K, N = 4, 192, 200                                # columns: three whole boxes and one of 8
+    blocks = [_rnd(gen, rows, K) for _ in range(n)]
+    w, bias = _rnd(gen, N, K, scale=0.1), _rnd(gen, N, scale=0.1)
+    pre = torch.cat(blocks).double() @ w.double().t() + bias.double()
+    want = pre if epi == 0 else torch.nn.functional.gelu(pre, approximate="none" if epi == 1 else "tanh")
+    flags = torch.zeros(n * ((rows + 127) // 128), dtype=torch.int32, device="cuda")
+    st = status_tensor(torch.device("cuda", 0))
+    for me in range(n):
+        out = torch.full((n * rows + 64, N), -777.0, device="cuda", dtype=BF16)
+        aux = torch.full_like(out, -777.0)
+        stage = torch.zeros(n * rows, K, device="cuda", dtype=BF16)
+        call("tt_gemm_ag_bf16", table(blocks), c_int(n), c_int(me), c_int(rows), ptr(w), c_int(0), c_long(K), ptr(out), c_long(N),
+             ptr(bias), ptr(aux) if epi else None, c_int(N), c_int(K), c_int(epi), ptr(stage), ptr(flags), c_int(me + 1), ptr(st), stream())
+        torch.cuda.synchronize()
+        for got, ref in ((out, want),) + (((aux, pre),) if epi else ()):
+            assert bool((got[n * rows:] == -777.0).all()), me
+            for r0 in range(0, n * rows, 8):             # 8 divides 328, so no block straddles two segments
+                assert rel(got[r0:r0 + 8], ref[r0:r0 + 8]) < 6e-3, (me, r0)
+    check_status()
+
+
 @pytest.mark.parametrize("state_dtype,master", [(torch.float32, "fp32"), (BF16, "split16")])
 def test_gradient_reduce_scatter_and_fused_adamw_all_gather(state_dtype, master):
     c_float, c_int, c_long, call, ptr, stream, check_status, status_tensor = _imports()
