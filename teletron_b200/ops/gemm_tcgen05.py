@@ -120,6 +120,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, layout: str, bias: Optional[torch.Ten
     a_mn, b_mn = _LAYOUTS[layout]
     dev = a.device
     c = out if out is not None else torch.empty(M, N, dtype=BF16, device=dev)
+    if epi and c.stride(0) != N and M > 1:      # the kernels walk the pre-activation with the pitch of C
+        raise _lib.NativeError("an epilogue with a pre-activation needs a contiguous output")
     if epi in (1, 2):
         aux = torch.empty(M, N, dtype=BF16, device=dev)
     elif epi in (3, 4):

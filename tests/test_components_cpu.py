@@ -512,6 +512,24 @@ def test_plan_of_small_products():
                 assert splits * ((M + 31) // 32 * 32) * N * 4 <= 1 << 29, (M, N, K)       # the scratch of a split product
 
 
+@pytest.mark.parametrize("epi", [1, 2, 3, 4])
+def test_gemm_refuses_an_output_window_beside_a_pre_activation(epi, monkeypatch):
+    """The pre-activation is contiguous and would be walked with the window's pitch, beyond its end."""
+    from teletron_b200.ops import _lib
+    from teletron_b200.ops import gemm_tcgen05 as G
+    launched = []
+    monkeypatch.setattr(G, "call", lambda *a: launched.append(a[0]))
+    monkeypatch.setattr(_lib, "raw_stream", lambda: 0)
+    layout = "nt" if epi < 3 else "nn"
+    a, b, wide = (torch.zeros(16, n, dtype=torch.bfloat16) for n in (16, 16, 32))
+    aux = None if epi < 3 else torch.zeros(16, 16, dtype=torch.bfloat16)
+    with pytest.raises(_lib.NativeError):
+        G.gemm(a, b, layout, epi=epi, aux=aux, out=wide[:, :16])
+    G.gemm(a, b, layout, epi=epi, aux=aux, out=torch.empty(16, 16, dtype=torch.bfloat16))
+    G.gemm(a, b, layout, out=wide[:, :16])
+    assert len(launched) == 2
+
+
 def test_read_video_decodes_a_container_file_with_opencv(tmp_path):
     """Without ``decord`` the dataset decodes ``.mp4`` / ``.avi`` clips through OpenCV: frame count, requested indices
     (wrapping past the end) and RGB channel order."""
