@@ -496,7 +496,7 @@ gemm_kernel(const __grid_constant__ TmapArray tmA, const __grid_constant__ CUten
                         }
                         store_block_coalesced(v, d, min(128, p.N - colb));
                     }
-                } else if (EPI <= 4 && p.tma_store) {
+                } else if (EPI == 3 || EPI == 4 || (EPI <= 2 && p.tma_store)) {      // 3, 4: C is always local and one segment
                     const int row0 = seg * p.seg_rows + m0 + quad * 32;
                     const uint32_t box = epi_stage + (uint32_t)(warp - 2) * 8192u;
                     if (m0 + quad * 32 < p.seg_rows)
@@ -536,13 +536,12 @@ gemm_kernel(const __grid_constant__ TmapArray tmA, const __grid_constant__ CUten
                     for (int g = 0; g < 4; ++g) {
                         const int col = col0 + g * 8;
                         if (row_ok && col + 8 <= p.N) {
-                            float bv[8], uv[8], o[8];
+                            float bv[8], o[8];
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) bv[j] = uv[j] = 0.f;
-                            if (EPI <= 2 && p.bias != nullptr) tt::unpack8(tt::ld8(p.bias + col), bv);
-                            if (EPI >= 3) tt::unpack8(tt::ld8(arow + col), uv);
+                            for (int j = 0; j < 8; ++j) bv[j] = 0.f;
+                            if (p.bias != nullptr) tt::unpack8(tt::ld8(p.bias + col), bv);
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) o[j] = epi_apply<EPI>(__uint_as_float(r[g * 8 + j]), bv[j], uv[j]);
+                            for (int j = 0; j < 8; ++j) o[j] = epi_apply<EPI>(__uint_as_float(r[g * 8 + j]), bv[j], 0.f);
                             if (EPI == 1 || EPI == 2) {
                                 float u[8];
 #pragma unroll
