@@ -485,7 +485,8 @@ done:
 // 2560).  So everything else is kept off it: dV takes P from T1, where it waits for nothing but the exponentials; dP(c+1) is
 // issued the moment dQ(c) has been read; S(c+2) follows dV(c+1) into T1 before dS(c+1) is through; lse and delta arrive
 // in shared memory with their chunk (from L2 they cost ~500 clocks a pass); the MMA warp issues from one elected lane
-// (200 clocks for eight products instead of 650).  24 heads x 32656 tokens: 36.2 -> 33.1 ms, 3 heads x 119056: 62.5 -> 56.4.
+// (200 clocks for eight products instead of 650).  24 heads x 32656 tokens: 36.2 -> 32.6 - 33.7 ms,
+// 3 heads x 119056: 62.5 -> 55.6 - 56.4.
 //
 // Shared memory: K, V resident; two slots each for the streamed Q (with the chunk's lse) and dO (with its delta); one dS tile.
 constexpr int kFRing = 2;
@@ -808,7 +809,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             __syncwarp();
             if (lane == 0) mbar_arrive(ds_ready);
             if (threadIdx.x == 64) TT_STAMPF(6);
-            // ---- P(c+1): runs while the tensor core forms dK(c), dV(c), dQ(c)
+            // ---- P(c+1): runs while the tensor core forms dK(c), dQ(c) (dV(c) is through: S(c+1) followed it into T1)
             if (c + 1 < n_chunks && !p_pass(c + 1)) goto done;
             if (threadIdx.x == 64) TT_STAMPF(7);
             // ---- dQ(c) out of T2 and into the global accumulator

@@ -13,7 +13,7 @@
 // per clock) and the special-function unit (16 exponentials per clock) each need 2048 clocks, so what counts is the
 // chain S -> softmax -> P V -> next S of a tile: the other tile covers only as much of it as it is itself busy.  Hence S is
 // read from tensor memory once, whole; the new maximum is found while the first exponentials run; and P V starts
-// when half of P is there.  24 heads x 32656 tokens: 11.1 -> 9.6 ms, 3 heads x 119056: 20.9 -> 17.9.
+// when half of P is there.  24 heads x 32656 tokens: 11.1 -> 9.3 - 9.6 ms, 3 heads x 119056: 20.9 -> 17.4 - 17.9.
 // The running row maximum is only raised when it grows by more than 2^8 ("lazy rescale"), so O is
 // corrected in tensor memory on rare iterations only.
 //

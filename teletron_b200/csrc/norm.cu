@@ -23,7 +23,7 @@ constexpr int kMaxCols = 8192;
 // XN (drop-in fused_adaln): the normalised row is stored as well, from the registers that hold it anyway; no mean.  Bound by
 // HBM: at 32656 x 3072 it takes 95 us (600 MB, 6.3 TB/s).  Forming x_norm from x, mean and rstd with separate elementwise
 // passes took another 0.8 ms, and scaling the backward's result by rstd in two more passes as much again; the pair with
-// the RMSNorm pair went from 2122 to 417 us there, and from 143 to 46 us at 256 rows.
+// the RMSNorm pair went from 2122 to 417 - 424 us there, and from 143 to 46 us at 256 rows.
 template <int VPL, bool GATE, bool XN = false>
 __global__ void __launch_bounds__(256, (VPL <= 12 ? 3 : 1)) ln_mod_fwd_kernel(
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ branch,

@@ -115,7 +115,8 @@ __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.w
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // Epilogue store of one warp's 32 rows x 64 columns of bf16 through a 4 KB box in shared memory (1024-byte aligned, 128-byte
-// rows, 16-byte pieces XOR-swizzled by row as SWIZZLE_128B expects; lane = row).  `o(g, f)` yields columns [8 g, 8 g + 8).
+// rows, 16-byte pieces XOR-swizzled by row as SWIZZLE_128B expects; lane = row).  `o(g)` yields 16-byte piece g of the
+// lane's row: columns [8 g, 8 g + 8) of bf16, [4 g, 4 g + 4) of a 32 x 32 box of fp32.
 template <typename F>
 __device__ __forceinline__ void store_box_32x64(uint32_t box, const CUtensorMap* tmap, int col, int row, int lane, F&& o) {
     // the caller alternates between two boxes: the group before last, which used this one, has been read

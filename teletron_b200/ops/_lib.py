@@ -54,8 +54,8 @@ def _load() -> Optional[ctypes.CDLL]:
         return None
     lib.tt_last_cuda_error.restype = ctypes.c_char_p
     # The GEMM entry points are called hundreds of times a step: with declared argument types they take plain integers, which
-    # spares a ctypes object per argument (the wrappers of the other calls are accepted as well).  The text MLP and a 512 x 512
-    # image's sampling step, which wait for the host, took 2 - 4 % longer without.
+    # spares a ctypes object per argument (the wrappers of the other calls are accepted as well).  With this and leaner checks in
+    # front a call takes the host 12.2 us instead of 14.1; no whole case gets faster by more than its runs differ.
     vp, ci, cl = ctypes.c_void_p, ctypes.c_int, ctypes.c_long
     for name in ("tt_gemm_bf16", "tt_gemm2_bf16"):
         getattr(lib, name).argtypes = [vp] * 5 + [ci] * 3 + [cl] * 3 + [ci] * 3 + [vp] * 2

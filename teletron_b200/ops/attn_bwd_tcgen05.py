@@ -3,7 +3,7 @@
 Two variants:
 
 * ``fused`` (default): one key-stationary kernel computes the scores once and forms dK, dV and this key tile's dQ
-  contribution (five products per tile pair); dQ is accumulated in an fp32 scratch with vector reductions, then scaled
+  contribution (five products per tile pair); dQ is accumulated in an fp32 scratch with bulk reductions, then scaled
   and rounded to bf16.  The order of those additions is not fixed, so dQ is reproducible to fp32 rounding only.
 * ``split`` (``TELETRON_B200_ATTN_BWD_FUSED=0``, or :func:`set_fused`): two deterministic, atomics-free kernels
   (key-stationary for dK / dV, query-stationary for dQ; seven products per tile pair).
