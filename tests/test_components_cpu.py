@@ -488,6 +488,9 @@ def test_single_attention_returns_video_and_text_apart():
     from teletron_b200.models.hunyuanvideo.blocks import SingleAttention
     g = torch.Generator().manual_seed(2)
     sa = SingleAttention(64, 2, 32, 1, 1e-6)
+    with torch.no_grad():
+        for p in sa.parameters():           # the layers leave their weights to the model's initialisation
+            p.copy_(torch.randn(p.shape, generator=g) * 0.2)
     h = torch.randn(2, 11, 64, generator=g)
     res = sa(h, 4, None, None, None, 3)
     assert isinstance(res, tuple) and [tuple(t.shape) for t in res] == [(2, 7, 64), (2, 4, 64)]
