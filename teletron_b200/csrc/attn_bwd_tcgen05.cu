@@ -65,6 +65,7 @@ struct BwdParams {
     int* status;
     const __nv_bfloat16* q_raw;     // q [BH, S, 128] and dout [B, S, H * 128] as plain pointers: the variant that keeps the
     const __nv_bfloat16* do_raw;    // stationary operands in tensor memory loads them with ordinary loads
+    const float* stats;             // one-pass variant: [B*H, chunks, 2, 128]: -lse * log2(e), then -delta; -inf and 0 for queries at and beyond S
     float* dq_acc;                  // one-pass variant: fp32 [B*H, s_pad, 128] accumulator for dQ (zeroed by the launcher)
     int s_pad;                      // rows per head in dq_acc: S rounded up to a multiple of 128
 #ifdef TT_ATTN_STAMPS
@@ -480,6 +481,7 @@ done:
 //   tensor core:  dK(c) dQ(c) ..... | ............... | dP(c+1) dV(c+1) S(c+2) .. | dK(c+1) dQ(c+1) ...
 //   softmax:      P(c+1) .......... | readout dQ(c) . | (dP(c+1)) dS(c+1) ....... | P(c+2) ...
 //
+// Used where CTA pairs (attn_bwd_pair_tcgen05.cu) are not faster: short heads, odd tiles, waves that a pair would start.
 // What bounds it is a chain through T2 and the dS tile: dS -> dK, dQ -> read-out -> the staged half leaves the dS tile ->
 // next dS (~4500 clocks a chunk; shared memory moves 480 KB a chunk, 3750 clocks at 128 bytes each, the tensor core needs
 // 2560).  So everything else is kept off it: dV takes P from T1, where it waits for nothing but the exponentials; dP(c+1) is
@@ -597,17 +599,15 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 const uint32_t wpar = ((uint32_t)(c / kFRing) & 1u) ^ 1u;
                 if (!mbar_wait(b1_empty(s), wpar, &abort_flag)) goto done;
                 TT_STAMPF(15);
-                // the rows of the statistics are `pitch` (a multiple of 64) long: the last chunk may have half of them
-                const uint32_t stat_bytes = 4u * (uint32_t)min(BC, p.pitch - chunk_of(c) * BC);
-                const long stat_at = (long)bh * p.pitch + chunk_of(c) * BC;
-                mbar_arrive_expect_tx(b1_full(s), kTile + stat_bytes);
-                bulk_load_1d(sStat + s * kFStatBytes, p.lse + stat_at, stat_bytes, b1_full(s));
+                const float* stats = p.stats + ((long)bh * p.s_pad + chunk_of(c) * BC) * 2;
+                mbar_arrive_expect_tx(b1_full(s), kTile + BC * 4);
+                bulk_load_1d(sStat + s * kFStatBytes, stats, BC * 4, b1_full(s));
 #pragma unroll
                 for (int h = 0; h < 2; ++h) tma_load_3d(sRing1 + s * kTile + h * kSlab, &tmQ, b1_full(s), h * 64, chunk_of(c) * BC, bh);
                 if (!mbar_wait(b2_empty(s), wpar, &abort_flag)) goto done;
                 TT_STAMPF(14);
-                mbar_arrive_expect_tx(b2_full(s), kTile + stat_bytes);
-                bulk_load_1d(sStat + s * kFStatBytes + BC * 4, p.delta + stat_at, stat_bytes, b2_full(s));
+                mbar_arrive_expect_tx(b2_full(s), kTile + BC * 4);
+                bulk_load_1d(sStat + s * kFStatBytes + BC * 4, stats + BC, BC * 4, b2_full(s));
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
                     tma_load_4d(sRing2 + s * kTile + h * kSlab, &tmDO, b2_full(s), h * 64, head, chunk_of(c) * BC, b);
@@ -736,12 +736,12 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         // this warp's 4 KB of the dQ staging: groups 0, 1 in the dS tile, groups 2, 3 in the chunk's dO slot
         const uint32_t stage_off = ((uint32_t)(quad * 2 + (part & 1)) << 12) + (uint32_t)lane * 128u;
 
-        // statistics of columns [8 i', 8 i' + 4) ... of this thread's 32 columns of chunk c (columns beyond the padded row: `pad`)
-        auto stat4 = [&](int c, int which, int i, float pad) {
+        // statistics of this thread's 32 columns of chunk c, four at a time
+        auto stat4 = [&](int c, int which, int i) {
             float4 v;
             const uint32_t a = sStat + (uint32_t)(c % kFRing) * kFStatBytes + (uint32_t)(which * BC + part * kCols + i * 4) * 4u;
             asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-            return chunk_of(c) * BC + part * kCols < p.pitch ? v : make_float4(pad, pad, pad, pad);
+            return v;
         };
         auto p_pass = [&](int c) -> bool {
             if (!mbar_wait(b1_full(c % kFRing), (uint32_t)(c / kFRing) & 1u, &abort_flag)) return false;      // lse(c)
@@ -753,8 +753,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-                if ((i & 1) == 0) lv = stat4(c, 0, i >> 1, INFINITY);
-                const float2 nl2 = __fmul2_rn((i & 1) ? make_float2(lv.z, lv.w) : make_float2(lv.x, lv.y), make_float2(-kLog2e, -kLog2e));
+                if ((i & 1) == 0) lv = stat4(c, 0, i >> 1);
+                const float2 nl2 = (i & 1) ? make_float2(lv.z, lv.w) : make_float2(lv.x, lv.y);
                 const float2 x = __ffma2_rn(make_float2(__uint_as_float(a[2 * i]), __uint_as_float(a[2 * i + 1])),
                                             make_float2(c_log2, c_log2), nl2);
                 const __nv_bfloat162 pb = __floats2bfloat162_rn(exp2f(x.x), exp2f(x.y));
@@ -784,10 +784,10 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    if ((i & 1) == 0) dv = stat4(c, 1, i >> 1, 0.f);
+                    if ((i & 1) == 0) dv = stat4(c, 1, i >> 1);
                     const float2 d2 = (i & 1) ? make_float2(dv.z, dv.w) : make_float2(dv.x, dv.y);
                     const float2 pr = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[i]));
-                    const float2 dp = __ffma2_rn(d2, make_float2(-1.f, -1.f), make_float2(__uint_as_float(g[2 * i]), __uint_as_float(g[2 * i + 1])));
+                    const float2 dp = __fadd2_rn(d2, make_float2(__uint_as_float(g[2 * i]), __uint_as_float(g[2 * i + 1])));
                     const float2 ds = __fmul2_rn(pr, dp);
                     const __nv_bfloat162 db = __floats2bfloat162_rn(ds.x, ds.y);
                     dk[i] = *reinterpret_cast<const uint32_t*>(&db);
@@ -873,6 +873,40 @@ done:
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
+    }
+}
+
+// stats and a cleared accumulator: delta[bh, s] = sum_d dO[b, s, h, d] * O[b, s, h, d], one warp per (token, head) and 512 bytes of dq_acc
+// (rows of a chunk are permuted in there, so the rows beyond S are cleared too).  One pass instead of four launches (two fills, the
+// row dots, a memset), and it saves the main kernel a product and a bounds check per score.
+__global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
+                                                            const float* __restrict__ lse, float* __restrict__ stats, float* __restrict__ dq_acc,
+                                                            int B, int S, int H, int pitch, int s_pad) {
+    const int lane = threadIdx.x & 31;
+    const long nwork = (long)B * s_pad * H;
+    for (long w = (long)blockIdx.x * 8 + (threadIdx.x >> 5); w < nwork; w += (long)gridDim.x * 8) {
+        const long tok = w / H;                     // heads fastest: dO and O are token-major
+        const int h = (int)(w - tok * H);
+        const long b = tok / s_pad;
+        const int s = (int)(tok - b * s_pad);
+        const long bh = b * H + h;
+        float v = 0.f;
+        if (s < S) {
+            const long at = ((b * S + s) * H + h) * D + lane * 4;
+            const uint2 a = *reinterpret_cast<const uint2*>(dout + at);
+            const uint2 o = *reinterpret_cast<const uint2*>(out + at);
+            const float2 a0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a.x));
+            const float2 a1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a.y));
+            const float2 o0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o.x));
+            const float2 o1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o.y));
+            v = tt::warp_sum(a0.x * o0.x + a0.y * o0.y + a1.x * o1.x + a1.y * o1.y);
+        }
+        *reinterpret_cast<float4*>(dq_acc + (bh * s_pad + s) * D + lane * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (lane == 0) {
+            float* st = stats + (bh * s_pad + (s & ~(BC - 1))) * 2 + (s & (BC - 1));
+            st[0] = s < S ? -kLog2e * lse[bh * pitch + s] : -INFINITY;
+            st[BC] = -v;
+        }
     }
 }
 
@@ -975,20 +1009,42 @@ extern "C" int tt_attn_bwd(const void* q, const void* k, const void* v, const vo
     return TT_OK;
 }
 
-// One-pass backward: delta preprocess, the fused key-stationary kernel (dK, dV written, dQ accumulated in fp32 into
-// `dq_acc`), then the scale-and-round pass into `dq`.  dq_acc: fp32 scratch of B * H * s_pad * 128 elements with
-// s_pad = S rounded up to a multiple of 128; it is zeroed here.
+// Microseconds per CTA and 128-query chunk, and per CTA besides (its first loads, tensor memory, the epilogue): 768 heads of 4 and 10 key
+// tiles took 558 and 2299 us on single CTAs, 532 and 2035 on pairs.  Over 24 .. 768 heads of 1 .. 21 tiles the kernel with the cheaper waves is
+// the faster one or within 4 % of it, but for 12 tiles, where pairs lose up to 5 %; an odd tile leaves half a pair idle (3 tiles: 364 against
+// 446 us), and a pair that starts a new wave costs it (48 heads of 9 tiles: 123 against 141).  Long heads: 32.7 and 28.4 ms at 24 x 32656 tokens.
+static bool pairs_are_faster(uint64_t heads, int tiles, int sms) {
+    const uint64_t single = (heads * tiles + sms - 1) / sms, pairs = (heads * ((tiles + 1) / 2) + sms / 2 - 1) / (sms / 2);
+    return (double)pairs * (2.25 * tiles + 15.1) <= (double)single * (2.9 * tiles + 13.7);
+}
+
+// attn_bwd_pair_tcgen05.cu
+int tt_attn_bwd_pair(const void* q, const void* k, const void* v, const void* dout, const float* stats, float* dq_acc, void* dq, void* dk,
+                     void* dv, int B, int H, int S, int kv_len, int mask_lo, int mask_hi, float scale, int* status, cudaStream_t st);
+
+// One-pass backward: row dots and statistics, the kernel that forms dK, dV and accumulates dQ in fp32 (on CTA pairs or single CTAs), then
+// the scale-and-round pass.  lse: [B*H, pitch]; workspace: B * H * roundup(S, 128) * 130 floats of any contents.
 extern "C" int tt_attn_bwd_fused(const void* q, const void* k, const void* v, const void* out, const void* dout,
-                                 const float* lse, float* delta, float* dq_acc, void* dq, void* dk, void* dv, int B, int H,
+                                 const float* lse, float* workspace, size_t workspace_floats, void* dq, void* dk, void* dv, int B, int H,
                                  int S, int kv_len, int mask_lo, int mask_hi, int pitch, float scale, int* status,
                                  void* stream) {
-    if (B <= 0 || H <= 0 || S <= 0 || kv_len <= 0 || kv_len > S || status == nullptr || delta == nullptr || dq_acc == nullptr)
-        return TT_ERR_ARG;
+    if (B <= 0 || H <= 0 || S <= 0 || kv_len <= 0 || kv_len > S || status == nullptr || workspace == nullptr) return TT_ERR_ARG;
     if (mask_lo < mask_hi && (mask_lo < 0 || (mask_lo == 0 && mask_hi >= kv_len))) return TT_ERR_ARG;
-    if (pitch < S || (pitch & 63) || ((uintptr_t)lse & 15) || ((uintptr_t)delta & 15) || ((uintptr_t)dq_acc & 15)) return TT_ERR_ARG;
+    for (const void* x : {q, k, v, out, dout, (const void*)workspace, (const void*)dq, (const void*)dk, (const void*)dv})
+        if ((uintptr_t)x & 15) return TT_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     const uint64_t BH = (uint64_t)B * H;
     const int s_pad = (S + BC - 1) / BC * BC;
+    if (pitch < S || workspace_floats < BH * (uint64_t)s_pad * (D + 2)) return TT_ERR_ARG;
+    float* dq_acc = workspace;
+    float* stats = workspace + BH * (uint64_t)s_pad * D;
+    const long nwork = (long)BH * s_pad, want = (nwork + 7) / 8;
+    // launched before the tensor maps are encoded: it also makes the device's context current in a thread that has not used it yet
+    attn_bwd_prep_kernel<<<(int)(want < 148L * 16 ? want : 148L * 16), 256, 0, st>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, lse, stats,
+                                                                                    dq_acc, B, S, H, pitch, s_pad);
+    TT_CHECK_LAUNCH();
+    if (pairs_are_faster(BH, s_pad / BC, tt_device().sms))
+        return tt_attn_bwd_pair(q, k, v, dout, stats, dq_acc, dq, dk, dv, B, H, S, kv_len, mask_lo, mask_hi, scale, status, st);
     CUtensorMap tq_s, tk_s, tv_s, tdo_s;
     int rc;
     if ((rc = tt_make_tmap_3d(&tq_s, q, BH, (uint64_t)S, D, D, (uint64_t)S * D, BS, 64)) != TT_OK) return rc;
@@ -996,23 +1052,16 @@ extern "C" int tt_attn_bwd_fused(const void* q, const void* k, const void* v, co
     if ((rc = tt_make_tmap_3d(&tv_s, v, BH, (uint64_t)S, D, D, (uint64_t)S * D, BS, 64)) != TT_OK) return rc;
     if ((rc = tt_make_tmap_bshd(&tdo_s, dout, (uint64_t)B, (uint64_t)S, (uint64_t)H, BS)) != TT_OK) return rc;
     static bool configured_dev[64] = {false};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    const int dev = tt_device().dev;
     if (!configured_dev[dev]) {
         cudaError_t e = cudaFuncSetAttribute(attn_bwd_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmemBytes);
         if (e != cudaSuccess) return tt_record_cuda(e);
         configured_dev[dev] = true;
     }
-    cudaError_t e = cudaMemsetAsync(dq_acc, 0, BH * (uint64_t)s_pad * D * sizeof(float), st);
-    if (e != cudaSuccess) return tt_record_cuda(e);
-    const long nwork = (long)B * S * H;
-    long want = (nwork + 7) / 8;
-    delta_kernel<<<(int)(want < 148L * 16 ? want : 148L * 16), 256, 0, st>>>((const __nv_bfloat16*)dout,
-                                                                            (const __nv_bfloat16*)out, delta, B, S, H, pitch);
-    TT_CHECK_LAUNCH();
     BwdParams p;
-    p.lse = lse;
-    p.delta = delta;
+    p.lse = nullptr;
+    p.delta = nullptr;
+    p.stats = stats;
     p.S = S;
     p.kv_len = kv_len;
     p.mask_lo = mask_lo;

@@ -46,7 +46,6 @@ constexpr int kThreads = 192;
 constexpr int kGroupM = 8;
 constexpr int kEpiBytes = 4 * 8192;                      // two 32 x 64 boxes per epilogue warp
 constexpr int kSmemBytes = kStages * kStageBytes + kEpiBytes + 1024 + 256;
-constexpr uint32_t kPeerMask = 0xFEFFFFFFu;             // clears the bit that tells the two CTAs of a pair apart
 
 struct Params2 {
     int M, N, K;
@@ -59,50 +58,6 @@ struct Params2 {
     int k1;                     // K columns >= k1 come from the second A tensor (a multiple of BK, or >= K: there is none)
     int part_rows;              // rows of one split's slice of the scratch buffer (M rounded up to whole 32-row boxes)
 };
-
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_alloc2(uint32_t smem_result, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_result), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish2() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// 2-D tiled load (no multicast) whose completion bytes go to the LEADER CTA's mbarrier
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t smem_dst, const CUtensorMap* tmap, uint32_t bar, int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
-            smem_dst),
-        "l"((uint64_t)tmap), "r"(bar & kPeerMask), "r"(c0), "r"(c1)
-        : "memory");
-}
-__device__ __forceinline__ void umma2_bf16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// arrives (once the MMAs issued so far have completed) on the barrier at this shared-memory offset in BOTH CTAs of the pair
-__device__ __forceinline__ void umma2_commit_both(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-                 "h"((uint16_t)3)
-                 : "memory");
-}
-// plain arrival on the leader CTA's copy of a barrier (from either CTA)
-__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar & kPeerMask) : "memory");
-}
 
 template <int EPI>
 __device__ __forceinline__ float epi2(float acc, float b, float u) {

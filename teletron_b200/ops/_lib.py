@@ -186,4 +186,5 @@ def call(fn_name: str, *args) -> None:
 
 c_long = ctypes.c_long
 c_int = ctypes.c_int
+c_size = ctypes.c_size_t
 c_float = ctypes.c_float

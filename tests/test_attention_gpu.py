@@ -176,3 +176,32 @@ def test_forward_running_maximum_with_masked_tiles(S, kv_len, mask, ramp):
     if mask:
         s[..., mask[0]:mask[1]] = float("-inf")
     torch.testing.assert_close(lse[..., :S].double(), s.logsumexp(-1), rtol=1e-4, atol=1e-3)
+
+
+@pytest.mark.parametrize("B,H,S,kv_len,mask", [
+    (1, 1, 257, 200, None), (1, 2, 384, None, None), (2, 3, 300, None, (20, 90)), (1, 1, 511, None, None), (1, 2, 513, 500, None),
+    (1, 3, 1237, 1201, (180, 256)), (1, 1, 2049, None, None),             # CTA pairs: odd tiles, ragged chunks, masks over a tile's edge
+    (1, 1, 129, None, None), (3, 50, 257, 250, (100, 130)), (40, 4, 33, None, None)])    # single CTAs: few tiles, waves of odd ones
+def test_one_pass_backward_against_64_bits(B, H, S, kv_len, mask):
+    """Both kernels of the one-pass backward at the edges of their tiles.  bf16 P and dS (2^-9 each) under fp32 sums leave about
+    3e-3; the two-kernel split differs from this by the order of sums only."""
+    from teletron_b200.ops import attn_bwd_tcgen05 as AB, attn_tcgen05 as A
+    from teletron_b200.ops.gemm_tcgen05 import check_status
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v = (torch.randn(B, H, S, 128, device="cuda", generator=g).bfloat16() for _ in range(3))
+    d = torch.randn(B, S, H * 128, device="cuda", generator=g).bfloat16()
+    out, lse, qc, kc, vc, sc, kv = A.forward(q, k, v, kv_len, None, mask)
+    got = AB.backward(d, qc, kc, vc, out, lse, sc, kv, mask_range=mask or (0, 0))
+    check_status()
+    qd, kd, vd = (t.double() for t in (q, k, v))
+    dd = d.double().view(B, S, H, 128).transpose(1, 2)
+    s = qd @ kd.transpose(-1, -2) * sc
+    dead = torch.zeros(S, dtype=torch.bool, device="cuda")
+    dead[kv:] = True
+    if mask:
+        dead[mask[0]:mask[1]] = True
+    p = s.masked_fill(dead, float("-inf")).softmax(-1)
+    ds = p * (dd @ vd.transpose(-1, -2) - (dd * (p @ vd)).sum(-1, keepdim=True)) * sc
+    for a, r in zip(got, (ds @ kd, ds.transpose(-1, -2) @ qd, p.transpose(-1, -2) @ dd)):
+        assert _rel(a, r) < 5e-3
+        assert torch.isfinite(a).all()
