@@ -22,7 +22,8 @@
 // single-stream block's [attention | MLP] never has to be concatenated.
 //
 // Layouts and epilogues are those of gemm_tcgen05.cu (nt / nn / tn; bias, GELU erf / tanh with pre-activation,
-// GELU backward).  In the reference these products are TransformerEngine -> cuBLASLt calls
+// GELU backward), and one more for weight gradients: epilogue 5 (tn) adds the bf16 tile to what C holds, in the TMA unit
+// (cp.reduce.async.bulk.tensor), so that a gradient buffer takes a product without a temporary and a pass that adds it.  In the reference these products are TransformerEngine -> cuBLASLt calls
 // (teletron/models/dit/dit_attention.py:65-104, dit_layerspec.py:266-298, 438-445).
 #include "common.cuh"
 #include "sm100.cuh"
@@ -61,7 +62,7 @@ struct Params2 {
 
 template <int EPI>
 __device__ __forceinline__ float epi2(float acc, float b, float u) {
-    if (EPI == 0) return acc + b;
+    if (EPI == 0 || EPI == 5) return acc + b;
     if (EPI == 1) return tt::gelu_erf(acc + b);
     if (EPI == 2) return tt::gelu_tanh(acc + b);
     if (EPI == 3) return acc * tt::gelu_erf_grad(u);
@@ -247,7 +248,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
 #pragma unroll
                     for (int j = 0; j < 8; ++j) bv[j] = uv[j] = 0.f;
                     if (EPI <= 2 && p.bias != nullptr && col + 8 <= p.N) tt::unpack8(tt::ld8(p.bias + col), bv);
-                    if (EPI >= 3 && row_ok && col + 8 <= p.N) tt::unpack8(tt::ld8(arow + col), uv);
+                    if ((EPI == 3 || EPI == 4) && row_ok && col + 8 <= p.N) tt::unpack8(tt::ld8(arow + col), uv);
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         o[j] = pre ? __uint_as_float(r[g * 8 + j]) + bv[j] : epi2<EPI>(__uint_as_float(r[g * 8 + j]), bv[j], uv[j]);
@@ -255,8 +256,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
                     return *reinterpret_cast<const uint4*>(&pk);
                 };
                 if (EPI == 1 || EPI == 2) store_box_32x64(box + 4096u * (nbox++ & 1u), &tmAux, col0, row0, lane, [&](int g) { return packed(g, true); });
-                store_box_32x64(box + 4096u * (nbox++ & 1u), &tmC, col0, row0, lane,
-                                [&](int g) { return packed(g, false); });
+                store_box_32x64<EPI == 5>(box + 4096u * (nbox++ & 1u), &tmC, col0, row0, lane,
+                                          [&](int g) { return packed(g, false); });
             }
             tc_fence_before();
             __syncwarp();
@@ -337,9 +338,11 @@ __global__ void __launch_bounds__(256) splitk_finish_kernel(const float* __restr
 // The product of every entry point.  a2 (or nullptr) supplies the K columns from k1 on; splits > 1 needs `scratch`.
 int run2(const void* a, const void* a2, int k1, long lda2, const void* b, void* c, const void* bias, void* aux, int M, int N, int K, long lda,
          long ldb, long ldc, int a_mn, int b_mn, int epi, int splits, float* scratch, int* status, void* stream) {
-    if (M <= 0 || N <= 0 || K <= 0 || (N & 7) || (K & 7) || (ldc & 7) || status == nullptr) return TT_ERR_ARG;
+    // with both operands K x MN (a_mn and b_mn) K is a row count, which need not be a multiple of 8: the rows beyond it load as zeros
+    if (M <= 0 || N <= 0 || K <= 0 || (N & 7) || ((K & 7) && !(a_mn && b_mn)) || (ldc & 7) || status == nullptr) return TT_ERR_ARG;
     if (a_mn && (M & 7)) return TT_ERR_ARG;
-    if (epi < 0 || epi > 4 || (epi != 0 && aux == nullptr)) return TT_ERR_ARG;
+    if (epi < 0 || epi > 5 || (epi >= 1 && epi <= 4 && aux == nullptr)) return TT_ERR_ARG;
+    if (epi == 5 && (!a_mn || !b_mn || bias != nullptr || splits != 1)) return TT_ERR_ARG;
     if (((uintptr_t)c & 15) || (bias && ((uintptr_t)bias & 15)) || (aux && ((uintptr_t)aux & 15))) return TT_ERR_ARG;
     if (a_mn && !b_mn) return TT_ERR_ARG;
     if (a2 != nullptr && (a_mn || k1 <= 0 || k1 >= K || (k1 % BK))) return TT_ERR_ARG;
@@ -386,6 +389,7 @@ int run2(const void* a, const void* a2, int k1, long lda2, const void* b, void* 
             if (epi == 4) GO(false, true, 4);
         } else if (amn && bmn) {
             if (epi == 0) GO(true, true, 0);
+            if (epi == 5) GO(true, true, 5);
         }
 #undef GO
         return TT_ERR_ARG;

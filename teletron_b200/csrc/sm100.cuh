@@ -108,6 +108,12 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tmap, uint32_t s
                  "r"(c0), "r"(c1)
                  : "memory");
 }
+// the same, added to what is there (one rounding to the tensor's type per element)
+__device__ __forceinline__ void tma_add_2d(const CUtensorMap* tmap, uint32_t smem_src, int c0, int c1) {
+    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"((uint64_t)tmap), "r"(smem_src),
+                 "r"(c0), "r"(c1)
+                 : "memory");
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // at most N of this thread's bulk groups have not been read out of shared memory yet
 template <int N>
@@ -117,7 +123,7 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 // Epilogue store of one warp's 32 rows x 64 columns of bf16 through a 4 KB box in shared memory (1024-byte aligned, 128-byte
 // rows, 16-byte pieces XOR-swizzled by row as SWIZZLE_128B expects; lane = row).  `o(g)` yields 16-byte piece g of the
 // lane's row: columns [8 g, 8 g + 8) of bf16, [4 g, 4 g + 4) of a 32 x 32 box of fp32.
-template <typename F>
+template <bool ADD = false, typename F>
 __device__ __forceinline__ void store_box_32x64(uint32_t box, const CUtensorMap* tmap, int col, int row, int lane, F&& o) {
     // the caller alternates between two boxes: the group before last, which used this one, has been read
     if (lane == 0) bulk_wait_read<1>();
@@ -132,7 +138,8 @@ __device__ __forceinline__ void store_box_32x64(uint32_t box, const CUtensorMap*
     fence_proxy_async();
     __syncwarp();
     if (lane == 0) {
-        tma_store_2d(tmap, box, col, row);
+        if (ADD) tma_add_2d(tmap, box, col, row);
+        else tma_store_2d(tmap, box, col, row);
         bulk_commit();
     }
 }

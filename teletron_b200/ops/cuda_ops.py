@@ -214,6 +214,38 @@ def _transformed(t: torch.Tensor) -> bool:
     return (torch.is_grad_enabled() and t.requires_grad) or forward_ad._current_level >= 0 or not torch._C._has_storage(t)
 
 
+def _flat_grad(ctx, weight: torch.Tensor, du: torch.Tensor) -> Optional[torch.Tensor]:
+    """The gradient buffer that autograd is about to add ``weight``'s gradient to, if the product may do that itself: the parameter lives
+    in a flat buffer (:class:`teletron_b200.parallel.grad_buffer.ParamAndGradBuffer`), its accumulation node is part of this backward
+    pass (``torch.autograd.grad`` collects the gradient instead), and nobody looks at the gradient on its way there: no hooks, no
+    ``create_graph``, no batched or forward-mode gradients, and the default stream, on which accumulation nodes run too."""
+    if _transformed(du) or torch.is_grad_enabled() or _lib.raw_stream() != 0:
+        return None
+    for fn, _ in ctx.next_functions:
+        param = getattr(fn, "variable", None)
+        if param is None or not getattr(param, "flat_grad", False) or param.data_ptr() != weight.data_ptr() or param.shape != weight.shape:
+            continue
+        g = param.grad
+        if g is None or g.dtype != BF16 or g.shape != param.shape or not g.is_contiguous() or g.requires_grad or g.device != du.device:
+            return None
+        if param._backward_hooks or param._post_accumulate_grad_hooks:
+            return None
+        try:
+            return g if torch._C._will_engine_execute_node(fn) else None
+        except RuntimeError:        # a leaf that torch.autograd.grad collects
+            return None
+    return None
+
+
+def _weight_grad(ctx, weight: torch.Tensor, du: torch.Tensor, x: torch.Tensor) -> Optional[torch.Tensor]:
+    """``du^T x``, or None once it has been added to the parameter's gradient buffer.  The addition in the product's epilogue moves
+    4 bytes per weight where a temporary and a separate addition move 10."""
+    buf = _flat_grad(ctx, weight, du)
+    if buf is not None and gemm.gemm_tn_add(du, x, buf):
+        return None
+    return _gemm_tn(du, x)
+
+
 def _bias_grad(du: torch.Tensor) -> torch.Tensor:
     """Column sums of ``du [rows, cols]`` in fp32, rounded once."""
     rows, cols = du.shape
@@ -274,7 +306,7 @@ class _Linear(torch.autograd.Function):
             else:
                 call("tt_gelu_bwd", ptr(dyc), ptr(u), ptr(du), c_long(u.numel()), c_int(_GELU_KIND[ctx.activation]), stream())
         dx = _gemm_nn(du, weight) if ctx.needs_input_grad[0] else None
-        dw = _gemm_tn(du, x2) if ctx.needs_input_grad[1] else None
+        dw = _weight_grad(ctx, weight, du, x2) if ctx.needs_input_grad[1] else None
         if db is None and ctx.has_bias and ctx.needs_input_grad[2]:
             db = _bias_grad(du)
         if dx is not None:
@@ -315,9 +347,13 @@ class _LinearMerged(torch.autograd.Function):
         d2 = _gemm_nn(du, weight[:, k1:]).view(*ctx.lead, a2.shape[1]) if ctx.needs_input_grad[1] else None
         dw = None
         if ctx.needs_input_grad[2]:
-            dw = torch.empty_like(weight)
-            gemm.gemm_tn_into(du, a1, dw[:, :k1])
-            gemm.gemm_tn_into(du, a2, dw[:, k1:])
+            buf = _flat_grad(ctx, weight, du)
+            if buf is not None and gemm_tcgen05.add_supported(du, a2, buf[:, k1:]) and gemm.gemm_tn_add(du, a1, buf[:, :k1]):
+                gemm.gemm_tn_add(du, a2, buf[:, k1:])
+            else:
+                dw = torch.empty_like(weight)
+                gemm.gemm_tn_into(du, a1, dw[:, :k1])
+                gemm.gemm_tn_into(du, a2, dw[:, k1:])
         db = _bias_grad(du) if (ctx.has_bias and ctx.needs_input_grad[3]) else None
         return d1, d2, dw, db
 
@@ -391,7 +427,7 @@ class _QKVProjection(torch.autograd.Function):
                  ptr(cosf if rl else None), ptr(sinf if rl else None), ptr(dqkv), ptr(partials), ptr(dqw), ptr(dkw),
                  c_long(rows), c_int(heads), c_long(rows // B), c_long(S), c_long(off), c_long(rl), c_float(eps), stream())
             dx = _gemm_nn(dqkv, ws).view(B, -1, K)
-            dw = _gemm_tn(dqkv, xs2)
+            dw = _weight_grad(ctx, ws, dqkv, xs2)
             db = _bias_grad(dqkv) if hb else None
             outs.append((dx, dw, db, dqw, dkw))
         (dx1, dw1, db1, dqw1, dkw1), (dx2, dw2, db2, dqw2, dkw2) = outs

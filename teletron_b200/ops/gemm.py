@@ -75,6 +75,15 @@ def gemm_tn(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     return torch.matmul(a.t(), b)
 
 
+def gemm_tn_add(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> bool:
+    """``out += a.T @ b`` without a temporary, where the kernel takes it (False: nothing was done)."""
+    if _BACKEND == "cublas" or not gemm_tcgen05.add_supported(a, b, out):
+        return False
+    COUNTERS["tcgen05"] += 1
+    gemm_tcgen05.gemm_add(a, b, out)
+    return True
+
+
 def gemm_tn_into(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """``out[:] = a.T @ b`` where ``out`` may be a column slice of a larger row-major matrix."""
     if _BACKEND != "cublas":

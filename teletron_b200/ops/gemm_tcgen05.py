@@ -144,6 +144,25 @@ def gemm(a: torch.Tensor, b: torch.Tensor, layout: str, bias: Optional[torch.Ten
     return (c, aux) if epi in (1, 2) else c
 
 
+def add_supported(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> bool:
+    """``out += a.T @ b`` in the product's epilogue: any row count, and no split over K (a split product has a pass of its own that
+    could add, but a gradient with so few tiles is small)."""
+    if not (PAIR_KERNEL and _lib.available() and a.is_cuda and a.dtype == BF16 and b.dtype == BF16 and out.dtype == BF16 and _rowmajor(a)
+            and _rowmajor(b) and _rowmajor(out)):
+        return False
+    (K, M), (K2, N) = a.shape, b.shape
+    return (K == K2 >= 1 and tuple(out.shape) == (M, N) and M % 8 == 0 and N % 8 == 0 and min(M, N) >= 8
+            and (use_pair_kernel(M, N) or _plan(M, N, K)[1] == 1))
+
+
+def gemm_add(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> None:
+    """``out += a.T @ b``: the product is rounded to bf16, then added with one more rounding, as a separate addition would."""
+    (K, M), N = a.shape, b.shape[1]
+    COUNTERS["pair"] += 1
+    call("tt_gemm2_bf16", a.data_ptr(), b.data_ptr(), out.data_ptr(), None, None, M, N, K, a.stride(0), b.stride(0), out.stride(0), 1, 1, 5,
+         status_tensor(a.device).data_ptr(), _lib.raw_stream())
+
+
 def two_supported(a: torch.Tensor, a2: torch.Tensor, b: torch.Tensor) -> bool:
     """``[a | a2] @ b.T`` without the concatenation: the seam has to lie between two 64-wide k-blocks."""
     return (PAIR_KERNEL and a2.dtype == BF16 and a2.is_cuda and _rowmajor(a2) and a.dim() == 2 and a.shape[0] == a2.shape[0]

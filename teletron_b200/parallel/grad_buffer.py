@@ -106,6 +106,7 @@ class ParamAndGradBuffer:
             view.copy_(p.data)
             p.data = view
             p.grad = self.grad_data[s:e].view(p.shape)
+            p.flat_grad = True              # weight-gradient products may add to p.grad themselves (ops/cuda_ops.py)
         self.params = [p for _, p in ordered]
         # buckets in reverse buffer order approximate backward order; each bucket is a multiple of
         # shard_count * 8 elements so reduce-scatter shards stay aligned

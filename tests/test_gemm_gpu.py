@@ -273,3 +273,77 @@ def test_small_products_as_planned(M, N, K, kind):
     for r0 in range(0, M, 32):
         assert _rel(c[r0:r0 + 32], ref[r0:r0 + 32]) < 3e-3 and _rel(c2[r0:r0 + 32], ref[r0:r0 + 32]) < 3e-3
     G.check_status()
+
+
+@pytest.mark.parametrize("K,M,N", [(1, 512, 3072), (7, 264, 520), (64, 256, 256), (250, 3072, 1024), (1000, 8, 4096), (333, 4096, 2056)])
+def test_weight_gradient_added_in_the_epilogue(K, M, N):
+    """``out += a.T @ b`` rounds the product to bf16 and adds with one more rounding: the bits of a separate addition up to the order of
+    the product's fp32 sums (a tie of one bf16 step in places).  Any row count; columns beside the window stay as they are."""
+    from teletron_b200.ops import gemm
+    from teletron_b200.ops.gemm_tcgen05 import add_supported, check_status
+    g = torch.Generator(device="cuda").manual_seed(K)
+    a, b = (torch.randn(K, n, device="cuda", generator=g).bfloat16() for n in (M, N))
+    whole = torch.randn(M, N + 64, device="cuda", generator=g).bfloat16()
+    before, out = whole.clone(), whole[:, 8:8 + N]
+    assert add_supported(a, b, out) and gemm.gemm_tn_add(a, b, out)
+    check_status()
+    ref = before[:, 8:8 + N].double() + (a.double().t() @ b.double()).bfloat16().double()
+    assert (out.double() - ref).abs().max() <= 2 ** -7 * ref.abs().max()
+    assert (out.double() - ref).norm() < 4e-3 * ref.norm()          # 2^-9 per rounding
+    assert torch.equal(whole[:, :8], before[:, :8]) and torch.equal(whole[:, 8 + N:], before[:, 8 + N:])
+
+
+def test_flat_gradient_buffers_receive_products_only_where_autograd_accumulates():
+    """Parameters in a flat buffer: ``backward`` adds each weight gradient exactly once per pass, with the bits of the separate addition;
+    ``autograd.grad``, hooks, ``create_graph`` and a side stream see gradients as before."""
+    from teletron_b200 import ops
+    from teletron_b200.ops.gemm_tcgen05 import COUNTERS
+    from teletron_b200.parallel.grad_buffer import DistributedDataParallel
+
+    class Net(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            g = torch.Generator(device="cuda").manual_seed(3)
+            mk = lambda *s: torch.nn.Parameter((torch.randn(*s, device="cuda", generator=g) * 0.05).bfloat16())  # noqa: E731
+            self.w1, self.b1, self.w2, self.w3 = mk(1024, 256), mk(1024), mk(256, 1024), mk(256, 512)
+
+        def forward(self, x):
+            h = ops.linear(ops.linear(x, self.w1, self.b1, "gelu"), self.w2)
+            return ops.linear_merged(h, x, self.w3)
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(1, 37, 256, device="cuda", generator=g).bfloat16()
+    dy = torch.randn(1, 37, 256, device="cuda", generator=g).bfloat16()
+    plain, net = Net(), Net()
+    ddp = DistributedDataParallel(net, None)
+    names = ("w1", "b1", "w2", "w3")
+    for _ in range(2):                                       # two micro-batches
+        plain(x).backward(dy)
+        n0 = COUNTERS["pair"]
+        ddp(x).backward(dy)
+    assert COUNTERS["pair"] > n0
+    for n in names:
+        torch.testing.assert_close(getattr(net, n).grad, getattr(plain, n).grad, rtol=1.6e-2, atol=1e-2)
+    kept = {n: getattr(net, n).grad.clone() for n in names}
+    got = torch.autograd.grad(net(x), [net.w1, net.w2, net.w3], dy)
+    want = torch.autograd.grad(plain(x), [plain.w1, plain.w2, plain.w3], dy)
+    for a, b in zip(got, want):
+        torch.testing.assert_close(a, b, rtol=1.6e-2, atol=1e-2)
+    assert all(torch.equal(getattr(net, n).grad, kept[n]) for n in names)          # collected, not accumulated
+    seen = []
+    h1 = net.w1.register_hook(lambda t: seen.append("w1"))
+    h2 = net.w2.register_post_accumulate_grad_hook(lambda p: seen.append("w2"))
+    net(x).backward(dy)
+    assert sorted(seen) == ["w1", "w2"]
+    h1.remove()
+    h2.remove()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        net(x).backward(dy)
+    torch.cuda.current_stream().wait_stream(side)
+    net(x).backward(dy, inputs=[net.b1])                    # nothing for the weights
+    for _ in range(2):
+        plain(x).backward(dy)
+    for n in ("w1", "w2", "w3"):
+        torch.testing.assert_close(getattr(net, n).grad, getattr(plain, n).grad, rtol=1.6e-2, atol=2e-2)
