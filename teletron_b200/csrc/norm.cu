@@ -270,10 +270,288 @@ __global__ void __launch_bounds__(MAXT, 1) ln_mod_bwd_kernel(
 // filled by one producer warp with untiled bulk copies (cp.async.bulk, completion on an mbarrier).  What is in flight
 // is then set by the ring (up to ~190 KB per SM) instead of by the registers a thread can spare for pending loads, which
 // kept the register version at a third of the copy bandwidth.  Consumer thread t owns columns [8t, 8t + 8) as before;
-// branch / upstream-gradient rows are fetched with ordinary loads issued before the block reduction.
+// branch / upstream-gradient rows are fetched with ordinary loads issued ahead of the arithmetic before them.
+//
+// The twelve consumer warps of a 3072-column row are too few to hide a block reduction and the chains of a row (without its
+// stores this kernel is no faster, without the first pass's arithmetic it is by a fifth).  So a batch's sums are handed over through
+// one of four buffers (an mbarrier each) and the first pass of the next batch runs before they are waited for; statistics are
+// loaded a batch ahead; the rows of a whole batch are one block of code, so that their chains overlap; the arithmetic is packed
+// (fp32x2).  Wider rows (two or three stages, fewer registers a thread) take the passes one after the other.  32656 x 3072: plain
+// 168 -> 132 us, gated 342 -> 256, from normalised rows (fused_adaln) 138 -> 117 (600 MB, 5.1 TB/s); 16000 x 6144: 190 -> 164, 423 -> 346, 171 -> 142.
 // ---------------------------------------------------------------------------------------------
 __device__ int g_norm_status = 0;       // TT_ERR_TIMEOUT when a bounded wait of the ring ran out (read by tt_norm_status)
 
+constexpr int kRedBufs = 4;             // a warp writes the sums of batch i + 4 once every warp has read those of batch i
+
+template <bool GATE, int MAXT, bool XHAT = false>
+__global__ void __launch_bounds__(MAXT + 32) ln_mod_bwd_ring_kernel(
+    const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ dres_in,
+    const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ branch,
+    const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ scale,
+    const float* __restrict__ mean, const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx,
+    __nv_bfloat16* __restrict__ dbranch, float* __restrict__ partials, int cols, long rows_per_batch, int stages) {
+    constexpr bool AHEAD = MAXT <= 384;     // four stages or more, and registers for a second batch's statistics
+    extern __shared__ uint8_t ring_raw[];
+    __shared__ float red[kRedBufs * 8 * 32];
+    __shared__ __align__(8) uint64_t red_bars[kRedBufs];
+    __shared__ volatile int abort_flag;
+    using namespace sm100;
+    const uint32_t base = (smem_u32(ring_raw) + 127u) & ~127u;
+    const uint32_t row_bytes = (uint32_t)cols * 2u;
+    const uint32_t stage_bytes = 2u * kRowBatch * row_bytes;              // dy rows then x rows
+    const uint32_t bars = base + (uint32_t)stages * stage_bytes;
+    auto full_bar = [&](int s) { return bars + 8u * s; };
+    auto empty_bar = [&](int s) { return bars + 8u * (stages + s); };
+    auto red_bar = [&](int i) { return smem_u32(red_bars) + 8u * i; };
+    const int n_cons = blockDim.x - 32;                                     // consumer threads (a multiple of 32)
+    const int n_warps = n_cons >> 5;
+    const int t = threadIdx.x;
+    const bool producer = t >= n_cons;
+    const long b = blockIdx.y;
+    if (t == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < stages; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), n_warps);
+        }
+        for (int i = 0; i < kRedBufs; ++i) mbar_init(red_bar(i), n_warps);
+        fence_barrier_init();
+        fence_proxy_async();
+    }
+    __syncthreads();
+    const long first = (long)blockIdx.x * kRowBatch, step = (long)gridDim.x * kRowBatch;
+    const int n_batches = first < rows_per_batch ? (int)((rows_per_batch - first + step - 1) / step) : 0;
+    if (producer) {
+        if (t == n_cons) {
+            int s = 0;
+            uint32_t phase = 0;
+            for (long r0 = first; r0 < rows_per_batch; r0 += step) {
+                if (!mbar_wait(empty_bar(s), phase ^ 1u, &abort_flag)) break;
+                const int live = (int)min((long)kRowBatch, rows_per_batch - r0);
+                mbar_arrive_expect_tx(full_bar(s), 2u * live * row_bytes);
+                const uint32_t dst = base + (uint32_t)s * stage_bytes;
+                for (int k = 0; k < live; ++k) {
+                    const long row = b * rows_per_batch + r0 + k;
+                    bulk_load_1d(dst + k * row_bytes, dy + row * cols, row_bytes, full_bar(s));
+                    bulk_load_1d(dst + (kRowBatch + k) * row_bytes, x + row * cols, row_bytes, full_bar(s));
+                }
+                if (++s == stages) {
+                    s = 0;
+                    phase ^= 1u;
+                }
+            }
+        }
+    } else {
+        const int nvec = cols >> 3;
+        const bool active = t < nvec;
+        const int lane = t & 31, warp = t >> 5;
+        const float inv_cols = 1.f / (float)cols;
+        float2 sc1[4], gt[4], acc_scale[4], acc_shift[4], acc_gate[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sc1[j] = gt[j] = acc_scale[j] = acc_shift[j] = acc_gate[j] = make_float2(0.f, 0.f);
+        auto unpack = [](const bf16x8& v, float2* o) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o[j] = __bfloat1622float2(v.v[j]);
+        };
+        if (active) {
+            unpack(ld8(scale + b * cols + t * 8), sc1);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sc1[j] = __fadd2_rn(sc1[j], make_float2(1.f, 1.f));
+            if (GATE) unpack(ld8(gate + b * cols + t * 8), gt);
+        }
+        struct Stats {
+            float mu[kRowBatch], rs[kRowBatch];
+        };
+        auto rows_of = [&](int i) { return (int)min((long)kRowBatch, rows_per_batch - (first + i * step)); };
+        auto load_stats = [&](int i) {
+            Stats v;
+            const int live = i < n_batches ? rows_of(i) : 0;
+#pragma unroll
+            for (int k = 0; k < kRowBatch; ++k) {
+                const long row = b * rows_per_batch + first + i * step + k;
+                v.mu[k] = !XHAT && k < live ? mean[row] : 0.f;
+                v.rs[k] = k < live ? rstd[row] : 0.f;
+            }
+            return v;
+        };
+        auto ring_row = [&](int s, int which, int k) {
+            uint4 a;
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w)
+                         : "r"(base + (uint32_t)s * stage_bytes + (uint32_t)t * 16u + (uint32_t)(which * kRowBatch + k) * row_bytes) : "memory");
+            return *reinterpret_cast<bf16x8*>(&a);
+        };
+        auto xhat = [&](float2 v, float mu, float rs) {
+            return XHAT ? v : __fmul2_rn(__fadd2_rn(v, make_float2(-mu, -mu)), make_float2(rs, rs));
+        };
+        // first pass over batch i (ring slot s): column sums into registers, the rows' sums into buffer i % kRedBufs
+        auto first_pass = [&](int i, int s, uint32_t phase, const Stats& st) -> bool {
+            if (!mbar_wait(full_bar(s), phase, &abort_flag)) return false;
+            const int live = rows_of(i);
+            float sums[2 * kRowBatch];
+#pragma unroll
+            for (int q = 0; q < 2 * kRowBatch; ++q) sums[q] = 0.f;
+            auto row_sums = [&](int k) {
+                float2 s1 = make_float2(0.f, 0.f), s2 = s1;
+                float2 dyv[4], xv[4];
+                unpack(ring_row(s, 0, k), dyv);
+                unpack(ring_row(s, 1, k), xv);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 xh = xhat(xv[j], st.mu[k], st.rs[k]);
+                    const float2 g = __fmul2_rn(dyv[j], sc1[j]);
+                    s1 = __fadd2_rn(s1, g);
+                    s2 = __ffma2_rn(g, xh, s2);
+                    acc_scale[j] = __ffma2_rn(dyv[j], xh, acc_scale[j]);
+                    acc_shift[j] = __fadd2_rn(acc_shift[j], dyv[j]);
+                }
+                sums[2 * k] = s1.x + s1.y;
+                sums[2 * k + 1] = s2.x + s2.y;
+            };
+            // whole batches without a test per row: each test is a block of its own, and the rows' chains cannot overlap
+            if (active) {
+                if (live == kRowBatch) {
+#pragma unroll
+                    for (int k = 0; k < kRowBatch; ++k) row_sums(k);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < kRowBatch - 1; ++k)
+                        if (k < live) row_sums(k);
+                }
+            }
+            // eight warp sums in nine shuffles (see block_sum_batch); lane 4 q ends up with value q
+            float a[4], b2[2];
+            const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) a[q] = (h16 ? sums[q + 4] : sums[q]) + __shfl_xor_sync(0xffffffffu, h16 ? sums[q] : sums[q + 4], 16);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) b2[q] = (h8 ? a[q + 2] : a[q]) + __shfl_xor_sync(0xffffffffu, h8 ? a[q] : a[q + 2], 8);
+            float c = (h4 ? b2[1] : b2[0]) + __shfl_xor_sync(0xffffffffu, h4 ? b2[0] : b2[1], 4);
+            c += __shfl_xor_sync(0xffffffffu, c, 2);
+            c += __shfl_xor_sync(0xffffffffu, c, 1);
+            if ((lane & 3) == 0) red[(i % kRedBufs) * 256 + (lane >> 2) * 32 + warp] = c;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(red_bar(i % kRedBufs));
+            return true;
+        };
+        Stats cur = load_stats(0), next;
+        if (AHEAD) next = load_stats(1);
+        int s = 0, s_next = 0;
+        uint32_t phase_next = 0;
+        auto advance = [&] {
+            if (++s_next == stages) {
+                s_next = 0;
+                phase_next ^= 1u;
+            }
+        };
+        bool ok = true;
+        if (AHEAD && n_batches > 0) {
+            ok = first_pass(0, 0, 0, cur);
+            advance();
+        }
+        for (int i = 0; ok && i < n_batches; ++i) {
+            const int live = rows_of(i);
+            const long row0 = b * rows_per_batch + first + i * step;
+            // rows that do not come through the ring: issue their loads now, they land while the ring data is reduced
+            bf16x8 pup[kRowBatch], pbr[kRowBatch];
+#pragma unroll
+            for (int k = 0; k < kRowBatch; ++k) {
+                if (active && k < live) {
+                    if (dres_in != nullptr) pup[k] = ld8(dres_in + (row0 + k) * cols + t * 8);
+                    if (GATE) pbr[k] = ld8(branch + (row0 + k) * cols + t * 8);
+                }
+            }
+            Stats later;
+            if (AHEAD) later = load_stats(i + 2);
+            if (!AHEAD) {
+                if (i > 0) cur = load_stats(i);
+                if (!(ok = first_pass(i, s_next, phase_next, cur))) break;
+                advance();
+            } else if (i + 1 < n_batches) {
+                if (!(ok = first_pass(i + 1, s_next, phase_next, next))) break;
+                advance();
+            }
+            // second pass over batch i: the rows are read from the ring again instead of being held in registers
+            if (!(ok = mbar_wait(red_bar(i % kRedBufs), (uint32_t)(i / kRedBufs) & 1u, &abort_flag))) break;
+            float tot = 0.f;
+            for (int w = lane >> 3; w < n_warps; w += 4) tot += red[(i % kRedBufs) * 256 + (lane & 7) * 32 + w];
+            tot += __shfl_xor_sync(0xffffffffu, tot, 8);
+            tot += __shfl_xor_sync(0xffffffffu, tot, 16);
+            float m[2 * kRowBatch];
+#pragma unroll
+            for (int q = 0; q < 2 * kRowBatch; ++q) m[q] = -__shfl_sync(0xffffffffu, tot, q) * inv_cols;
+            auto row_grad = [&](int k) {
+                const long at = (row0 + k) * cols + t * 8;
+                float2 dyv[4], xv[4], d[4];
+                unpack(ring_row(s, 0, k), dyv);
+                unpack(ring_row(s, 1, k), xv);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 xh = xhat(xv[j], cur.mu[k], cur.rs[k]);
+                    d[j] = __ffma2_rn(dyv[j], sc1[j], make_float2(m[2 * k], m[2 * k]));
+                    d[j] = __ffma2_rn(xh, make_float2(m[2 * k + 1], m[2 * k + 1]), d[j]);
+                    d[j] = __fmul2_rn(d[j], make_float2(cur.rs[k], cur.rs[k]));
+                }
+                if (dres_in != nullptr) {
+                    float2 up[4];
+                    unpack(pup[k], up);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) d[j] = __fadd2_rn(d[j], up[j]);
+                }
+                bf16x8 o;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) o.v[j] = __floats2bfloat162_rn(d[j].x, d[j].y);
+                st8(dx + at, o);
+                if (GATE) {
+                    float2 br[4];
+                    unpack(pbr[k], br);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        acc_gate[j] = __ffma2_rn(d[j], br[j], acc_gate[j]);
+                        const float2 g = __fmul2_rn(d[j], gt[j]);
+                        o.v[j] = __floats2bfloat162_rn(g.x, g.y);
+                    }
+                    st8(dbranch + at, o);
+                }
+            };
+            if (active) {
+                if (live == kRowBatch) {
+#pragma unroll
+                    for (int k = 0; k < kRowBatch; ++k) row_grad(k);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < kRowBatch - 1; ++k)
+                        if (k < live) row_grad(k);
+                }
+            }
+            // every consumer warp has finished with the slot: it can be refilled
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty_bar(s));
+            if (++s == stages) s = 0;
+            if (AHEAD) {
+                cur = next;
+                next = later;
+            }
+        }
+        if (active) {
+            constexpr int K = GATE ? 3 : 2;
+            float* p = partials + ((b * gridDim.x + blockIdx.x) * K) * (long)cols + t * 8;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                *reinterpret_cast<float2*>(p + 2 * j) = acc_scale[j];
+                *reinterpret_cast<float2*>(p + cols + 2 * j) = acc_shift[j];
+                if (GATE) *reinterpret_cast<float2*>(p + 2 * cols + 2 * j) = acc_gate[j];
+            }
+        }
+    }
+    __syncthreads();
+    if (abort_flag) {
+        if (t == 0) atomicExch(&g_norm_status, TT_ERR_TIMEOUT);
+        for (int i = 0; i < 200; ++i) __nanosleep(1000);      // let bulk copies in flight land before the ring goes away
+    }
+}
+
+// The gated form for 385 to 512 threads (3080 to 4096 columns), where the kernel above does not fit its 96 registers: one batch at a time,
+// unpacked, a named barrier for the sums (32656 x 4096: 375 us; the form above 421 - 469).
 __device__ __forceinline__ void consumer_sum_batch(float* v, float* red, int parity, int nthreads) {
     // block_sum_batch for the consumer threads only (named barrier 1: the producer warp never joins it)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -298,8 +576,7 @@ __device__ __forceinline__ void consumer_sum_batch(float* v, float* red, int par
     for (int q = 0; q < 8; ++q) v[q] = __shfl_sync(0xffffffffu, t, q);
 }
 
-template <bool GATE, int MAXT, bool XHAT = false>
-__global__ void __launch_bounds__(MAXT + 32) ln_mod_bwd_ring_kernel(
+__global__ void __launch_bounds__(512 + 32) ln_mod_bwd_ring_wide_gate_kernel(
     const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ dres_in,
     const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ branch,
     const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ scale,
@@ -365,7 +642,7 @@ __global__ void __launch_bounds__(MAXT + 32) ln_mod_bwd_ring_kernel(
             unpack8(ld8(scale + b * cols + t * 8), sc1);
 #pragma unroll
             for (int j = 0; j < 8; ++j) sc1[j] += 1.f;
-            if (GATE) unpack8(ld8(gate + b * cols + t * 8), gt);
+            unpack8(ld8(gate + b * cols + t * 8), gt);
         }
         int s = 0, parity = 0;
         uint32_t phase = 0;
@@ -377,11 +654,11 @@ __global__ void __launch_bounds__(MAXT + 32) ln_mod_bwd_ring_kernel(
 #pragma unroll
             for (int k = 0; k < kRowBatch; ++k) {
                 const long row = b * rows_per_batch + (k < live ? r0 + k : r0);
-                mu[k] = XHAT ? 0.f : mean[row];
+                mu[k] = mean[row];
                 rs[k] = rstd[row];
                 if (active && k < live) {
                     if (dres_in != nullptr) pup[k] = ld8(dres_in + row * cols + t * 8);
-                    if (GATE) pbr[k] = ld8(branch + row * cols + t * 8);
+                    pbr[k] = ld8(branch + row * cols + t * 8);
                 }
             }
             if (!mbar_wait(full_bar(s), phase, &abort_flag)) break;
@@ -404,7 +681,7 @@ __global__ void __launch_bounds__(MAXT + 32) ln_mod_bwd_ring_kernel(
                     unpack8(ring_row(1, k), xv);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const float xh = XHAT ? xv[j] : (xv[j] - mu[k]) * rs[k];
+                        const float xh = (xv[j] - mu[k]) * rs[k];
                         const float g = dyv[j] * sc1[j];
                         s1 += g;
                         s2 += g * xh;
@@ -426,7 +703,7 @@ __global__ void __launch_bounds__(MAXT + 32) ln_mod_bwd_ring_kernel(
                     unpack8(ring_row(1, k), xv);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const float xh = XHAT ? xv[j] : (xv[j] - mu[k]) * rs[k];
+                        const float xh = (xv[j] - mu[k]) * rs[k];
                         d[j] = rs[k] * (dyv[j] * sc1[j] - m1 - xh * m2);
                     }
                     if (dres_in != nullptr) {
@@ -436,16 +713,14 @@ __global__ void __launch_bounds__(MAXT + 32) ln_mod_bwd_ring_kernel(
                         for (int j = 0; j < 8; ++j) d[j] += up[j];
                     }
                     st8(dx + row * cols + t * 8, pack8(d));
-                    if (GATE) {
-                        float br[8], db[8];
-                        unpack8(pbr[k], br);
+                    float br[8], db[8];
+                    unpack8(pbr[k], br);
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            acc_gate[j] += d[j] * br[j];
-                            db[j] = d[j] * gt[j];
-                        }
-                        st8(dbranch + row * cols + t * 8, pack8(db));
+                    for (int j = 0; j < 8; ++j) {
+                        acc_gate[j] += d[j] * br[j];
+                        db[j] = d[j] * gt[j];
                     }
+                    st8(dbranch + row * cols + t * 8, pack8(db));
                 }
             }
             // every consumer warp has finished with the slot: it can be refilled
@@ -457,13 +732,12 @@ __global__ void __launch_bounds__(MAXT + 32) ln_mod_bwd_ring_kernel(
             }
         }
         if (active) {
-            constexpr int K = GATE ? 3 : 2;
-            float* p = partials + ((b * gridDim.x + blockIdx.x) * K) * (long)cols + t * 8;
+            float* p = partials + ((b * gridDim.x + blockIdx.x) * 3) * (long)cols + t * 8;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 p[j] = acc_scale[j];
                 p[cols + j] = acc_shift[j];
-                if (GATE) p[2 * cols + j] = acc_gate[j];
+                p[2 * cols + j] = acc_gate[j];
             }
         }
     }
@@ -891,6 +1165,17 @@ extern "C" int tt_adaln_fwd(const void* x, const void* scale, const void* shift,
 }
 
 namespace {
+template <bool GATE, bool XHAT>
+decltype(&ln_mod_bwd_ring_wide_gate_kernel) pick_ring(int size) {
+    if constexpr (GATE) {
+        if (size == 1) return ln_mod_bwd_ring_wide_gate_kernel;
+        return size == 2 ? ln_mod_bwd_ring_kernel<true, 800> : ln_mod_bwd_ring_kernel<true, 384>;
+    } else {
+        return size == 2 ? ln_mod_bwd_ring_kernel<false, 800, XHAT> : size == 1 ? ln_mod_bwd_ring_kernel<false, 512, XHAT>
+                                                                               : ln_mod_bwd_ring_kernel<false, 384, XHAT>;
+    }
+}
+
 // `xhat`: x holds normalised rows (no mean, no gate)
 int ln_mod_bwd(const void* dy, const void* dres_in, const void* x, const void* branch, const void* gate, const void* scale,
                const float* mean, const float* rstd, void* dx, void* dbranch, float* partials, void* dscale, void* dshift, void* dgate,
@@ -918,13 +1203,12 @@ int ln_mod_bwd(const void* dy, const void* dres_in, const void* x, const void* b
         if (g > nblk) g = nblk;
         nblk_used = g;
         const int smem = (int)(stages * stage_bytes) + 16 * stages + 256;
-        const bool wide = threads > 512;
-        auto kern = has_gate ? (wide ? ln_mod_bwd_ring_kernel<true, 1024> : ln_mod_bwd_ring_kernel<true, 512>)
-                  : xhat   ? (wide ? ln_mod_bwd_ring_kernel<false, 1024, true> : ln_mod_bwd_ring_kernel<false, 512, true>)
-                           : (wide ? ln_mod_bwd_ring_kernel<false, 1024> : ln_mod_bwd_ring_kernel<false, 512>);
-        static int configured[6][64] = {{0}};
+        // registers a thread may have: 128 up to 384 threads (3072 columns, the model's width), 96 up to 512, 72 up to 800
+        const int size = threads > 512 ? 2 : threads > 384 ? 1 : 0;
+        auto kern = has_gate ? pick_ring<true, false>(size) : xhat ? pick_ring<false, true>(size) : pick_ring<false, false>(size);
+        static int configured[9][64] = {{0}};
         if (dev < 0 || dev >= 64) dev = 0;
-        const int which = (has_gate ? 2 : (xhat ? 4 : 0)) + (wide ? 1 : 0);
+        const int which = (has_gate ? 3 : (xhat ? 6 : 0)) + size;
         if (configured[which][dev] < smem) {
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return tt_record_cuda(e);

@@ -219,11 +219,11 @@ def _flat_grad(ctx, weight: torch.Tensor, du: torch.Tensor) -> Optional[torch.Te
     in a flat buffer (:class:`teletron_b200.parallel.grad_buffer.ParamAndGradBuffer`), its accumulation node is part of this backward
     pass (``torch.autograd.grad`` collects the gradient instead), and nobody looks at the gradient on its way there: no hooks, no
     ``create_graph``, no batched or forward-mode gradients, and the default stream, on which accumulation nodes run too."""
-    if _transformed(du) or torch.is_grad_enabled() or _lib.raw_stream() != 0:
+    if not getattr(weight, "flat_grad", False) or _transformed(du) or torch.is_grad_enabled() or _lib.raw_stream() != 0:
         return None
     for fn, _ in ctx.next_functions:
         param = getattr(fn, "variable", None)
-        if param is None or not getattr(param, "flat_grad", False) or param.data_ptr() != weight.data_ptr() or param.shape != weight.shape:
+        if param is not weight:
             continue
         g = param.grad
         if g is None or g.dtype != BF16 or g.shape != param.shape or not g.is_contiguous() or g.requires_grad or g.device != du.device:

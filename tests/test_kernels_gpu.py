@@ -365,3 +365,32 @@ def test_bias_gradient_of_transformed_gradients(merged):
     with fwd.dual_level():
         (gb,) = torch.autograd.grad(y, b, fwd.make_dual(dy.detach(), torch.ones_like(dy)), retain_graph=True)
         assert torch.equal(fwd.unpack_dual(gb).tangent, torch.full_like(b, 32.0))
+
+
+@pytest.mark.parametrize("B,S,C", [(1, 3003, 3072), (2, 1501, 1024), (1, 3001, 3080), (1, 2999, 4096), (2, 1400, 6144)])
+@pytest.mark.parametrize("gate", [False, True])
+def test_layernorm_backward_ring_over_many_batches(B, S, C, gate):
+    """Enough four-row batches per CTA for the ring's stages and the four buffers of row sums to wrap around, ragged ends; the forms for
+    up to 384, 512 and 800 threads.  One bf16 rounding per output; column sums of S rows in fp32."""
+    from teletron_b200 import ops
+    from teletron_b200.ops import reference
+    g = torch.Generator(device="cuda").manual_seed(S + C)
+    rn = lambda *s, k=1.0: (torch.randn(*s, device=_dev(), generator=g) * k).bfloat16()  # noqa: E731
+    ins = [rn(B, S, C) * 2 + 0.5, rn(B, S, C), rn(B, C, k=0.3), rn(B, C, k=0.3), rn(B, C, k=0.3)]       # residual, branch, gate, scale, shift
+    up = [rn(B, S, C), rn(B, S, C)]
+    if not gate:
+        ins, up = [ins[0], ins[3], ins[4]], up[1:]
+    for t in ins:
+        t.requires_grad_()
+    ref = [t.detach().double().requires_grad_() for t in ins]
+    if gate:
+        out = ops.gate_residual_layernorm_modulate(*ins)
+        r = ref[0] + ref[2][:, None] * ref[1]
+        r = r + (out[0].detach().double() - r.detach())            # normalise the rounded residual, as the kernel does
+        out_ref = (r, reference.layernorm_modulate(r, ref[3], ref[4]))
+    else:
+        out, out_ref = (ops.layernorm_modulate(*ins),), (reference.layernorm_modulate(*ref),)
+    got = torch.autograd.grad(out, ins, up)
+    want = torch.autograd.grad(out_ref, ref, [t.double() for t in up])
+    for a, b in zip(got, want):
+        assert ((a.double() - b).norm() / b.norm()).item() < 4e-3
