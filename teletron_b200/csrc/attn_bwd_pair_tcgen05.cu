@@ -17,7 +17,7 @@
 // dP(c+1) -> dS(c+1) runs beside the exchange.
 //
 //   tensor core:  dK(c) dP(c+1) | dQ(c) dV(c+1) | S(c+2) ...
-//   softmax:      P(c+1) ................ | dQ(c) read-out | dS(c+1) ... | P(c+2)
+//   softmax:      P(c+1) ................ | dS(c+1) ... | P(c+2)        dQ warps:  read out dQ(c), stage it
 //
 // Shared memory holds exactly one copy of each streamed operand (Q as the operand of S and of dK, dO as that of dP and of dV: four
 // tiles of 16 KB), refilled as soon as its product has retired, a whole chunk before it is needed again.
@@ -27,8 +27,8 @@
 // not have to be on them is kept off: eight warps of their own read dQ out of tensor memory (the softmax warps doing it: 32.6 ms); the
 // exchange is a bulk copy from a buffer (stores to the peer's memory from the softmax warps held up every other shared-memory access for
 // ~1000 clocks a chunk); statistics come scaled and padded, one ld.shared each.  Registers are split by role (setmaxnreg): spills
-// in the MMA or the read-out warps cost up to 10 ms.  24 heads x 32656 tokens: 28.4 ms, 29.0 under sustained load (single CTAs: 32.7 and
-// 34.2); 3 heads x 119056: 48.5 (56.1).
+// in the MMA or the read-out warps cost up to 10 ms.  24 heads x 32656 tokens: 28.3 ms, 29.0 under sustained load (single CTAs: 32.7 and
+// 34.2); 3 heads x 119056: 47.5 (56.1).
 //
 // Synchronisation (mbarriers, bounded waits): "leader" barriers live in CTA 0, whose MMA thread issues for the pair; commits arrive
 // in both CTAs.  The bytes of the exchange complete on a barrier of the receiving CTA; CTA 1 passes that on to the leader.
@@ -165,10 +165,10 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     constexpr uint32_t kT1 = 0, kDQ = 64, kT2 = 128, kAccV = 256, kAccK = 384;
     // barrier addresses are computed anew from here on: kept from the initialisation they would be spilled
     asm volatile("mov.u32 %0, %0;" : "+r"(base));
-    if (warp < kFirstSoftmax) reg_dec<kRegsMisc>();
-    else if (warp < kFirstDrain) reg_inc<kRegsSoftmax>();
-    else reg_dec<kRegsDrain>();
-
+    // The split stands inside the branches that the roles share: ahead of them, where the paths meet again, the compiler holds every role
+    // to the smallest share and spills (24 heads x 6144 tokens: 1.144 -> 1.103 ms, x 32656: 28.7 -> 28.3).
+    if (warp < kFirstSoftmax) {
+    reg_dec<kRegsMisc>();
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer (one per CTA: its halves)
         if (elect_one()) {
@@ -237,14 +237,9 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             constexpr uint32_t idesc_t = idesc_bf16(2 * BK, BC, false, false);   // T = A B^T, both K-major
             constexpr uint32_t idesc_a = idesc_bf16(2 * BK, D, false, true);     // acc += (tensor-memory A) B, B MN-major
             constexpr uint32_t idesc_q = idesc_bf16(BC, D, true, true);          // dQ = dS K: both operands MN-major
-            // Products advance their operands by the address field of the descriptors (units of 16 bytes).  `fresh` keeps the compiler from
-            // computing all ~100 descriptors ahead of the chunk loop, where they would be spilled and every issue would wait for loads.
-            auto fresh = [](uint64_t d) {
-                asm volatile("" : "+l"(d));
-                return d;
-            };
+            // with all ~100 descriptors hoisted out of the chunk loop they are spilled, and every issue waits for loads
             auto issue_t = [&](uint32_t t_col, int oa, int ob) {
-                const uint64_t da = fresh(smem_desc_sw128(base + oa, 16, 1024)), db = fresh(smem_desc_sw128(base + ob, 16, 1024));
+                const uint64_t da = fresh_desc(smem_desc_sw128(base + oa, 16, 1024)), db = fresh_desc(smem_desc_sw128(base + ob, 16, 1024));
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk)
                     umma2_bf16_ss(tmem + t_col, da + (uint64_t)(((kk >> 2) * kSlab + (kk & 3) * 32) >> 4),
@@ -270,7 +265,7 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 if (!mbar_wait(bar(dovFull), (uint32_t)c & 1u, &abort_flag)) return false;
                 if (!mbar_wait(bar(pReady), (uint32_t)c & 1u, &abort_flag)) return false;
                 tc_fence_after();
-                const uint64_t db = fresh(smem_desc_sw128(base + oDOv, kSlab, 1024));
+                const uint64_t db = fresh_desc(smem_desc_sw128(base + oDOv, kSlab, 1024));
 #pragma unroll
                 for (int kk = 0; kk < BC / 16; ++kk)
                     umma2_bf16_ts(tmem + kAccV, tmem + kT1 + p_col(kk >> 1) + (kk & 1) * 8, db + (uint64_t)(kk * (2048 >> 4)),
@@ -288,7 +283,7 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 if (!mbar_wait(bar(qkFull), par, &abort_flag)) goto done;
                 if (!mbar_wait(bar(dsReady), par, &abort_flag)) goto done;      // dS(c) in T2
                 tc_fence_after();
-                const uint64_t dqk = fresh(smem_desc_sw128(base + oQk, kSlab, 1024));
+                const uint64_t dqk = fresh_desc(smem_desc_sw128(base + oQk, kSlab, 1024));
 #pragma unroll
                 for (int kk = 0; kk < BC / 16; ++kk)                                // dK += dS^T Q
                     umma2_bf16_ts(tmem + kAccK, tmem + kT2 + (kk >> 1) * 32 + (kk & 1) * 8, dqk + (uint64_t)(kk * (2048 >> 4)),
@@ -302,7 +297,7 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 if (!mbar_wait(bar(exIn), par, &abort_flag)) goto done;         // and the other ones
                 if (!mbar_wait(bar(exPeer), par, &abort_flag)) goto done;
                 tc_fence_after();
-                const uint64_t dds = fresh(smem_desc_sw128(base + oDS, kSlab, 1024)), dkb = fresh(smem_desc_sw128(base + oKB, kSlab, 1024));
+                const uint64_t dds = fresh_desc(smem_desc_sw128(base + oDS, kSlab, 1024)), dkb = fresh_desc(smem_desc_sw128(base + oKB, kSlab, 1024));
 #pragma unroll
                 for (int kk = 0; kk < 2 * BK / 16; ++kk)                            // dQ(c) = dS K over the pair's 256 keys
                     umma2_bf16_ss(tmem + kDQ, dds + (uint64_t)(kk * (2048 >> 4)), dkb + (uint64_t)(kk * (2048 >> 4)), idesc_q, kk ? 1u : 0u);
@@ -337,7 +332,9 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             }
             bulk_wait_all();
         }
+    }
     } else if (warp >= kFirstDrain) {
+        reg_dec<kRegsDrain>();
         // ------------------------------------------------------------ dQ read-out: two halves of 32 columns through one buffer
         // lane l of the CTA holds query 64 rank + l % 64, columns 64 (l / 64) + 0 .. 63
         const int quad = warp & 3, half = (warp - kFirstDrain) >> 2;
@@ -364,6 +361,7 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             if (lane == 0) mbar_arrive(bar(staged));
         }
     } else {
+        reg_inc<kRegsSoftmax>();
         // ------------------------------------------------------------ softmax / dS
         const int part = (warp - kFirstSoftmax) >> 2;                  // queries [32 part, 32 part + 32) of every chunk
         const int quad = warp & 3;

@@ -320,6 +320,13 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr, uint32_t
     return d;
 }
 
+// Products advance their operands by adding to the descriptors' address field (units of 16 bytes).  Passed through this first, a
+// descriptor's steps are computed where they are used: otherwise the compiler hoists all of them out of the tile loop.
+__device__ __forceinline__ uint64_t fresh_desc(uint64_t d) {
+    asm volatile("" : "+l"(d));
+    return d;
+}
+
 // Instruction descriptor for kind::f16 with bf16 inputs and fp32 accumulation.
 __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n, bool a_mn_major, bool b_mn_major) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn_major ? 1u : 0u) << 15) | ((b_mn_major ? 1u : 0u) << 16) |
