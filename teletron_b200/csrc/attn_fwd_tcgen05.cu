@@ -346,7 +346,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 }
             }
         }
-        if (row < p.S) p.lse[(long)bh * p.lse_pitch + row] = (m + log2f(l)) * 0.6931471805599453f;
+        // the padding that this CTA's rows cover (all of it for a pitch of S rounded up to 64) says "no such query" to the backward
+        if (row < p.lse_pitch) p.lse[(long)bh * p.lse_pitch + row] = row < p.S ? (m + log2f(l)) * 0.6931471805599453f : INFINITY;
     }
 
 done:
@@ -364,7 +365,8 @@ done:
 
 }  // namespace
 
-// q, k, v: [BH, S, 128] bf16 contiguous; out [B, S, H*128] bf16; lse [BH, lse_pitch] fp32 (rows < S written).
+// q, k, v: [BH, S, 128] bf16 contiguous; out [B, S, H*128] bf16; lse [BH, lse_pitch] fp32: rows < S, and +inf in the
+// padding up to the next multiple of 256 rows.
 static int attn_fwd_launch(const void* q, const void* k, const void* v, void* out, float* lse, int B, int H, int S,
                            int kv_len, int mask_lo, int mask_hi, int lse_pitch, float scale, int* status, void* stream,
                            void* const* peer_out, int n_peers, int my_rank, int text_len, int s_local, long dest_ld);
@@ -395,6 +397,7 @@ static int attn_fwd_launch(const void* q, const void* k, const void* v, void* ou
                            void* const* peer_out, int n_peers, int my_rank, int text_len, int s_local, long dest_ld) {
     if (B <= 0 || H <= 0 || S <= 0 || kv_len <= 0 || kv_len > S || lse_pitch < S || status == nullptr) return TT_ERR_ARG;
     if (mask_lo < mask_hi && (mask_lo < 0 || (mask_lo == 0 && mask_hi >= kv_len))) return TT_ERR_ARG;
+    const int dev = tt_device().dev;            // first: it also makes the device's context current in a thread that has not used it
     CUtensorMap tq, tk, tv;
     int rc;
     const uint64_t BH = (uint64_t)B * H;
@@ -404,8 +407,6 @@ static int attn_fwd_launch(const void* q, const void* k, const void* v, void* ou
     static bool configured[2][64] = {{false}};       // per device: the attribute belongs to the device's context
     const int pre = scale > 0.f ? 0 : 1;
     auto kern = pre ? attn_fwd_kernel<true> : attn_fwd_kernel<false>;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
     if (!configured[pre][dev]) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
         if (e != cudaSuccess) return tt_record_cuda(e);

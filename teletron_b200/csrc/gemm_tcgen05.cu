@@ -634,6 +634,9 @@ int sm_count() { return tt_device().sms; }
 tt_device_info tt_device() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return {0, 148};
+    // cuTensorMapEncodeTiled needs a current context, which a thread that has only allocated from a cache does not have yet
+    static thread_local int bound = -1;
+    if (bound != dev && cudaSetDevice(dev) == cudaSuccess) bound = dev;
     if (g_sms[dev] == 0) {
         int n = 0;
         if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;

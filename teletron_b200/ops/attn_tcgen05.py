@@ -39,7 +39,7 @@ def forward(q, k, v, kv_valid_len: Optional[int], scale: Optional[float], mask_r
     q, k, v = (check(t.contiguous(), BF16, n) for t, n in ((q, "q"), (k, "k"), (v, "v")))
     out = torch.empty(B, S, H * D, dtype=BF16, device=q.device)
     pitch = (S + 63) // 64 * 64       # the backward reads statistics in aligned chunks of 64 queries
-    lse = torch.full((B, H, pitch), float("inf"), dtype=torch.float32, device=q.device)
+    lse = torch.empty(B, H, pitch, dtype=torch.float32, device=q.device)      # the kernel writes +inf into the padding
     kv_len = S if kv_valid_len is None else min(int(kv_valid_len), S)
     sc = (1.0 / math.sqrt(D)) if scale is None else float(scale)
     lo, hi = _mask(mask_range, kv_len)

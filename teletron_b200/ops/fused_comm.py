@@ -354,7 +354,7 @@ class _FusedAttentionOutProj(torch.autograd.Function):
         if cached is None:
             out = torch.empty(1, ws.S_tot, ws.h_loc * 128, dtype=BF16, device=q.device)
             pitch = (ws.S_tot + 63) // 64 * 64
-            lse = torch.full((1, ws.h_loc, pitch), float("inf"), dtype=torch.float32, device=q.device)
+            lse = torch.empty(1, ws.h_loc, pitch, dtype=torch.float32, device=q.device)
             call("tt_attn_fwd_push", ptr(q), ptr(k), ptr(v), ptr(out), ptr(lse), c_int(ws.h_loc), c_int(ws.S_tot), c_int(kvl),
                  c_int(mlo), c_int(mhi), c_int(pitch), c_float(sc), ptr(status_tensor(q.device)), stream(), ws.table("g"), c_int(ws.cp),
                  c_int(ws.rank), c_int(T), c_int(s), c_long(H_all * 128))

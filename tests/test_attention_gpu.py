@@ -205,3 +205,18 @@ def test_one_pass_backward_against_64_bits(B, H, S, kv_len, mask):
     for a, r in zip(got, (ds @ kd, ds.transpose(-1, -2) @ qd, p.transpose(-1, -2) @ dd)):
         assert _rel(a, r) < 5e-3
         assert torch.isfinite(a).all()
+
+
+@pytest.mark.parametrize("S,scale", [(1, None), (63, None), (64, None), (129, -0.1), (250, None), (449, None), (1237, None)])
+def test_forward_fills_the_padding_of_its_statistics(S, scale):
+    """The log-sum-exp rows are S rounded up to 64 long; the forward itself writes +inf behind the last query."""
+    from teletron_b200.ops import attn_tcgen05 as A
+    from teletron_b200.ops.gemm_tcgen05 import check_status
+    pitch = (S + 63) // 64 * 64
+    junk = torch.full((2, 3, pitch), -7.0, device="cuda")
+    del junk                                        # the allocator hands the same block out again
+    q, k, v = (torch.randn(2, 3, S, 128, device="cuda").bfloat16() for _ in range(3))
+    lse = A.forward(q, k, v, None, scale)[1]
+    check_status()
+    assert lse.shape[-1] == pitch and torch.isfinite(lse[..., :S]).all()
+    assert (lse[..., S:] == float("inf")).all()
