@@ -1106,13 +1106,21 @@ extern "C" int tt_norm_status(void) {
     return v;
 }
 
+// Threads per CTA of the forward (a warp a row).  With fewer rows than eight an SM they are spread over the SMs instead of filling CTAs of
+// eight on a few of them, where a row's loads queue behind its neighbours': 256 x 3072 6.9 -> 6.0 us (gated 10.1 -> 9.4, fused_adaln
+// 7.4 -> 6.1), 40 rows 6.8 -> 5.8, 1000 rows 7.2 -> 6.2; from 1037 rows on nothing changes.
+static int fwd_block(long rows) {
+    const long warps = (rows + 147) / 148;
+    return warps < 8 ? 32 * (int)warps : 256;
+}
+
 #define LAUNCH_FWD(VPL)                                                                                         \
     do {                                                                                                        \
         if (has_gate)                                                                                           \
-            ln_mod_fwd_kernel<VPL, true><<<grid, 256, 0, st>>>(X, BR, G, SC, SH, NR, Y, nullptr, mean, rstd,    \
+            ln_mod_fwd_kernel<VPL, true><<<grid, block, 0, st>>>(X, BR, G, SC, SH, NR, Y, nullptr, mean, rstd,    \
                                                                rows, cols, rows_per_batch, eps);                \
         else                                                                                                    \
-            ln_mod_fwd_kernel<VPL, false><<<grid, 256, 0, st>>>(X, BR, G, SC, SH, NR, Y, nullptr, mean, rstd,   \
+            ln_mod_fwd_kernel<VPL, false><<<grid, block, 0, st>>>(X, BR, G, SC, SH, NR, Y, nullptr, mean, rstd,   \
                                                                 rows, cols, rows_per_batch, eps);               \
     } while (0)
 
@@ -1130,7 +1138,8 @@ extern "C" int tt_ln_mod_fwd(const void* x, const void* branch, const void* gate
     auto NR = (__nv_bfloat16*)new_res;
     auto Y = (__nv_bfloat16*)y;
     cudaStream_t st = (cudaStream_t)stream;
-    long want = (rows + 7) / 8;
+    const int block = fwd_block(rows);
+    const long want = (rows * 32 + block - 1) / block;
     const int grid = (int)(want < 148L * 16 ? want : 148L * 16);
     const int vpl = ((cols >> 3) + 31) / 32;
     if (vpl <= 4) LAUNCH_FWD(4);
@@ -1147,11 +1156,12 @@ extern "C" int tt_adaln_fwd(const void* x, const void* scale, const void* shift,
                             float eps, void* stream) {
     if (bad_cols(cols) || rows <= 0) return TT_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
-    const long want = (rows + 7) / 8;
+    const int block = fwd_block(rows);
+    const long want = (rows * 32 + block - 1) / block;
     const int grid = (int)(want < 148L * 16 ? want : 148L * 16);
     const int vpl = ((cols >> 3) + 31) / 32;
 #define ADALN_FWD(VPL)                                                                                                          \
-    ln_mod_fwd_kernel<VPL, false, true><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, nullptr, nullptr, (const __nv_bfloat16*)scale, \
+    ln_mod_fwd_kernel<VPL, false, true><<<grid, block, 0, st>>>((const __nv_bfloat16*)x, nullptr, nullptr, (const __nv_bfloat16*)scale, \
                                                               (const __nv_bfloat16*)shift, nullptr, (__nv_bfloat16*)y,          \
                                                               (__nv_bfloat16*)xn, nullptr, rstd, rows, cols, rows, eps)
     if (vpl <= 4) ADALN_FWD(4);

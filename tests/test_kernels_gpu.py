@@ -394,3 +394,17 @@ def test_layernorm_backward_ring_over_many_batches(B, S, C, gate):
     want = torch.autograd.grad(out_ref, ref, [t.double() for t in up])
     for a, b in zip(got, want):
         assert ((a.double() - b).norm() / b.norm()).item() < 4e-3
+
+
+@pytest.mark.parametrize("rows", [1, 148, 149, 297, 1036, 1037, 1185])
+def test_layernorm_forward_block_sizes(rows):
+    """The forward's CTAs hold one to eight rows by the row count: the edges of that rule, with and without the gated residual."""
+    from teletron_b200 import ops
+    from teletron_b200.ops import reference
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    rn = lambda *s: torch.randn(*s, device=_dev(), generator=g).bfloat16()  # noqa: E731
+    x, br, ga, sc, sh = rn(1, rows, 264), rn(1, rows, 264), rn(1, 264), rn(1, 264), rn(1, 264)
+    assert _rel(ops.layernorm_modulate(x, sc, sh), reference.layernorm_modulate(x.float(), sc.float(), sh.float())) < 4e-3
+    r, y = ops.gate_residual_layernorm_modulate(x, br, ga, sc, sh)
+    assert _rel(r, x.float() + ga.float()[:, None] * br.float()) < 4e-3
+    assert _rel(y, reference.layernorm_modulate(r.float(), sc.float(), sh.float())) < 4e-3
