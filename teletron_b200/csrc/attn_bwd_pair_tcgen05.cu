@@ -31,7 +31,9 @@
 // 34.2); 3 heads x 119056: 47.5 (56.1).
 //
 // Synchronisation (mbarriers, bounded waits): "leader" barriers live in CTA 0, whose MMA thread issues for the pair; commits arrive
-// in both CTAs.  The bytes of the exchange complete on a barrier of the receiving CTA; CTA 1 passes that on to the leader.
+// in both CTAs.  The bytes of the exchange complete on a barrier of the receiving CTA.  CTA 1's relay thread passes that on to the leader,
+// together with its softmax warps' own half of dS, which they have stored for products that the leader issues: its one arrival a chunk
+// releases at cluster scope (a fence each time; on every arrival of the softmax warps: 52 ms instead of 38 at 24 heads x 32656 tokens).  utils/pair_pipeline_model.py checks the protocol.
 #include "common.cuh"
 #include "sm100.cuh"
 #include "teletron_b200.h"
@@ -112,11 +114,11 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         kvFull, qsFull, qkFull, dopFull, dovFull,
         sRead,                   // S(c) is in registers everywhere: T1 takes P(c) and dQ(c-1)
         pReady, dsReady, dqRead,
-        exPeer,                  // CTA 1 has received its half of the exchange
-        dsOwn,                   // both CTAs have stored their own half of dS(c) in their dS tiles
+        exPeer,                  // CTA 1's dS tile is complete, both halves
         // in both CTAs, reached by commits
         qsEmpty, qkEmpty, dopEmpty, dovEmpty, sFull, dpFull, dqFull, accFinal,
         // each CTA's own
+        dsOwn,                   // its own half of dS(c) is in the dS tile
         exIn,                    // the peer's half of dS has arrived in the dS tile
         exStaged,                // the peer's half of dS(c) is complete in oOut
         staged, stageFree,       // [2]: that half of dQ(c) has left the staging buffer
@@ -143,8 +145,7 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             int count = 1;
             if (i == sRead || i == pReady || i == dsReady) count = 2 * 4 * kGroups;      // every softmax warp of both CTAs
             if (i == dqRead) count = 2 * 8;
-            if (i == dsOwn) count = 4 * kGroups;
-            if (i == exStaged) count = 2 * kGroups;
+            if (i == dsOwn || i == exStaged) count = 2 * kGroups;
             if (i == staged) count = 4;
             if (i >= quadRead) count = 2;
             mbar_init(bar(i), (uint32_t)count);
@@ -223,12 +224,13 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             }
         }
     } else if (warp == 1 && rank == 1) {
-        // ------------------------------------------------------------ relay: the exchange has arrived here
+        // ------------------------------------------------------------ relay: the dS tile of this CTA is complete
         if (elect_one()) {
             for (int c = 0; c < n_chunks; ++c) {
                 mbar_arrive_expect_tx(bar(exIn), kSlab);
+                if (!mbar_wait(bar(dsOwn), (uint32_t)c & 1u, &abort_flag)) goto done;
                 if (!mbar_wait(bar(exIn), (uint32_t)c & 1u, &abort_flag)) goto done;
-                mbar_arrive_leader(bar(exPeer));
+                mbar_arrive_leader_release(bar(exPeer));
             }
         }
     } else if (warp == 1) {
@@ -293,9 +295,9 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 // T1's last columns: S(c+1) has been read (and dQ(c-1) before it was issued); behind the last chunk only dQ(c-1) is left
                 if (more && !mbar_wait(bar(sRead), par ^ 1u, &abort_flag)) goto done;
                 if (!more && c > 0 && !mbar_wait(bar(dqRead), par ^ 1u, &abort_flag)) goto done;
-                if (!mbar_wait(bar(dsOwn), par, &abort_flag)) goto done;        // dS(c) in the dS tiles: own halves
-                if (!mbar_wait(bar(exIn), par, &abort_flag)) goto done;         // and the other ones
-                if (!mbar_wait(bar(exPeer), par, &abort_flag)) goto done;
+                if (!mbar_wait(bar(dsOwn), par, &abort_flag)) goto done;        // dS(c) in the dS tile here: own half
+                if (!mbar_wait(bar(exIn), par, &abort_flag)) goto done;         // and the other one
+                if (!mbar_wait<true>(bar(exPeer), par, &abort_flag)) goto done; // and both in CTA 1
                 tc_fence_after();
                 const uint64_t dds = fresh_desc(smem_desc_sw128(base + oDS, kSlab, 1024)), dkb = fresh_desc(smem_desc_sw128(base + oKB, kSlab, 1024));
 #pragma unroll
@@ -461,8 +463,7 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) {
-                    if (mine) mbar_arrive_leader(bar(dsOwn));
-                    else mbar_arrive(bar(exStaged));
+                    mbar_arrive(bar(mine ? dsOwn : exStaged));
                 }
             }
         }

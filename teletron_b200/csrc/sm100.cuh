@@ -56,12 +56,27 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 
 constexpr long long kWaitCycles = 2000000000LL;   // ~1 s at B200 clocks
 
+// the same at cluster scope: what threads of another CTA released there before they arrived is visible behind it
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Returns false when the wait was abandoned (timeout here, or abort raised elsewhere in the CTA).
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-    if (mbar_try_wait(bar, parity)) return true;
+    auto try_wait = [&] { return CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
+    if (try_wait()) return true;
     const long long t0 = clock64();
     for (uint32_t it = 1;; ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (try_wait()) return true;
         if ((it & 255u) == 0u) {
             if (*abort_flag) return false;
             if (clock64() - t0 > kWaitCycles) {
@@ -266,6 +281,10 @@ __device__ __forceinline__ void umma2_commit_both(uint32_t bar) {
 // plain arrival on the leader CTA's copy of a barrier (from either CTA)
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar & kPeerMask) : "memory");
+}
+// the same, releasing at cluster scope what this thread has written or has acquired from its CTA
+__device__ __forceinline__ void mbar_arrive_leader_release(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar & kPeerMask) : "memory");
 }
 // this shared-memory address in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
