@@ -1,0 +1,112 @@
+"""Weight gradients that a product adds to a flat gradient buffer itself: whoever could see a gradient on its way to the buffer still
+does.  The product is a stand-in on the CPU; the decision is the one of the kernels' autograd functions."""
+
+import pytest
+import torch
+
+from teletron_b200.ops import _lib, cuda_ops, gemm
+
+
+class _Product(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, w):
+        ctx.save_for_backward(x, w)
+        return x @ w.t()
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, w = ctx.saved_tensors
+        return dy @ w, cuda_ops._weight_grad(ctx, w, dy, x)
+
+
+@pytest.fixture
+def added(monkeypatch):
+    """Weights whose gradient a product has added itself, in order."""
+    log = []
+
+    def add(a, b, out):
+        log.append(tuple(out.shape))
+        out.add_((a.t() @ b).to(out.dtype))
+        return True
+    monkeypatch.setattr(gemm, "gemm_tn_add", add)
+    monkeypatch.setattr(_lib, "raw_stream", lambda: 0)
+    return log
+
+
+def _weight(rows=4):
+    w = torch.nn.Parameter(torch.randn(rows, 4).bfloat16())
+    w.grad = torch.zeros_like(w)
+    w.flat_grad = True
+    return w
+
+
+def _node(w):
+    return w.expand_as(w).grad_fn.next_functions[0][0]
+
+
+X = torch.randn(3, 4).bfloat16()
+
+
+def test_product_is_added_where_nobody_looks(added):
+    w = _weight()
+    for _ in range(2):
+        _Product.apply(X, w).sum().backward()
+    assert added == [(4, 4)] * 2
+    torch.testing.assert_close(w.grad, (2 * X.sum(0)).expand(4, 4).bfloat16(), rtol=2 ** -7, atol=2 ** -7)
+
+
+@pytest.mark.parametrize("register", ["register_hook", "register_prehook"])
+@pytest.mark.parametrize("held", [True, False])
+def test_hooks_on_the_accumulation_node_see_the_gradient(added, register, held):
+    """The form that data-parallel wrappers use: a hook on the node that accumulates, which the wrapper keeps alive, or which lives as
+    long as the graph."""
+    w, seen = _weight(), []
+
+    def hook(*grads):
+        seen.append(grads[-1][0] if register == "register_hook" else grads[0][0])
+    node = _node(w)
+    if held:
+        getattr(node, register)(hook)
+        y = _Product.apply(X, w)
+    else:
+        y = _Product.apply(X, w)
+        getattr(y.grad_fn.next_functions[1][0], register)(hook)
+        del node
+    y.sum().backward()
+    assert added == [] and len(seen) == 1 and seen[0] is not None
+    assert torch.equal(seen[0], w.grad)
+
+
+def test_prehook_on_the_accumulation_node_changes_the_gradient(added):
+    w = _weight()
+    node = _node(w)
+    handle = node.register_prehook(lambda g: (g[0] * 0,))
+    _Product.apply(X, w).sum().backward()
+    assert not w.grad.any()
+    handle.remove()
+    _Product.apply(X, w).sum().backward()
+    assert added == [(4, 4)] and w.grad.any()
+
+
+def test_tensor_hooks_and_multi_grad_hooks_see_the_gradient(added):
+    w, seen = _weight(), []
+    handles = [w.register_hook(seen.append), torch.autograd.graph.register_multi_grad_hook((w,), lambda g: seen.append(g[0]))]
+    _Product.apply(X, w).sum().backward()
+    assert added == [] and len(seen) == 2 and all(g is not None for g in seen)
+    for h in handles:
+        h.remove()
+    w.register_post_accumulate_grad_hook(lambda p: seen.append(p.grad))
+    _Product.apply(X, w).sum().backward()
+    assert added == [] and len(seen) == 3
+
+
+def test_weight_used_twice_with_and_without_a_hook(added):
+    w = _weight()
+    _Product.apply(_Product.apply(X, w), w).sum().backward()
+    assert len(added) == 2
+    seen, before = [], w.grad.clone()
+    y = _Product.apply(_Product.apply(X, w), w)
+    y.grad_fn.next_functions[1][0].register_prehook(lambda g: seen.append(g[0]))
+    y.sum().backward()
+    assert len(added) == 2 and len(seen) == 1
+    torch.testing.assert_close(w.grad, before + seen[0])
