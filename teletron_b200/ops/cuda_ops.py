@@ -234,9 +234,9 @@ def _flat_grad(ctx, weight: torch.Tensor, du: torch.Tensor) -> Optional[torch.Te
     """The gradient buffer that autograd is about to add ``weight``'s gradient to, if the product may do that itself: the parameter lives
     in a flat buffer (:class:`teletron_b200.parallel.grad_buffer.ParamAndGradBuffer`), its accumulation node is part of this backward
     pass (``torch.autograd.grad`` collects the gradient instead), and nobody looks at the gradient on its way there: no hooks on
-    the parameter or on its node, no ``create_graph``, no batched or forward-mode gradients, and the default stream, on which
-    accumulation nodes run too."""
-    if not getattr(weight, "flat_grad", False) or _transformed(du) or torch.is_grad_enabled() or _lib.raw_stream() != 0:
+    the parameter or on its node, no ``create_graph``, no batched or forward-mode gradients, no anomaly mode, and the default
+    stream, on which accumulation nodes run too."""
+    if not getattr(weight, "flat_grad", False) or _transformed(du) or torch.is_grad_enabled() or _lib.raw_stream() != 0 or torch.is_anomaly_enabled():
         return None
     for fn, _ in ctx.next_functions:
         param = getattr(fn, "variable", None)

@@ -110,3 +110,14 @@ def test_weight_used_twice_with_and_without_a_hook(added):
     y.sum().backward()
     assert len(added) == 2 and len(seen) == 1
     torch.testing.assert_close(w.grad, before + seen[0])
+
+
+def test_anomaly_detection_sees_a_nan_weight_gradient(added):
+    """Anomaly mode looks at the gradients that functions return."""
+    w = _weight()
+    x = torch.full((3, 4), float("nan")).bfloat16()
+    with pytest.warns(UserWarning), torch.autograd.detect_anomaly():
+        y = _Product.apply(x, w)
+        with pytest.raises(RuntimeError, match="nan values"):
+            y.sum().backward()
+    assert added == [] and not w.grad.isnan().any()
