@@ -261,6 +261,7 @@ def _weight_grad(ctx, weight: torch.Tensor, du: torch.Tensor, x: torch.Tensor) -
     4 bytes per weight where a temporary and a separate addition move 10."""
     buf = _flat_grad(ctx, weight, du)
     if buf is not None and gemm.gemm_tn_add(du, x, buf):
+        torch.autograd.graph.increment_version(buf)
         return None
     return _gemm_tn(du, x)
 
@@ -369,6 +370,7 @@ class _LinearMerged(torch.autograd.Function):
             buf = _flat_grad(ctx, weight, du)
             if buf is not None and gemm_tcgen05.add_supported(du, a2, buf[:, k1:]) and gemm.gemm_tn_add(du, a1, buf[:, :k1]):
                 gemm.gemm_tn_add(du, a2, buf[:, k1:])
+                torch.autograd.graph.increment_version(buf)
             else:
                 dw = torch.empty_like(weight)
                 gemm.gemm_tn_into(du, a1, dw[:, :k1])

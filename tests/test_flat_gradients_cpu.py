@@ -26,7 +26,7 @@ def added(monkeypatch):
 
     def add(a, b, out):
         log.append(tuple(out.shape))
-        out.add_((a.t() @ b).to(out.dtype))
+        out.data.add_((a.t() @ b).to(out.dtype))        # through raw pointers: autograd does not see it
         return True
     monkeypatch.setattr(gemm, "gemm_tn_add", add)
     monkeypatch.setattr(_lib, "raw_stream", lambda: 0)
@@ -121,3 +121,13 @@ def test_anomaly_detection_sees_a_nan_weight_gradient(added):
         with pytest.raises(RuntimeError, match="nan values"):
             y.sum().backward()
     assert added == [] and not w.grad.isnan().any()
+
+
+def test_buffer_saved_for_another_backward_is_known_to_have_changed(added):
+    w = _weight()
+    k = torch.ones((), dtype=torch.bfloat16, requires_grad=True)
+    z = (w.grad * k).sum()                  # saves the buffer
+    _Product.apply(X, w).sum().backward()
+    assert added == [(4, 4)]
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        z.backward()
