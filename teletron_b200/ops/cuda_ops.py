@@ -218,16 +218,31 @@ def _no_hook(*_):
     return None
 
 
-def _node_hooked(node) -> bool:
-    """Whether Python hooks are registered on an accumulation node (the form that data-parallel wrappers use).  A node does not tell,
-    but a hook that is registered lands in the dictionary that holds the others (3.5 us for the two kinds)."""
-    for register in (node.register_prehook, node.register_hook):
-        handle = register(_no_hook)
-        hooks = handle.hooks_dict_ref()
-        handle.remove()
-        if hooks:
-            return True
-    return False
+class _AfterDefaultStream:
+    """Pre-hook of an accumulation node whose gradient a product adds on the default stream.  The node runs on the stream it was created
+    on, and the caller of ``backward`` waits for that one only: a node of another stream waits for the product first."""
+
+    def __call__(self, grads):
+        self.handle.remove()
+        if _lib.raw_stream() != 0:
+            torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
+
+
+def _claim_node(node) -> bool:
+    """False if Python hooks are registered on an accumulation node (the form that data-parallel wrappers use).  A node does not
+    tell, but a hook that is registered lands in the dictionary that holds the others.  Otherwise its pre-hook is in place."""
+    handle = node.register_hook(_no_hook)
+    hooks = handle.hooks_dict_ref()
+    handle.remove()
+    if hooks:
+        return False
+    join = _AfterDefaultStream()
+    join.handle = node.register_prehook(join)
+    hooks = join.handle.hooks_dict_ref()
+    if len(hooks) > 1:
+        join.handle.remove()
+        return all(type(h) is _AfterDefaultStream for h in hooks.values())      # of another use of the weight in this pass
+    return True
 
 
 def _flat_grad(ctx, weight: torch.Tensor, du: torch.Tensor) -> Optional[torch.Tensor]:
@@ -235,7 +250,7 @@ def _flat_grad(ctx, weight: torch.Tensor, du: torch.Tensor) -> Optional[torch.Te
     in a flat buffer (:class:`teletron_b200.parallel.grad_buffer.ParamAndGradBuffer`), its accumulation node is part of this backward
     pass (``torch.autograd.grad`` collects the gradient instead), and nobody looks at the gradient on its way there: no hooks on
     the parameter or on its node, no ``create_graph``, no batched or forward-mode gradients, no anomaly mode, and the default
-    stream, on which accumulation nodes run too."""
+    stream."""
     if not getattr(weight, "flat_grad", False) or _transformed(du) or torch.is_grad_enabled() or _lib.raw_stream() != 0 or torch.is_anomaly_enabled():
         return None
     for fn, _ in ctx.next_functions:
@@ -252,7 +267,7 @@ def _flat_grad(ctx, weight: torch.Tensor, du: torch.Tensor) -> Optional[torch.Te
                 return None
         except RuntimeError:        # a leaf that torch.autograd.grad collects
             return None
-        return None if _node_hooked(fn) else g
+        return g if _claim_node(fn) else None
     return None
 
 

@@ -347,3 +347,30 @@ def test_flat_gradient_buffers_receive_products_only_where_autograd_accumulates(
         plain(x).backward(dy)
     for n in ("w1", "w2", "w3"):
         torch.testing.assert_close(getattr(net, n).grad, getattr(plain, n).grad, rtol=1.6e-2, atol=2e-2)
+
+
+def test_flat_gradient_added_before_an_accumulation_node_of_another_stream_runs():
+    """The node was created under a side stream, which is all that the caller of ``backward`` waits for: the product that the default
+    stream adds meanwhile has to come before it."""
+    from teletron_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x, dy = (torch.randn(64, 256, device="cuda", generator=g).bfloat16() for _ in range(2))
+    w = torch.nn.Parameter(torch.zeros(256, 256, device="cuda", dtype=torch.bfloat16))
+    w.grad = torch.zeros_like(w)
+    w.flat_grad = True
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        node = w.expand_as(w).grad_fn.next_functions[0][0]
+    ops.linear(x, w).backward(dy)
+    torch.cuda.synchronize()
+    want = w.grad.clone()
+    w.grad.zero_()
+    y = ops.linear(x, w)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(100_000_000)              # the product waits behind this, ~50 ms
+    with torch.cuda.stream(side):
+        y.backward(dy)
+        got = w.grad.clone()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and want.any()
+    assert node.variable is w
