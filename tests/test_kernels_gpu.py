@@ -408,3 +408,17 @@ def test_layernorm_forward_block_sizes(rows):
     r, y = ops.gate_residual_layernorm_modulate(x, br, ga, sc, sh)
     assert _rel(r, x.float() + ga.float()[:, None] * br.float()) < 4e-3
     assert _rel(y, reference.layernorm_modulate(r.float(), sc.float(), sh.float())) < 4e-3
+
+
+def test_noise_level_of_a_pipeline_built_under_a_device_context():
+    """Built under ``torch.device("cuda")`` the pipeline's table of noise levels is on the device already."""
+    from teletron_b200.models.hunyuanvideo import FlowConfig, HunyuanPipeline, tiny_config
+    cfg = tiny_config(in_channels=16)
+    shape = (2, 16, 1, 4, 4)
+    with torch.device("cuda"):
+        there = HunyuanPipeline(cfg, FlowConfig(model_type="t2v"), dtype=torch.bfloat16)
+    here = HunyuanPipeline(cfg, FlowConfig(model_type="t2v"), device=_dev(), dtype=torch.bfloat16)
+    assert there.scheduler.sigmas.is_cuda and not here.scheduler.sigmas.is_cuda
+    a, b = (p._draw(2, shape, _dev(), torch.bfloat16) for p in (there, here))
+    torch.testing.assert_close(a[0], b[0], rtol=1e-6, atol=0)
+    assert a[0].is_cuda and b[0].is_cuda and torch.equal(a[1], b[1])
