@@ -1023,19 +1023,20 @@ int tt_attn_bwd_pair(const void* q, const void* k, const void* v, const void* do
                      void* dv, int B, int H, int S, int kv_len, int mask_lo, int mask_hi, float scale, int* status, cudaStream_t st);
 
 // One-pass backward: row dots and statistics, the kernel that forms dK, dV and accumulates dQ in fp32 (on CTA pairs or single CTAs), then
-// the scale-and-round pass.  lse: [B*H, pitch]; workspace: B * H * roundup(S, 128) * 130 floats of any contents.
+// the scale-and-round pass.  lse: [B*H, pitch], pitch a multiple of 64; workspace: B * H * roundup(S, 128) * 130 floats of any contents.
 extern "C" int tt_attn_bwd_fused(const void* q, const void* k, const void* v, const void* out, const void* dout,
                                  const float* lse, float* workspace, size_t workspace_floats, void* dq, void* dk, void* dv, int B, int H,
                                  int S, int kv_len, int mask_lo, int mask_hi, int pitch, float scale, int* status,
                                  void* stream) {
     if (B <= 0 || H <= 0 || S <= 0 || kv_len <= 0 || kv_len > S || status == nullptr || workspace == nullptr) return TT_ERR_ARG;
     if (mask_lo < mask_hi && (mask_lo < 0 || (mask_lo == 0 && mask_hi >= kv_len))) return TT_ERR_ARG;
-    for (const void* x : {q, k, v, out, dout, (const void*)workspace, (const void*)dq, (const void*)dk, (const void*)dv})
+    for (const void* x : {q, k, v, dout, (const void*)lse, (const void*)workspace, (const void*)dq, (const void*)dk, (const void*)dv})
         if ((uintptr_t)x & 15) return TT_ERR_ARG;
+    if ((uintptr_t)out & 7) return TT_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     const uint64_t BH = (uint64_t)B * H;
     const int s_pad = (S + BC - 1) / BC * BC;
-    if (pitch < S || workspace_floats < BH * (uint64_t)s_pad * (D + 2)) return TT_ERR_ARG;
+    if (pitch < S || (pitch & 63) || workspace_floats < BH * (uint64_t)s_pad * (D + 2)) return TT_ERR_ARG;
     float* dq_acc = workspace;
     float* stats = workspace + BH * (uint64_t)s_pad * D;
     const long nwork = (long)BH * s_pad, want = (nwork + 7) / 8;

@@ -1,0 +1,25 @@
+"""What the C entries refuse before they touch a device.  The pointers are made up, so nothing here runs where there is one."""
+
+import pytest
+import torch
+
+from teletron_b200.ops import _lib
+from teletron_b200.ops._lib import c_float, c_int, c_size
+
+pytestmark = pytest.mark.skipif(torch.cuda.is_available() or not _lib.available(), reason="needs the library and no device")
+
+ARG, BASE = 1, 1 << 20
+
+
+def _attn_bwd(out=BASE, lse=BASE, dq=BASE, pitch=192, work=None, S=130):
+    p = _lib.ctypes.c_void_p
+    floats = 2 * 256 * 130 if work is None else work
+    return _lib.lib().tt_attn_bwd_fused(p(BASE), p(BASE), p(BASE), p(out), p(BASE), p(lse), p(BASE), c_size(floats), p(dq), p(BASE), p(BASE),
+                                        c_int(1), c_int(2), c_int(S), c_int(S), c_int(0), c_int(0), c_int(pitch), c_float(0.1), p(BASE), p(0))
+
+
+def test_attention_backward_takes_and_refuses_what_it_did():
+    """Statistics in rows of a multiple of 64, 16-byte aligned; the forward's output is read in 8-byte pieces."""
+    assert _attn_bwd() != ARG and _attn_bwd(out=BASE + 8) != ARG
+    assert _attn_bwd(pitch=130) == ARG and _attn_bwd(pitch=128) == ARG and _attn_bwd(lse=BASE + 4) == ARG
+    assert _attn_bwd(out=BASE + 4) == ARG and _attn_bwd(dq=BASE + 8) == ARG and _attn_bwd(work=2 * 256 * 130 - 1) == ARG
