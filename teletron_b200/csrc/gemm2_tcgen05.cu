@@ -338,8 +338,8 @@ __global__ void __launch_bounds__(256) splitk_finish_kernel(const float* __restr
 // The product of every entry point.  a2 (or nullptr) supplies the K columns from k1 on; splits > 1 needs `scratch`.
 int run2(const void* a, const void* a2, int k1, long lda2, const void* b, void* c, const void* bias, void* aux, int M, int N, int K, long lda,
          long ldb, long ldc, int a_mn, int b_mn, int epi, int splits, float* scratch, int* status, void* stream) {
-    // with both operands K x MN (a_mn and b_mn) K is a row count, which need not be a multiple of 8: the rows beyond it load as zeros
-    if (M <= 0 || N <= 0 || K <= 0 || (N & 7) || ((K & 7) && !(a_mn && b_mn)) || (ldc & 7) || status == nullptr) return TT_ERR_ARG;
+    // epilogue 5 (both operands K x MN) takes any K, there a row count: the rows beyond it load as zeros
+    if (M <= 0 || N <= 0 || K <= 0 || (N & 7) || ((K & 7) && epi != 5) || (ldc & 7) || status == nullptr) return TT_ERR_ARG;
     if (a_mn && (M & 7)) return TT_ERR_ARG;
     if (epi < 0 || epi > 5 || (epi >= 1 && epi <= 4 && aux == nullptr)) return TT_ERR_ARG;
     if (epi == 5 && (!a_mn || !b_mn || bias != nullptr || splits != 1)) return TT_ERR_ARG;

@@ -23,3 +23,16 @@ def test_attention_backward_takes_and_refuses_what_it_did():
     assert _attn_bwd() != ARG and _attn_bwd(out=BASE + 8) != ARG
     assert _attn_bwd(pitch=130) == ARG and _attn_bwd(pitch=128) == ARG and _attn_bwd(lse=BASE + 4) == ARG
     assert _attn_bwd(out=BASE + 4) == ARG and _attn_bwd(dq=BASE + 8) == ARG and _attn_bwd(work=2 * 256 * 130 - 1) == ARG
+
+
+def _gemm2(K, epi, entry="tt_gemm2_bf16"):
+    lib = _lib.lib()
+    if entry == "tt_gemm2_bf16_splitk":
+        return lib.tt_gemm2_bf16_splitk(BASE, BASE, BASE, 0, 0, 256, 256, K, 256, 256, 256, 1, 1, epi, 2, BASE, BASE, 0)
+    return lib.tt_gemm2_bf16(BASE, BASE, BASE, 0, 0, 256, 256, K, 256, 256, 256, 1, 1, epi, BASE, 0)
+
+
+def test_only_the_adding_epilogue_takes_any_row_count():
+    assert _gemm2(128, 0) != ARG and _gemm2(128, 0, "tt_gemm2_bf16_splitk") != ARG
+    assert _gemm2(7, 5) != ARG and _gemm2(129, 5) != ARG
+    assert _gemm2(7, 0) == ARG and _gemm2(129, 0) == ARG and _gemm2(129, 0, "tt_gemm2_bf16_splitk") == ARG
