@@ -50,7 +50,7 @@ constexpr int kHalfSlab = 64 * 128;         // [64 rows x 64 columns] bf16: 8 KB
 constexpr int kGroups = 4;                  // softmax warpgroups: 32 queries of every chunk each
 constexpr int kThreads = 128 + 128 * kGroups + 256;     // TMA, MMA (CTA 1: relay), exchange, reductions; softmax; dQ read-out
 constexpr int kFirstSoftmax = 4, kFirstDrain = kFirstSoftmax + 4 * kGroups;     // warps
-// registers per thread: 80 at launch, then split; the sum stays below what the block was launched with
+// registers per thread: what the compiler launches the block with, then split (the launcher checks it)
 constexpr int kRegsLaunch = 72, kRegsMisc = 56, kRegsSoftmax = 88, kRegsDrain = 48;
 static_assert(128 * (kRegsMisc + kGroups * kRegsSoftmax + 2 * kRegsDrain) <= kThreads * kRegsLaunch, "register split");
 constexpr int kStageFloats = 64 * 64;       // half of the dQ of one chunk and CTA
@@ -541,7 +541,12 @@ int tt_attn_bwd_pair(const void* q, const void* k, const void* v, const void* do
     static bool configured[64] = {false};
     const int dev = tt_device().dev;
     if (!configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(attn_bwd_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+        // setmaxnreg.inc waits, without a bound, for registers that the block was launched with
+        cudaFuncAttributes at;
+        cudaError_t e = cudaFuncGetAttributes(&at, attn_bwd_pair_kernel);
+        if (e != cudaSuccess) return tt_record_cuda(e);
+        if (at.numRegs < kRegsLaunch) return TT_ERR_LIMIT;
+        e = cudaFuncSetAttribute(attn_bwd_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
         if (e != cudaSuccess) return tt_record_cuda(e);
         configured[dev] = true;
     }
