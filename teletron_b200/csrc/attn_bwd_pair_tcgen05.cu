@@ -31,9 +31,11 @@
 // 34.2); 3 heads x 119056: 47.5 (56.1).
 //
 // Synchronisation (mbarriers, bounded waits): "leader" barriers live in CTA 0, whose MMA thread issues for the pair; commits arrive
-// in both CTAs.  The bytes of the exchange complete on a barrier of the receiving CTA.  CTA 1's relay thread passes that on to the leader,
-// together with its softmax warps' own half of dS, which they have stored for products that the leader issues: its one arrival a chunk
-// releases at cluster scope (a fence each time; on every arrival of the softmax warps: 52 ms instead of 38 at 24 heads x 32656 tokens).  utils/pair_pipeline_model.py checks the protocol.
+// in both CTAs.  The bytes of the exchange complete, at cluster scope, on a barrier of the receiving CTA.  CTA 1's relay thread passes that
+// on to the leader, and with it its softmax warps' own half of dS, which they have stored for products that the leader issues: for those
+// it fences at cluster scope, while the exchange is under way.  (Released by the arrival itself, behind the exchange: 30.6 ms instead of
+// 28.5 at 24 heads x 32656 tokens, 52.3 instead of 47.6 at 3 x 119056; by arrivals of the softmax warps: 14 ms more.)
+// utils/pair_pipeline_model.py checks the protocol.
 #include "common.cuh"
 #include "sm100.cuh"
 #include "teletron_b200.h"
@@ -229,8 +231,9 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             for (int c = 0; c < n_chunks; ++c) {
                 mbar_arrive_expect_tx(bar(exIn), kSlab);
                 if (!mbar_wait(bar(dsOwn), (uint32_t)c & 1u, &abort_flag)) goto done;
+                fence_cluster();
                 if (!mbar_wait(bar(exIn), (uint32_t)c & 1u, &abort_flag)) goto done;
-                mbar_arrive_leader_release(bar(exPeer));
+                mbar_arrive_leader_relaxed(bar(exPeer));
             }
         }
     } else if (warp == 1) {

@@ -14,8 +14,8 @@ of them.  Reported are conditions above that fail, deadlocks, reads that find ot
 which one writes that the graph does not order.
 
 Scopes.  Shared memory of one CTA that its threads wrote with ordinary stores and that an instruction issued in the other CTA reads has
-to be released and acquired at cluster scope somewhere between the two: for such pairs an arrival of CTA scope on the other
-CTA's barrier, or a wait of CTA scope for it, orders nothing.  (Tensor memory is handed over under the tcgen05 fences, copies and
+to be released and acquired at cluster scope somewhere between the two: for such pairs an arrival on the other CTA's barrier orders
+what came before the arriving thread's last cluster fence, if the wait for it is of cluster scope, and nothing otherwise.  (Tensor memory is handed over under the tcgen05 fences, copies and
 commits complete on barriers at cluster scope.)
 
 The programs are transcribed from the kernel; a change of its synchronisation has to be mirrored here.
@@ -34,13 +34,14 @@ P_CELL = (0, 2, 1, 3)               # 16-column cell of T1 that takes group g's 
 @dataclass(frozen=True)
 class Variant:
     """Switches that re-introduce hazards the kernel's synchronisation exists to prevent (to show the model sees them)."""
-    cluster_scope: bool = True          # CTA 1's half of dS is released and acquired at cluster scope
+    cluster_fence: bool = True          # CTA 1's relay fences at cluster scope behind its softmax warps' half of dS
+    cluster_acquire: bool = True        # and the leader acquires there
     wait_last_dq_read: bool = True      # behind the last chunk, dQ waits until the dQ before it has been read
     wait_quad_read: bool = True         # groups 2, 3 store P once groups 0, 1 have read their scores
     wait_dq_before_ds: bool = True      # dS(c) is stored once dQ(c - 1) has been formed
 
 
-# Operations: ("wait", (barrier, cta), parity, cluster scope?), ("arrive", (barrier, cta), weight, cluster scope?), ("read" / "write",
+# Operations: ("wait", (barrier, cta), parity, cluster scope?), ("arrive", (barrier, cta), weight), ("fence", "cluster"), ("read" / "write",
 # buffer, tag), ("tc", reads, writes, commits) and ("copy", reads, writes, barrier or None, label), ("drained", label): the copy
 # with that label has read its source.
 
@@ -49,10 +50,10 @@ def _producer(r: int, n: int) -> List[Tuple]:
         return ("copy", [], [((buf, r), tag)], (bar, 0), None)
 
     def expect(bar):
-        return [("arrive", (bar, 0), 1, False)] if r == 0 else []
+        return [("arrive", (bar, 0), 1)] if r == 0 else []
 
     def stats(c):
-        return [("arrive", (f"stFull{c & 1}", r), 1, False), ("copy", [], [((f"stat{c & 1}", r), ("stat", c))], (f"stFull{c & 1}", r), None)]
+        return [("arrive", (f"stFull{c & 1}", r), 1), ("copy", [], [((f"stat{c & 1}", r), ("stat", c))], (f"stFull{c & 1}", r), None)]
 
     ops = expect("kvFull") + [load("KV", "KV", "kvFull")] + stats(0) + (stats(1) if n > 1 else [])
     for c in range(n + 1):
@@ -93,13 +94,13 @@ def _mma(n: int, v: Variant) -> List[Tuple]:
     ops = [wait("kvFull", 0)] + scores(0) + dp(0) + dv(0) + (scores(1) if n > 1 else [])
     for c in range(n):
         par, more = c & 1, c + 1 < n
-        ops += [("arrive", ("exIn", 0), 1, False), wait("qkFull", par), wait("dsReady", par),
+        ops += [("arrive", ("exIn", 0), 1), wait("qkFull", par), wait("dsReady", par),
                 tc([(f"T2.{2 * g}", ("dS", c)) for g in range(GROUPS)] + [("Qk", ("Qk", c))], [("accK", ("dK", c))], "qkEmpty")]
         if more:
             ops += dp(c + 1) + [wait("sRead", par ^ 1)]
         elif c > 0 and v.wait_last_dq_read:
             ops.append(wait("dqRead", par ^ 1))
-        ops += [wait("dsOwn", par), wait("exIn", par), wait("exPeer", par, v.cluster_scope),
+        ops += [wait("dsOwn", par), wait("exIn", par), wait("exPeer", par, v.cluster_acquire),
                 tc([("dSown", ("dS", c)), ("dSpeer", ("dS", c)), ("KV", "KV")], [(f"T1.{i}", ("dQ", c)) for i in range(4, 8)], "dqFull")]
         if more:
             ops += dv(c + 1)
@@ -111,8 +112,8 @@ def _mma(n: int, v: Variant) -> List[Tuple]:
 def _relay(n: int, v: Variant) -> List[Tuple]:
     ops: List[Tuple] = []
     for c in range(n):
-        ops += [("arrive", ("exIn", 1), 1, False), ("wait", ("dsOwn", 1), c & 1, False), ("wait", ("exIn", 1), c & 1, False),
-                ("arrive", ("exPeer", 0), 1, v.cluster_scope)]
+        ops += [("arrive", ("exIn", 1), 1), ("wait", ("dsOwn", 1), c & 1, False)] + ([("fence", "cluster")] if v.cluster_fence else [])
+        ops += [("wait", ("exIn", 1), c & 1, False), ("arrive", ("exPeer", 0), 1)]
     return ops
 
 
@@ -128,7 +129,7 @@ def _reducer(r: int, n: int) -> List[Tuple]:
     ops: List[Tuple] = []
     for i in range(2 * n):
         ops += [("wait", ("staged", r), i & 1, False), ("copy", [(("stage", r), ("dQ", i >> 1, i & 1))], [], None, ("red", r, i)),
-                ("drained", ("red", r, i)), ("arrive", (f"stageFree{i & 1}", r), 1, False)]
+                ("drained", ("red", r, i)), ("arrive", (f"stageFree{i & 1}", r), 1)]
     return ops
 
 
@@ -137,10 +138,10 @@ def _drain(r: int, half: int, n: int) -> List[Tuple]:
     for c in range(n):
         ops.append(("wait", ("dqFull", r), c & 1, False))
         ops += [("read", (f"T1.{4 + 2 * half + i}", r), ("dQ", c)) for i in (0, 1)]
-        ops.append(("arrive", ("dqRead", 0), 4, False))
+        ops.append(("arrive", ("dqRead", 0), 4))
         if c > 0 or half > 0:
             ops.append(("wait", (f"stageFree{half ^ 1}", r), (c if half else c - 1) & 1, False))
-        ops += [("write", ("stage", r), ("dQ", c, half)), ("arrive", ("staged", r), 4, False)]
+        ops += [("write", ("stage", r), ("dQ", c, half)), ("arrive", ("staged", r), 4)]
     return ops
 
 
@@ -152,17 +153,17 @@ def _softmax(r: int, g: int, n: int, v: Variant) -> List[Tuple]:
         ops += [("wait", (f"stFull{par}", r), (c >> 1) & 1, False), ("wait", ("sFull", r), par, False)]
         ops += [("read", (f"T1.{2 * g + i}", r), ("S", c)) for i in (0, 1)]
         if g < 2:
-            ops.append(("arrive", ("quadRead", r), 1, False))
-        ops += [("arrive", ("sRead", 0), 4, False), ("read", (f"stat{par}", r), ("stat", c))]
+            ops.append(("arrive", ("quadRead", r), 1))
+        ops += [("arrive", ("sRead", 0), 4), ("read", (f"stat{par}", r), ("stat", c))]
         if g >= 2 and v.wait_quad_read:
             ops.append(("wait", ("quadRead", r), par, False))
-        ops += [("write", (f"T1.{P_CELL[g]}", r), ("P", c)), ("arrive", ("pReady", 0), 4, False), ("wait", ("dpFull", r), par, False)]
+        ops += [("write", (f"T1.{P_CELL[g]}", r), ("P", c)), ("arrive", ("pReady", 0), 4), ("wait", ("dpFull", r), par, False)]
         ops += [("read", (f"T2.{2 * g + i}", r), ("dP", c)) for i in (0, 1)]
-        ops += [("read", (f"stat{par}", r), ("stat", c)), ("write", (f"T2.{2 * g}", r), ("dS", c)), ("arrive", ("dsReady", 0), 4, False)]
+        ops += [("read", (f"stat{par}", r), ("stat", c)), ("write", (f"T2.{2 * g}", r), ("dS", c)), ("arrive", ("dsReady", 0), 4)]
         if c > 0 and v.wait_dq_before_ds:
             ops.append(("wait", ("dqFull", r), par ^ 1, False))
         # the two groups of a half write rows of one tile: a buffer each, read together
-        ops += [("write", ("dSown" if mine else "out", r, g & 1), ("dS", c)), ("arrive", ("dsOwn" if mine else "exStaged", r), 4, False)]
+        ops += [("write", ("dSown" if mine else "out", r, g & 1), ("dS", c)), ("arrive", ("dsOwn" if mine else "exStaged", r), 4)]
     return ops + [("wait", ("accFinal", r), 0, False), ("read", ("accV", r), ("dV", n - 1)), ("read", ("accK", r), ("dK", n - 1))]
 
 
@@ -213,9 +214,9 @@ def check(chunks: int, variant: Variant = Variant()) -> List[str]:
             progs[f"softmax {r}.{g}"] = (r, _softmax(r, g, n, variant))
     G, out = _Graph(), []
     pending: Dict[Tuple, int] = {}
-    phase_arrivals: Dict[Tuple, List[Tuple[int, int, bool]]] = defaultdict(list)    # barrier -> arrivals of the current phase
+    phase_arrivals: Dict[Tuple, List[Tuple]] = defaultdict(list)    # barrier -> arrivals of the current phase
     completed: Dict[Tuple, List[int]] = defaultdict(list)                           # barrier -> completion nodes
-    foreign: Dict[Tuple, List[List[int]]] = defaultdict(list)                       # ... the cluster-scope arrivals from the other CTA
+    foreign: Dict[Tuple, List[List[int]]] = defaultdict(list)                       # ... the fences ahead of arrivals from the other CTA
     complete_with: Dict[Tuple, List[int]] = defaultdict(list)                       # ... and all its arrivals, as a bit set
     arrival_phase: List[Tuple[int, Tuple, int]] = []
     waits: List[Tuple[int, Tuple, int]] = []                                        # node, barrier, phases completed when it passed
@@ -223,23 +224,23 @@ def check(chunks: int, variant: Variant = Variant()) -> List[str]:
     accesses: Dict[Tuple, List[Tuple[int, bool, bool]]] = defaultdict(list)         # node, writes?, by ordinary stores?
     copies: Dict[Tuple, int] = {}
 
-    def arrive(bar, node, weight, cta, cluster, asynchronous=False):
+    def arrive(bar, node, weight, cta, fence, asynchronous):
         arrival_phase.append((node, bar, len(completed[bar])))
-        phase_arrivals[bar].append((node, cta, cluster or asynchronous))
+        phase_arrivals[bar].append((node, asynchronous or cta == bar[1], fence))
         left = pending.get(bar, counts[bar[0]]) - weight
         if left < 0:
             out.append(f"{G.label[node]}: beyond the count of {bar}")
         if left <= 0:
             done = G.node(f"{bar} phase {len(completed[bar])}", bar[1])
             far, arrivals = [], 0
-            for a, where, ok in phase_arrivals.pop(bar):
+            for a, plain, behind in phase_arrivals.pop(bar):
                 arrivals |= 1 << a
                 G.into[done].append(a)
                 G.into_late[done].append(a)
-                if where == bar[1] or asynchronous:
+                if plain:
                     G.into_cluster[done].append(a)
-                elif ok:
-                    far.append(a)
+                elif behind is not None:
+                    far.append(behind)
             completed[bar].append(done)
             foreign[bar].append(far)
             complete_with[bar].append(arrivals)
@@ -256,6 +257,7 @@ def check(chunks: int, variant: Variant = Variant()) -> List[str]:
 
     pc = {a: 0 for a in progs}
     last: Dict[str, int] = {a: G.node(a, r) for a, (r, _) in progs.items()}
+    fences: Dict[str, int] = {}
     last_tc = None
     moved = True
     while moved:
@@ -276,11 +278,13 @@ def check(chunks: int, variant: Variant = Variant()) -> List[str]:
                     if op[3]:
                         G.into_cluster[node] += foreign[bar][-1]
                 waits.append((node, bar, done))
+            elif op[0] == "fence":
+                node = fences[a] = G.node(name, r, last[a])
             elif op[0] == "drained":
                 node = G.node(name, r, last[a], copies[op[1]])
             elif op[0] == "arrive":
                 node = G.node(name, r, last[a])
-                arrive(op[1], node, op[2], r, op[3])
+                arrive(op[1], node, op[2], r, fences.get(a), False)
             elif op[0] in ("read", "write"):
                 node = G.node(name, r, last[a])
                 access(node, op[1], op[2], op[0] == "write", not op[1][0].startswith(("T1", "T2", "acc")))
@@ -292,7 +296,7 @@ def check(chunks: int, variant: Variant = Variant()) -> List[str]:
                 for b, t in op[2]:
                     access(run, b, t, True, False)
                 if op[3] is not None:
-                    arrive(op[3], run, 1, r, True, True)
+                    arrive(op[3], run, 1, r, None, True)
                 if op[4] is not None:
                     copies[op[4]] = run
             else:
@@ -303,7 +307,7 @@ def check(chunks: int, variant: Variant = Variant()) -> List[str]:
                 for b, t in op[2]:
                     access(last_tc, b, t, True, False)
                 for bar in op[3]:
-                    arrive(bar, last_tc, 1, r, True, True)
+                    arrive(bar, last_tc, 1, r, None, True)
             last[a] = node
             pc[a] += 1
             moved = True
@@ -311,7 +315,7 @@ def check(chunks: int, variant: Variant = Variant()) -> List[str]:
     if stuck:
         return out + ["deadlock: " + ", ".join(stuck)]
 
-    # reachability as bit sets; the nodes' numbers are a topological order, but for completions, which follow their last arrival at once
+    # reachability as bit sets; a node's number is above those of its predecessors
     def reach(into):
         before = [0] * len(into)
         for i, preds in enumerate(into):
@@ -324,6 +328,7 @@ def check(chunks: int, variant: Variant = Variant()) -> List[str]:
     for i, preds in enumerate(G.into_late):
         for p in preds:
             late_before[i] |= all_before[p] | (1 << p)
+
     def known(node, bar, k):        # every arrival of phase k comes before the node looks at the barrier
         return complete_with[bar][k] & ~late_before[node] == 0
 

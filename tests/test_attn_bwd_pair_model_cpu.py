@@ -13,7 +13,8 @@ def test_pair_protocol_orders_every_buffer(chunks):
 
 
 @pytest.mark.parametrize("variant,needle", [
-    (Variant(cluster_scope=False), "('dSown', 1, 0) at cluster scope"),
+    (Variant(cluster_fence=False), "('dSown', 1, 0) at cluster scope"),
+    (Variant(cluster_acquire=False), "('dSown', 1, 1) at cluster scope"),
     (Variant(wait_last_dq_read=False), "are not ordered on ('T1.4', 0)"),
     (Variant(wait_quad_read=False), "are not ordered on ('T1.1', 0)"),
     (Variant(wait_dq_before_ds=False), "are not ordered on ('out', 0, 0)"),
