@@ -384,7 +384,8 @@ class _LinearMerged(torch.autograd.Function):
         if ctx.needs_input_grad[2]:
             buf = _flat_grad(ctx, weight, du)
             if buf is not None and gemm_tcgen05.add_supported(du, a2, buf[:, k1:]) and gemm.gemm_tn_add(du, a1, buf[:, :k1]):
-                gemm.gemm_tn_add(du, a2, buf[:, k1:])
+                if not gemm.gemm_tn_add(du, a2, buf[:, k1:]):
+                    raise _lib.NativeError("half of a merged projection's weight gradient could not be added")
                 torch.autograd.graph.increment_version(buf)
             else:
                 dw = torch.empty_like(weight)

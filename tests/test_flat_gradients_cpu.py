@@ -131,3 +131,16 @@ def test_buffer_saved_for_another_backward_is_known_to_have_changed(added):
     assert added == [(4, 4)]
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         z.backward()
+
+
+def test_merged_projection_adds_both_halves_or_fails(added, monkeypatch):
+    """The first half is in the buffer already when the second is refused: that must not pass for a whole gradient."""
+    w = torch.nn.Parameter(torch.randn(4, 8).bfloat16())
+    w.grad, w.flat_grad = torch.zeros_like(w), True
+    monkeypatch.setattr(cuda_ops.gemm_tcgen05, "add_supported", lambda a, b, out: True)
+    cuda_ops.linear_merged(X, X, w).sum().backward()
+    assert added == [(4, 4), (4, 4)] and torch.equal(w.grad[:, :4], w.grad[:, 4:]) and w.grad.any()
+    first = gemm.gemm_tn_add
+    monkeypatch.setattr(gemm, "gemm_tn_add", lambda a, b, out: len(added) < 3 and first(a, b, out))
+    with pytest.raises(_lib.NativeError):
+        cuda_ops.linear_merged(X, X, w).sum().backward()
