@@ -1018,17 +1018,23 @@ static bool pairs_are_faster(uint64_t heads, int tiles, int sms) {
     return (double)pairs * (2.25 * tiles + 15.1) <= (double)single * (2.9 * tiles + 13.7);
 }
 
+extern "C" int tt_attn_bwd_uses_pairs(int heads, int S, int sms) {
+    return heads > 0 && S > 0 && sms > 1 && pairs_are_faster((uint64_t)heads, (S + BC - 1) / BC, sms) ? 1 : 0;
+}
+
 // attn_bwd_pair_tcgen05.cu
 int tt_attn_bwd_pair(const void* q, const void* k, const void* v, const void* dout, const float* stats, float* dq_acc, void* dq, void* dk,
                      void* dv, int B, int H, int S, int kv_len, int mask_lo, int mask_hi, float scale, int* status, cudaStream_t st);
 
 // One-pass backward: row dots and statistics, the kernel that forms dK, dV and accumulates dQ in fp32 (on CTA pairs or single CTAs), then
 // the scale-and-round pass.  lse: [B*H, pitch], pitch a multiple of 64; workspace: B * H * roundup(S, 128) * 130 floats of any contents.
+// route: 0 by pairs_are_faster, 1 single CTAs, 2 CTA pairs.
 extern "C" int tt_attn_bwd_fused(const void* q, const void* k, const void* v, const void* out, const void* dout,
                                  const float* lse, float* workspace, size_t workspace_floats, void* dq, void* dk, void* dv, int B, int H,
-                                 int S, int kv_len, int mask_lo, int mask_hi, int pitch, float scale, int* status,
+                                 int S, int kv_len, int mask_lo, int mask_hi, int pitch, float scale, int route, int* status,
                                  void* stream) {
     if (B <= 0 || H <= 0 || S <= 0 || kv_len <= 0 || kv_len > S || status == nullptr || workspace == nullptr) return TT_ERR_ARG;
+    if (route < 0 || route > 2) return TT_ERR_ARG;
     if (mask_lo < mask_hi && (mask_lo < 0 || (mask_lo == 0 && mask_hi >= kv_len))) return TT_ERR_ARG;
     for (const void* x : {q, k, v, dout, (const void*)lse, (const void*)workspace, (const void*)dq, (const void*)dk, (const void*)dv})
         if ((uintptr_t)x & 15) return TT_ERR_ARG;
@@ -1044,7 +1050,7 @@ extern "C" int tt_attn_bwd_fused(const void* q, const void* k, const void* v, co
     attn_bwd_prep_kernel<<<(int)(want < 148L * 16 ? want : 148L * 16), 256, 0, st>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, lse, stats,
                                                                                     dq_acc, B, S, H, pitch, s_pad);
     TT_CHECK_LAUNCH();
-    if (pairs_are_faster(BH, s_pad / BC, tt_device().sms))
+    if (route == 2 || (route == 0 && pairs_are_faster(BH, s_pad / BC, tt_device().sms)))
         return tt_attn_bwd_pair(q, k, v, dout, stats, dq_acc, dq, dk, dv, B, H, S, kv_len, mask_lo, mask_hi, scale, status, st);
     CUtensorMap tq_s, tk_s, tv_s, tdo_s;
     int rc;

@@ -121,10 +121,13 @@ int tt_attn_fwd_push(const void* q, const void* k, const void* v, void* out, flo
 int tt_attn_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse,
                 float* delta, void* dq, void* dk, void* dv, int B, int H, int S, int kv_len, int mask_lo, int mask_hi,
                 int pitch, float scale, int* status, void* stream);
-/* one pass over the scores, dQ accumulated in fp32 with bulk reductions; workspace: B * H * roundup(S, 128) * 130 floats */
+/* one pass over the scores, dQ accumulated in fp32 with bulk reductions; workspace: B * H * roundup(S, 128) * 130 floats;
+ * route: 0 the faster kernel, 1 single CTAs, 2 CTA pairs */
 int tt_attn_bwd_fused(const void* q, const void* k, const void* v, const void* out, const void* dout, const float* lse,
                       float* workspace, size_t workspace_floats, void* dq, void* dk, void* dv, int B, int H, int S,
-                      int kv_len, int mask_lo, int mask_hi, int pitch, float scale, int* status, void* stream);
+                      int kv_len, int mask_lo, int mask_hi, int pitch, float scale, int route, int* status, void* stream);
+/* the kernel that route 0 takes on a device of `sms` SMs (1: CTA pairs); touches no device */
+int tt_attn_bwd_uses_pairs(int heads, int S, int sms);
 
 /* ---- symmetric heap + in-kernel collectives over IPC-mapped peer memory (comm.cu) ---- */
 int tt_symm_alloc(size_t bytes, void** out);                 /* cudaMalloc + zero */

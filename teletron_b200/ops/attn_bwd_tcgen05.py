@@ -35,7 +35,12 @@ def supported(q: torch.Tensor) -> bool:
     return _lib.available() and q.is_cuda and q.dtype == BF16 and q.dim() == 4 and q.shape[-1] == 128
 
 
-def backward(dout, q, k, v, out, lse, scale: float, kv_len: int, outs=None, mask_range=(0, 0)):
+def uses_pairs(heads: int, S: int, sms: int = 148) -> bool:
+    """Whether the one-pass backward of ``heads`` (batch included) x ``S`` tokens takes the CTA-pair kernel."""
+    return bool(_lib.lib().tt_attn_bwd_uses_pairs(c_int(heads), c_int(S), c_int(sms)))
+
+
+def backward(dout, q, k, v, out, lse, scale: float, kv_len: int, outs=None, mask_range=(0, 0), route: int = 0):
     """``outs``: optional ``(dq, dk, dv)`` tensors to write into (contiguous, shaped like ``q``), e.g. regions of a
     symmetric heap that peers will read."""
     B, H, S, D = q.shape
@@ -54,7 +59,7 @@ def backward(dout, q, k, v, out, lse, scale: float, kv_len: int, outs=None, mask
         work = torch.empty(B * H * ((S + 127) // 128 * 128) * (D + 2), dtype=torch.float32, device=q.device)
         call("tt_attn_bwd_fused", ptr(q), ptr(k), ptr(v), ptr(out), ptr(dout), ptr(lse), ptr(work), c_size(work.numel()), ptr(dq), ptr(dk),
              ptr(dv), c_int(B), c_int(H), c_int(S), c_int(kv_len), c_int(mask_range[0]), c_int(mask_range[1]), c_int(pitch),
-             c_float(scale), ptr(status_tensor(q.device)), stream())
+             c_float(scale), c_int(route), ptr(status_tensor(q.device)), stream())
         return dq, dk, dv
     delta = torch.zeros(B, H, pitch, dtype=torch.float32, device=q.device)
     COUNTERS["split"] += 1
