@@ -27,7 +27,7 @@ _LAYOUTS = {"nt": (0, 0), "nn": (0, 1), "tn": (1, 1)}
 # TELETRON_B200_GEMM_2CTA=0 keeps everything on the single-CTA kernel
 PAIR_KERNEL = os.environ.get("TELETRON_B200_GEMM_2CTA", "1") != "0"
 PAIR_MIN_TILES = 74
-COUNTERS = {"pair": 0, "single": 0, "split": 0}
+COUNTERS = {"pair": 0, "single": 0, "split": 0, "add": 0}       # "add": those of "pair" that added to their output
 # What a split product takes the host to issue: a scratch allocation and a second launch on top of the 12.4 us of the others.
 SPLIT_ISSUE_US = 17.5
 
@@ -159,6 +159,7 @@ def gemm_add(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> None:
     """``out += a.T @ b``: the product is rounded to bf16, then added with one more rounding, as a separate addition would."""
     (K, M), N = a.shape, b.shape[1]
     COUNTERS["pair"] += 1
+    COUNTERS["add"] += 1
     call("tt_gemm2_bf16", a.data_ptr(), b.data_ptr(), out.data_ptr(), None, None, M, N, K, a.stride(0), b.stride(0), out.stride(0), 1, 1, 5,
          status_tensor(a.device).data_ptr(), _lib.raw_stream())
 

@@ -123,6 +123,13 @@ def test_anomaly_detection_sees_a_nan_weight_gradient(added):
     assert added == [] and not w.grad.isnan().any()
 
 
+def test_gradient_that_is_differentiated_again_is_returned(added):
+    w = _weight()
+    x = X.clone().requires_grad_()
+    _Product.apply(x, w).square().sum().backward(create_graph=True)
+    assert added == [] and w.grad.requires_grad
+
+
 def test_buffer_saved_for_another_backward_is_known_to_have_changed(added):
     w = _weight()
     k = torch.ones((), dtype=torch.bfloat16, requires_grad=True)

@@ -277,8 +277,8 @@ def test_small_products_as_planned(M, N, K, kind):
 
 @pytest.mark.parametrize("K,M,N", [(1, 512, 3072), (7, 264, 520), (64, 256, 256), (250, 3072, 1024), (1000, 8, 4096), (333, 4096, 2056)])
 def test_weight_gradient_added_in_the_epilogue(K, M, N):
-    """``out += a.T @ b`` rounds the product to bf16 and adds with one more rounding: the bits of a separate addition up to the order of
-    the product's fp32 sums (a tie of one bf16 step in places).  Any row count; columns beside the window stay as they are."""
+    """``out += a.T @ b`` rounds the product to bf16 and adds with one more rounding: the bits of a separate addition of this kernel's
+    product (which added to zeros gives that).  Any row count; columns beside the window stay as they are."""
     from teletron_b200.ops import gemm
     from teletron_b200.ops.gemm_tcgen05 import add_supported, check_status
     g = torch.Generator(device="cuda").manual_seed(K)
@@ -291,14 +291,22 @@ def test_weight_gradient_added_in_the_epilogue(K, M, N):
     assert (out.double() - ref).abs().max() <= 2 ** -7 * ref.abs().max()
     assert (out.double() - ref).norm() < 4e-3 * ref.norm()          # 2^-9 per rounding
     assert torch.equal(whole[:, :8], before[:, :8]) and torch.equal(whole[:, 8 + N:], before[:, 8 + N:])
+    product = torch.zeros(M, N, device="cuda", dtype=torch.bfloat16)
+    assert gemm.gemm_tn_add(a, b, product)
+    assert torch.equal(out, before[:, 8:8 + N] + product)
 
 
 def test_flat_gradient_buffers_receive_products_only_where_autograd_accumulates():
-    """Parameters in a flat buffer: ``backward`` adds each weight gradient exactly once per pass, with the bits of the separate addition;
-    ``autograd.grad``, hooks, ``create_graph`` and a side stream see gradients as before."""
+    """Parameters in a flat buffer: ``backward`` adds each weight gradient exactly once per pass (four products: the merged projection has
+    two halves); ``autograd.grad``, hooks on the parameter or on its node, and a side stream see gradients as before."""
     from teletron_b200 import ops
     from teletron_b200.ops.gemm_tcgen05 import COUNTERS
     from teletron_b200.parallel.grad_buffer import DistributedDataParallel
+
+    def additions(f):
+        n0 = COUNTERS["add"]
+        f()
+        return COUNTERS["add"] - n0
 
     class Net(torch.nn.Module):
         def __init__(self):
@@ -319,13 +327,13 @@ def test_flat_gradient_buffers_receive_products_only_where_autograd_accumulates(
     names = ("w1", "b1", "w2", "w3")
     for _ in range(2):                                       # two micro-batches
         plain(x).backward(dy)
-        n0 = COUNTERS["pair"]
-        ddp(x).backward(dy)
-    assert COUNTERS["pair"] > n0
+        assert additions(lambda: ddp(x).backward(dy)) == 4
     for n in names:
         torch.testing.assert_close(getattr(net, n).grad, getattr(plain, n).grad, rtol=1.6e-2, atol=1e-2)
     kept = {n: getattr(net, n).grad.clone() for n in names}
+    n0 = COUNTERS["add"]
     got = torch.autograd.grad(net(x), [net.w1, net.w2, net.w3], dy)
+    assert COUNTERS["add"] == n0
     want = torch.autograd.grad(plain(x), [plain.w1, plain.w2, plain.w3], dy)
     for a, b in zip(got, want):
         torch.testing.assert_close(a, b, rtol=1.6e-2, atol=1e-2)
@@ -333,20 +341,64 @@ def test_flat_gradient_buffers_receive_products_only_where_autograd_accumulates(
     seen = []
     h1 = net.w1.register_hook(lambda t: seen.append("w1"))
     h2 = net.w2.register_post_accumulate_grad_hook(lambda p: seen.append("w2"))
-    net(x).backward(dy)
+    assert additions(lambda: net(x).backward(dy)) == 2          # w3's
     assert sorted(seen) == ["w1", "w2"]
     h1.remove()
     h2.remove()
+    node = net.w3.expand_as(net.w3).grad_fn.next_functions[0][0]
+    h3 = node.register_hook(lambda _, g: seen.append(g[0].shape))
+    assert additions(lambda: net(x).backward(dy)) == 2          # w1's and w2's
+    assert seen[2:] == [net.w3.shape]
+    h3.remove()
+    del node
     side = torch.cuda.Stream()
     side.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(side):
-        net(x).backward(dy)
+        assert additions(lambda: net(x).backward(dy)) == 0
     torch.cuda.current_stream().wait_stream(side)
-    net(x).backward(dy, inputs=[net.b1])                    # nothing for the weights
-    for _ in range(2):
+    assert additions(lambda: net(x).backward(dy, inputs=[net.b1])) == 0
+    assert additions(lambda: net(x).backward(dy, inputs=[net.w2])) == 1
+    for _ in range(3):
         plain(x).backward(dy)
+    plain(x).backward(dy, inputs=[plain.w2])
     for n in ("w1", "w2", "w3"):
         torch.testing.assert_close(getattr(net, n).grad, getattr(plain, n).grad, rtol=1.6e-2, atol=2e-2)
+
+
+def test_flat_gradient_buffers_of_the_two_stream_projection():
+    """One autograd node with two weights: both products are added, each to its own buffer, in any row count."""
+    from teletron_b200 import ops
+    from teletron_b200.ops.gemm_tcgen05 import COUNTERS, check_status
+    from teletron_b200.parallel.grad_buffer import DistributedDataParallel
+    heads, S, T = 2, 45, 11
+    H = heads * 128
+
+    class Net(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            g = torch.Generator(device="cuda").manual_seed(13)
+            for i in (1, 2):
+                for n, shape, k in (("w", (3 * H, H), 0.05), ("b", (3 * H,), 0.1), ("qw", (128,), 0.2), ("kw", (128,), 0.2)):
+                    setattr(self, f"{n}{i}", torch.nn.Parameter(_mk(shape, g, k)))
+
+        def forward(self, x, y):
+            return ops.joint_qkv_projection(x, self.w1, self.b1, self.qw1, self.kw1, cos, sin, y, self.w2, self.b2, self.qw2, self.kw2, heads)
+
+    g = torch.Generator(device="cuda").manual_seed(14)
+    x, y = _mk((1, S, H), g), _mk((1, T, H), g)
+    ang = torch.rand(S, 64, device="cuda", generator=g) * 6.28
+    cos, sin = ang.cos().repeat_interleave(2, 1), ang.sin().repeat_interleave(2, 1)
+    d = [_mk((1, heads, S + T, 128), g) for _ in range(3)]
+    plain, net = Net(), Net()
+    ddp = DistributedDataParallel(net, None)
+    for _ in range(2):
+        torch.autograd.backward(plain(x, y), d)
+        n0 = COUNTERS["add"]
+        torch.autograd.backward(ddp(x, y), d)
+        assert COUNTERS["add"] == n0 + 2
+    check_status()
+    for (n, a), (_, b) in zip(net.named_parameters(), plain.named_parameters()):
+        assert _rel(a.grad, b.grad) < 4e-3, n
 
 
 def test_flat_gradient_added_before_an_accumulation_node_of_another_stream_runs():
