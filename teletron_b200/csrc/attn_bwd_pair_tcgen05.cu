@@ -27,14 +27,14 @@
 // not have to be on them is kept off: eight warps of their own read dQ out of tensor memory (the softmax warps doing it: 32.6 ms); the
 // exchange is a bulk copy from a buffer (stores to the peer's memory from the softmax warps held up every other shared-memory access for
 // ~1000 clocks a chunk); statistics come scaled and padded, one ld.shared each.  Registers are split by role (setmaxnreg): spills
-// in the MMA or the read-out warps cost up to 10 ms.  24 heads x 32656 tokens: 28.3 ms, 29.0 under sustained load (single CTAs: 32.7 and
-// 34.2); 3 heads x 119056: 47.5 (56.1).
+// in the MMA or the read-out warps cost up to 10 ms.  24 heads x 32656 tokens: 28.4 ms, 29.0 under sustained load (single CTAs: 32.7 and
+// 34.2); 3 heads x 119056: 47.4 (55.8); 24 x 6144: 1.00 (1.15).
 //
 // Synchronisation (mbarriers, bounded waits): "leader" barriers live in CTA 0, whose MMA thread issues for the pair; commits arrive
 // in both CTAs.  The bytes of the exchange complete, at cluster scope, on a barrier of the receiving CTA.  CTA 1's relay thread passes that
 // on to the leader, and with it its softmax warps' own half of dS, which they have stored for products that the leader issues: for those
 // it fences at cluster scope, while the exchange is under way.  (Released by the arrival itself, behind the exchange: 30.6 ms instead of
-// 28.5 at 24 heads x 32656 tokens, 52.3 instead of 47.6 at 3 x 119056; by arrivals of the softmax warps: 14 ms more.)
+// 28.4 at 24 heads x 32656 tokens, 52.3 instead of 47.4 at 3 x 119056; by arrivals of the softmax warps: 14 ms more.)
 // utils/pair_pipeline_model.py checks the protocol.
 #include "common.cuh"
 #include "sm100.cuh"
@@ -169,7 +169,7 @@ attn_bwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // barrier addresses are computed anew from here on: kept from the initialisation they would be spilled
     asm volatile("mov.u32 %0, %0;" : "+r"(base));
     // The split stands inside the branches that the roles share: ahead of them, where the paths meet again, the compiler holds every role
-    // to the smallest share and spills (24 heads x 6144 tokens: 1.144 -> 1.103 ms, x 32656: 28.7 -> 28.3).
+    // to the smallest share and spills (24 heads x 32656 tokens: 28.7 -> 28.3 ms).
     if (warp < kFirstSoftmax) {
     reg_dec<kRegsMisc>();
     if (warp == 0) {

@@ -276,7 +276,8 @@ __global__ void __launch_bounds__(MAXT, 1) ln_mod_bwd_kernel(
 // stores this kernel is no faster, without the first pass's arithmetic it is by a fifth).  So a batch's sums are handed over through
 // one of four buffers (an mbarrier each) and the first pass of the next batch runs before they are waited for; statistics are
 // loaded a batch ahead; the rows of a whole batch are one block of code, so that their chains overlap; the arithmetic is packed
-// (fp32x2).  Wider rows (two or three stages, fewer registers a thread) take the passes one after the other.  32656 x 3072: plain
+// (fp32x2).  Wider rows (two or three stages, fewer registers a thread) take the passes one after the other;
+// the gated form beyond 4096 columns spills there (72 registers, about 270 bytes stored a thread).  32656 x 3072: plain
 // 168 -> 132 us, gated 342 -> 256, from normalised rows (fused_adaln) 138 -> 117 (600 MB, 5.1 TB/s); 16000 x 6144: 190 -> 164, 423 -> 346, 171 -> 142.
 // ---------------------------------------------------------------------------------------------
 __device__ int g_norm_status = 0;       // TT_ERR_TIMEOUT when a bounded wait of the ring ran out (read by tt_norm_status)

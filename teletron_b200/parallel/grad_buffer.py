@@ -106,7 +106,10 @@ class ParamAndGradBuffer:
             view.copy_(p.data)
             p.data = view
             p.grad = self.grad_data[s:e].view(p.shape)
-            p.flat_grad = True              # weight-gradient products may add to p.grad themselves (ops/cuda_ops.py)
+            # Weight-gradient products may add to p.grad themselves (ops/cuda_ops.py) where nobody looks at the gradient on its way: not
+            # with hooks, so not while bucket reductions overlap the backward, nor inside the fused collectives.  Hooks that a
+            # C++ extension adds to the accumulation node are not seen: set this to False for such parameters.
+            p.flat_grad = True
         self.params = [p for _, p in ordered]
         # buckets in reverse buffer order approximate backward order; each bucket is a multiple of
         # shard_count * 8 elements so reduce-scatter shards stay aligned
